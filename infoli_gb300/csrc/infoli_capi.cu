@@ -38,6 +38,10 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kMaxStepsPerLaunch = 8192;
+// Of a stream plan's entries, what L2 (129 MB) is asked to keep from step to
+// step.  16,000 cells at 30 % (154 MB of entries): 38.1 us per step with 70 MB,
+// 38.3 with 50, 39.8 with 85, 42.2 with 100.
+constexpr double kStreamL2Bytes = 70e6;
 constexpr size_t kTraceSlotBytes = 64u << 20;
 
 // Device memory of simulation handles comes from one stream-ordered pool per
@@ -142,6 +146,7 @@ struct infoli_sim {
   float last_ms = 0.0f;
   int last_launches = 0;
   int async_pending = 0;  // infoli_sim_launch work not yet checked for device errors
+  float l2_keep = 1.0f;   // stream plans, see StepArgs
   int64_t dev_bytes = 0;  // device memory held for the plan and the state
 };
 
@@ -307,6 +312,7 @@ int fill_args(infoli_sim* s, StepArgs* a) {
   a->gcol = s->d_gcol;
   a->perm = s->d_perm;
   a->n_cells = s->n;
+  a->l2_keep = s->l2_keep;
   return INFOLI_OK;
 }
 
@@ -327,6 +333,8 @@ int check_device_error(infoli_sim* s) {
   CK(cudaStreamSynchronize(s->stream));
   if (err != DEV_OK) {
     cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream);
+    if (err == DEV_ERR_CONFIG)
+      return infoli__fail(INFOLI_ERR_CUDA, "the step kernel was launched without the clusters of its plan");
     return infoli__fail(INFOLI_ERR_TIMEOUT, "device wait gave up (code %d): %s", err,
                         err == DEV_ERR_BARRIER_TIMEOUT ? "grid barrier timeout"
                         : err == DEV_ERR_STAMP_TIMEOUT ? "stamped V_dend exchange timeout"
@@ -408,12 +416,17 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
                     : !strcmp(sm, "gather")  ? kSyncGather
                     : !strcmp(sm, "tgather") ? kSyncTiledGather
                     : !strcmp(sm, "bits")    ? kSyncBits
+                    : !strcmp(sm, "stream")  ? kSyncStream
                                              : kSyncAuto;
   // 512-thread CTAs (128 registers per thread) whenever the network fits in
   // one cell per thread at that size; 1024 threads for larger networks.
   // INFOLI_THREADS=512|1024 overrides.
   int want_threads = 0;
   if (const char* ts = getenv("INFOLI_THREADS")) want_threads = atoi(ts) == 512 ? 512 : 1024;
+  // stream plans run 1024 threads; their clusters only where the simulation may
+  // have the whole GPU (a share of the SMs need not come in whole clusters)
+  pin.no_stream = want_threads == 512 ? 1 : 0;
+  for (int i = 0; i < 2; ++i) pin.cluster_ctas[i] = d->grid > 0 ? 0 : max_stream_ctas(2 << i, pin.smem_budget);
   std::string perr;
   bool planned = false;
   for (int threads : {512, kThreads}) {
@@ -476,7 +489,7 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
         pool_alloc(&s->d_vll[1], np * sizeof(unsigned long long), dv, st0) != cudaSuccess)
       return fail(infoli__fail(INFOLI_ERR_NOMEM, "sim_create: device allocation failed"));
   }
-  if (s->plan.shape.gather == 3) {
+  if (s->plan.shape.gather >= 3) {
     if (pool_alloc(&s->d_vds[0], np * sizeof(float), dv, st0) != cudaSuccess ||
         pool_alloc(&s->d_vds[1], np * sizeof(float), dv, st0) != cudaSuccess)
       return fail(infoli__fail(INFOLI_ERR_NOMEM, "sim_create: device allocation failed"));
@@ -500,6 +513,8 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
   if (cudaEventCreate(&s->ev_t0) != cudaSuccess || cudaEventCreate(&s->ev_t1) != cudaSuccess)
     return fail(infoli__fail(INFOLI_ERR_CUDA, "event creation failed"));
   const Plan& pl = s->plan;
+  const double entry_bytes = (double)pl.edges.size() * sizeof(uint16_t) + (double)pl.edge_g.size() * sizeof(float);
+  if (entry_bytes > 0) s->l2_keep = (float)std::min(1.0, kStreamL2Bytes / entry_bytes);
   s->dev_bytes = (int64_t)(pl.cta.size() * sizeof(CtaWork) + pl.tiles.size() * sizeof(TileDesc) +
                            pl.chunks.size() * sizeof(ChunkDesc) + pl.cell_slots.size() * sizeof(CellSlots) +
                            pl.edges.size() * sizeof(uint16_t) + pl.edge_g.size() * sizeof(float) +

@@ -49,6 +49,7 @@ struct StepArgs {
   float* vds[2];              // bitmask plans: V_dend x kVScale (the staged tiles), V^step in vds[step & 1]
   const int* probes;          // stamped mode: progress-probe cells (CtaWork::probe_begin..)
   const int2* gdesc;          // stamped mode: {slot, recv} per lane-chunk (32 per group)
+  float l2_keep;              // stream plans: share of the entries' lines that L2 should keep
   int n_cells;                // cells in the network (stamped words >= n_cells are never written)
   float* st;                  // F_COUNT x n_pad floats
   double* ca;                 // Ca2Plus, n_pad doubles
@@ -94,6 +95,14 @@ size_t step_kernel_smem(const StepArgs& a);
 
 // Cooperative launch of the persistent kernel over `grid` CTAs.
 cudaError_t launch_step_kernel(const StepArgs& a, int grid, int threads, cudaStream_t stream);
+
+// The same for stream plans (infoli_stream.cu), in clusters of
+// a.shape.cluster CTAs; launch_step_kernel calls it for them.
+cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t stream);
+
+// Most CTAs of the stream kernel the device runs at once in clusters of
+// `cluster` with `smem` bytes of dynamic shared memory each (0: none).
+int max_stream_ctas(int cluster, size_t smem);
 
 // Largest co-resident grid for `threads` threads and the given dynamic smem.
 int max_coresident_ctas(int threads, size_t smem, cudaError_t* err = nullptr);

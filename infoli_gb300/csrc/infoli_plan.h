@@ -119,9 +119,15 @@ typedef struct {
                    // two zero words after each row (CtaWork::pad0 = words per row);
                    // tiles cover whole 32-sender columns (TileDesc::chunk_begin /
                    // chunk_end = first / end column); `slices` threads share a row
+                   // 4: stream plan (see StreamLayout): one or more CTAs per receiver group,
+                   // each staging its share of V_dend whole (tile_cap floats) and
+                   // streaming its lane-chunks' entries from global memory
   int slices;      // bitmask plan: threads per receiver (column slices)
   int poll_words;  // stamped: the most words one CTA polls per step (window
                    // senders + progress probes); picks the poll batch size
+  int cluster;     // stream plan: CTAs per cluster (sender shares)
+  int rows_cap;    // stream plan with cluster > 1: staged V_dend of the cluster's receivers
+  int split_units; // stream plan: gate units over all warps, gate state in shared memory
 } SmemShape;
 
 static inline INFOLI_HD size_t tgather_smem_bytes(SmemShape s) {
@@ -184,6 +190,55 @@ static inline INFOLI_HD SmemLayout smem_layout(SmemShape s) {
   L.edges = off;
   off += (size_t)s.res_edges * sizeof(uint16_t);
   off = (off + 15) & ~(size_t)15;
+  L.total = off;
+  return L;
+}
+
+// Stream plans.  A cluster of `cluster` CTAs owns a contiguous run of
+// receivers (rows CtaWork::tile_begin .. + n_tiles); every CTA of it owns a
+// contiguous part of them (cell_begin, n_cells: one thread per cell runs the
+// cell update) and holds one share of the senders, tile_cap consecutive
+// V_dend, in shared memory (share k: cells k * tile_cap ..).  The rows'
+// entries in that share are cut into lane-chunks, one lane each; 32 chunks of
+// like length form a group, a warp walks the groups assigned to it
+// (probes[pad0 + warp] .. probes[pad0 + warp + 1], relative to group_begin).
+// Group i: gdesc[i] = {first quad row, quads per lane}, a quad row being 32
+// lanes x 4 entries; gcol[32 i + lane] = row | slot << 16.  Entry k of lane l
+// lies at (first * 128) + (k / 8) * 256 + l * 8 + k % 8 in the edge array while
+// whole 8-entry pairs last (16-byte loads), the odd quad after them at
+// + l * 4 + k % 4; its conductance at (first * 128) + (k / 4) * 128 + l * 4 + k % 4.
+// An entry is the index of a float from the start of dynamic shared memory;
+// padding entries name the row's own V_dend (a term of exactly 0).  Partial
+// sums: cell_slots[cell * cluster + k] = its slots in CTA k of the cluster.
+//   [share of V_dend][cluster > 1: the rows' V_dend][partial sums, with KAHAN
+//   as (sum, compensation) pairs][mbarrier][split_units: 12 cell arrays, Ca2+,
+//   gate state]
+enum { kStreamThreads = 1024, kStreamWarps = 32, kStreamMaxCluster = 4, kStreamCellArrays = 12 };
+typedef struct {
+  size_t rows, part, mbar, cells, gca, gates, total;
+} StreamLayout;
+
+static inline INFOLI_HD StreamLayout stream_layout(SmemShape s) {
+  StreamLayout L;
+  size_t off = (size_t)s.tile_cap * sizeof(float);
+  L.rows = off;
+  off += (size_t)s.rows_cap * sizeof(float);
+  off = (off + 15) & ~(size_t)15;
+  L.part = off;
+  off += (size_t)s.max_slots * sizeof(float) * (s.kahan ? 2 : 1);
+  off = (off + 15) & ~(size_t)15;
+  L.mbar = off;
+  off += 16;
+  L.cells = off;
+  L.gca = off;
+  L.gates = off;
+  if (s.split_units) {
+    off += (size_t)kStreamCellArrays * (size_t)s.cells_cap * sizeof(float);
+    L.gca = off;
+    off += (size_t)s.cells_cap * sizeof(double);
+    L.gates = off;
+    off += (size_t)kGateFloats * (size_t)s.cells_cap * sizeof(float);
+  }
   L.total = off;
   return L;
 }

@@ -22,6 +22,7 @@ size_t plan_smem_bytes(int tile_cap, int nbuf, int threads, int cells_cap, int m
 namespace {
 
 constexpr int kCellCost = 8;  // edge-equivalents charged per cell when balancing CTAs
+constexpr int kStreamSplitCells = 256;  // stream plans: gate units over all warps up to this many cells per CTA
 constexpr int kSmallNetworkCtas = 100;  // the most CTAs the small-network floor asks for
 
 // Contiguous partition of cells into at most `grid` CTAs, each at most
@@ -612,6 +613,363 @@ static bool make_bits_plan(const PlanInput& in, Plan* out, std::string* err) {
   return true;
 }
 
+// ------------------------------------------------------------ stream plans
+
+namespace {
+
+// A row's entries in one share of the senders, cut into pieces of at most
+// `len` entries as even as possible.
+inline int stream_pieces(int entries, int len) { return entries ? (entries + len - 1) / len : 0; }
+
+struct StreamCut {
+  int len = 0;         // longest lane-chunk
+  double cost = 0.0;   // busiest warp, in entries per lane
+  int slots = 0;
+};
+
+// Groups (padded lengths, descending) of rows cut at `len`, and the busiest
+// warp's load when they are dealt longest first to the least loaded warp.
+// kGroupCost: a group's fixed cost (descriptor and first entries from L2,
+// the write of 32 partial sums), kSlotCost: a slot's in the owner's sum.
+constexpr double kStreamGroupCost = 8.0, kStreamSlotCost = 0.4;
+
+StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, std::vector<int>& hist) {
+  StreamCut c;
+  c.len = len;
+  hist.assign((size_t)std::min(len, max_len) + 2, 0);
+  int most = 0;
+  for (int e : rows) {
+    const int p = stream_pieces(e, len);
+    if (!p) continue;
+    most = std::max(most, p);
+    c.slots += p;
+    hist[(size_t)(e / p)] += p - e % p;
+    if (e % p) hist[(size_t)(e / p) + 1] += e % p;
+  }
+  double load[kStreamWarps] = {0.0};
+  int in_group = 0, group_len = 0;
+  auto place = [&](int l) {
+    int best = 0;
+    for (int w = 1; w < kStreamWarps; ++w)
+      if (load[w] < load[best]) best = w;
+    load[best] += ((l + 3) & ~3) + kStreamGroupCost;
+  };
+  for (int l = (int)hist.size() - 1; l > 0; --l) {
+    int left = hist[(size_t)l];
+    while (left > 0) {
+      if (in_group == 0) group_len = l;
+      const int take = std::min(left, 32 - in_group);
+      in_group += take;
+      left -= take;
+      if (in_group == 32) {
+        place(group_len);
+        in_group = 0;
+      }
+    }
+  }
+  if (in_group) place(group_len);
+  c.cost = *std::max_element(load, load + kStreamWarps) + kStreamSlotCost * most;
+  return c;
+}
+
+}  // namespace
+
+static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
+  const int n = in.n;
+  const size_t slot_bytes = in.kahan ? 2 * sizeof(float) : sizeof(float);
+  // ---- cluster size: the fewest sender shares whose V_dend fits
+  SmemShape sh{};
+  sh.threads = kStreamThreads;
+  sh.kahan = in.kahan;
+  sh.edge_g = in.g != nullptr;
+  sh.gather = 4;
+  sh.nbuf = 1;
+  std::vector<int> starts;
+  int max_rows = 0;
+  for (int cs = 1; cs <= kStreamMaxCluster; cs *= 2) {
+    int most = in.grid_max;
+    if (cs > 1) {
+      const int lim = in.cluster_ctas[cs == 2 ? 0 : 1];
+      most = lim < 0 ? in.grid_max : std::min(in.grid_max, lim);
+    }
+    int grid = in.grid > 0 ? std::min(in.grid, most) : most;
+    grid = std::max(grid, (n + kStreamThreads - 1) / kStreamThreads);
+    const int nclus = grid / cs;
+    if (grid > most || nclus < 1 || (int64_t)nclus * cs * kStreamThreads < n) continue;
+    const int share = (((n + cs - 1) / cs) + 31) & ~31;
+    if (share > 65536 - 8 * kStreamThreads) continue;  // 16-bit indices cover the share and the rows after it
+    std::vector<int> st = partition_cells(n, in.row_ptr, nclus, kStreamThreads * cs);
+    int mr = 1;
+    for (size_t b = 0; b + 1 < st.size(); ++b) mr = std::max(mr, st[b + 1] - st[b]);
+    sh.cluster = cs;
+    sh.tile_cap = share;
+    sh.rows_cap = cs > 1 ? ((mr + 3) & ~3) + 8 : 0;
+    sh.max_slots = mr;
+    if (stream_layout(sh).total > in.smem_budget) continue;
+    starts.swap(st);
+    max_rows = mr;
+    break;
+  }
+  if (starts.empty()) {
+    *err = "make_plan: the senders' shares do not fit in shared memory";
+    return false;
+  }
+  const int cs = sh.cluster, share = sh.tile_cap;
+  const int nclus = (int)starts.size() - 1, ctas = nclus * cs;
+  sh.cells_cap = 32;
+  for (int b = 0; b < nclus; ++b) {
+    const int per = (starts[b + 1] - starts[b] + cs - 1) / cs;
+    sh.cells_cap = std::max(sh.cells_cap, (per + 31) & ~31);
+  }
+  // gate units over all warps with the gate state in shared memory, where few
+  // cells per CTA leave most warps without an own cell and the state fits
+  sh.max_slots = max_rows;
+  if (sh.cells_cap <= kStreamSplitCells) {
+    sh.split_units = 1;
+    if (stream_layout(sh).total > in.smem_budget) sh.split_units = 0;
+  }
+  sh.max_slots = 0;
+  const int slots_cap = (int)std::min<size_t>(65535, (in.smem_budget - stream_layout(sh).total) / slot_bytes);
+
+  Plan& P = *out;
+  P = Plan();
+  P.grid = ctas;
+  P.threads = kStreamThreads;
+  P.cell_slots.assign((size_t)n * cs, CellSlots{0, 0});
+  struct Local {
+    std::vector<int2_t> gdesc;  // {first quad row (local), quads}
+    std::vector<int32_t> lane;  // row | slot << 16
+    std::vector<uint16_t> ent;
+    std::vector<float> g;
+    int warp[kStreamWarps + 1];
+    int slots = 0;
+    bool ok = true;
+  };
+  std::vector<Local> loc((size_t)ctas);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int b = 0; b < ctas; ++b) {
+    Local& L = loc[(size_t)b];
+    const int cl = b / cs, k = b % cs;
+    const int r0 = starts[cl], rows = starts[cl + 1] - r0;
+    const int lo = k * share, hi = std::min(n, lo + share);
+    const int own = cs > 1 ? share + (r0 & 3) : r0;  // float index of the first row's own V_dend
+    // entries of every row in this share
+    std::vector<uint16_t> idx;
+    std::vector<float> gv;
+    std::vector<int> cnt((size_t)rows, 0);
+    std::vector<size_t> at((size_t)rows + 1, 0);
+    const int64_t e0 = in.row_ptr[r0], e1 = in.row_ptr[r0 + rows];
+    idx.reserve((size_t)(e1 - e0) / cs + 16);
+    int max_len = 0;
+    for (int r = 0; r < rows; ++r) {
+      for (int64_t e = in.row_ptr[r0 + r]; e < in.row_ptr[r0 + r + 1]; ++e) {
+        const int s = in.col[e];
+        if (s < lo || s >= hi) continue;
+        idx.push_back((uint16_t)(s - lo));
+        if (in.g) gv.push_back(in.g[e]);
+      }
+      at[(size_t)r + 1] = idx.size();
+      cnt[(size_t)r] = (int)(at[(size_t)r + 1] - at[(size_t)r]);
+      max_len = std::max(max_len, cnt[(size_t)r]);
+    }
+    // lane-chunk length: the cheapest of a few whose slots fit
+    std::vector<int> hist;
+    StreamCut best;
+    for (int len : {16, 20, 24, 28, 32, 40, 48, 56, 64, 80, 96, 112, 128, 160, 192, 224, 256, 320, 384, 512, 768, 1024,
+                    2048, 4096, 1 << 30}) {
+      const StreamCut c = stream_cut_cost(cnt, len, max_len, hist);
+      if (c.slots < slots_cap && (best.len == 0 || c.cost < best.cost)) best = c;
+      if (len >= max_len) break;
+    }
+    if (best.len == 0) {
+      L.ok = false;
+      continue;
+    }
+    // lane-chunks, receiver-major slots
+    struct Piece {
+      int row, slot, len;
+      size_t begin;
+    };
+    std::vector<Piece> pc;
+    int slot = 0;
+    for (int r = 0; r < rows; ++r) {
+      const int p = stream_pieces(cnt[(size_t)r], best.len);
+      P.cell_slots[(size_t)(r0 + r) * cs + k] = CellSlots{slot, p};
+      size_t o = at[(size_t)r];
+      for (int q = 0; q < p; ++q) {
+        const int len = cnt[(size_t)r] / p + (q < cnt[(size_t)r] % p ? 1 : 0);
+        pc.push_back({r, slot++, len, o});
+        o += (size_t)len;
+      }
+    }
+    L.slots = slot;
+    std::stable_sort(pc.begin(), pc.end(), [](const Piece& x, const Piece& y) { return x.len > y.len; });
+    const int ng = ((int)pc.size() + 31) / 32;
+    // groups to warps, longest first to the least loaded; a warp's groups contiguous
+    std::vector<int> of_warp((size_t)ng);
+    {
+      double load[kStreamWarps] = {0.0};
+      for (int g = 0; g < ng; ++g) {
+        int w = 0;
+        for (int q = 1; q < kStreamWarps; ++q)
+          if (load[q] < load[w]) w = q;
+        load[w] += ((pc[(size_t)g * 32].len + 3) & ~3) + kStreamGroupCost;
+        of_warp[(size_t)g] = w;
+      }
+    }
+    std::vector<int> next;
+    std::vector<int> head(32 * 32);
+    int placed = 0;
+    for (int w = 0; w < kStreamWarps; ++w) {
+      L.warp[w] = placed;
+      for (int g = 0; g < ng; ++g) {
+        if (of_warp[(size_t)g] != w) continue;
+        ++placed;
+        const int quads = (pc[(size_t)g * 32].len + 3) / 4, pairs = quads / 2, len = quads * 4;
+        const size_t base = L.ent.size();
+        L.gdesc.push_back(int2_t{(int)(base / 128), quads});
+        L.ent.resize(base + (size_t)quads * 128);
+        if (in.g) L.g.resize(base + (size_t)quads * 128);
+        // Lanes reading position k of a group should hit different banks: the
+        // entries of each lane are bucketed by bank, and position by position
+        // every lane takes one from a bank no other lane has taken, where it
+        // has such an entry left (banks tried from a start that rotates).
+        std::fill(head.begin(), head.end(), -1);
+        unsigned avail[32];
+        int left[32], pad[32];
+        size_t lb[32];
+        next.assign((size_t)32 * len, -1);
+        for (int l = 0; l < 32; ++l) {
+          const size_t i = (size_t)g * 32 + l;
+          avail[l] = 0;
+          left[l] = 0;
+          lb[l] = 0;
+          pad[l] = own;
+          int desc = (int)((unsigned)slot << 16);  // lanes past the last chunk: the spare slot
+          if (i < pc.size()) {
+            desc = pc[i].row | (int)((unsigned)pc[i].slot << 16);
+            pad[l] = own + pc[i].row;
+            left[l] = pc[i].len;
+            lb[l] = pc[i].begin;
+            for (int q = pc[i].len - 1; q >= 0; --q) {
+              const int bank = idx[lb[l] + (size_t)q] & 31;
+              next[(size_t)l * len + q] = head[(size_t)l * 32 + bank];
+              head[(size_t)l * 32 + bank] = q;
+              avail[l] |= 1u << bank;
+            }
+          }
+          L.lane.push_back(desc);
+        }
+        for (int q = 0; q < len; ++q) {
+          unsigned taken = 0;
+          int late[32], nlate = 0;
+          int pick[32];
+          for (int l = 0; l < 32; ++l) {
+            pick[l] = -1;
+            if (left[l] == 0) taken |= 1u << (pad[l] & 31);
+          }
+          auto take = [&](int l, unsigned cand) {
+            const int rot = (l + q) & 31;
+            const unsigned c = rot ? (cand >> rot) | (cand << (32 - rot)) : cand;
+            const int bank = (__builtin_ctz(c) + rot) & 31;
+            int& h = head[(size_t)l * 32 + bank];
+            pick[l] = h;
+            h = next[(size_t)l * len + h];
+            if (h < 0) avail[l] &= ~(1u << bank);
+            taken |= 1u << bank;
+            --left[l];
+          };
+          for (int j = 0; j < 32; ++j) {
+            const int l = (j + q) & 31;
+            if (left[l] == 0) continue;
+            const unsigned cand = avail[l] & ~taken;
+            if (cand)
+              take(l, cand);
+            else
+              late[nlate++] = l;
+          }
+          for (int j = 0; j < nlate; ++j) take(late[j], avail[late[j]]);
+          for (int l = 0; l < 32; ++l) {
+            const size_t e = q < pairs * 8 ? base + (size_t)(q / 8) * 256 + l * 8 + q % 8
+                                           : base + (size_t)pairs * 256 + l * 4 + q % 4;
+            L.ent[e] = pick[l] < 0 ? (uint16_t)pad[l] : idx[lb[l] + (size_t)pick[l]];
+            if (in.g)
+              L.g[base + (size_t)(q / 4) * 128 + l * 4 + q % 4] = pick[l] < 0 ? 0.0f : gv[lb[l] + (size_t)pick[l]];
+          }
+        }
+      }
+    }
+    L.warp[kStreamWarps] = placed;
+  }
+  int max_slots = 0;
+  size_t total = 0, groups = 0;
+  for (const Local& L : loc) {
+    if (!L.ok) {
+      *err = "make_plan: the rows' partial sums do not fit in shared memory";
+      return false;
+    }
+    max_slots = std::max(max_slots, L.slots + 1);  // + the spare slot of lanes without a chunk
+    total += L.ent.size();
+    groups += L.gdesc.size();
+  }
+  sh.max_slots = max_slots;
+  if (stream_layout(sh).total > in.smem_budget) {
+    *err = "make_plan: could not fit shared memory";
+    return false;
+  }
+  P.edges.resize(total);
+  if (in.g) P.edge_g.resize(total);
+  P.gdesc.reserve(groups);
+  P.gcol.reserve(groups * 32);
+  std::vector<size_t> off((size_t)ctas + 1, 0);
+  for (int b = 0; b < ctas; ++b) {
+    Local& L = loc[(size_t)b];
+    off[(size_t)b + 1] = off[(size_t)b] + L.ent.size();
+    const int cl = b / cs, k = b % cs;
+    const int r0 = starts[cl], rows = starts[cl + 1] - r0, per = (rows + cs - 1) / cs;
+    CtaWork w{};
+    w.cell_begin = r0 + std::min(rows, k * per);
+    w.n_cells = r0 + std::min(rows, (k + 1) * per) - w.cell_begin;
+    w.tile_begin = r0;
+    w.n_tiles = rows;
+    w.n_slots = L.slots;
+    w.group_begin = (int)P.gdesc.size();
+    w.n_groups = (int)L.gdesc.size();
+    w.pad0 = (int)P.probes.size();
+    w.pad1 = k;
+    P.cta.push_back(w);
+    P.probes.insert(P.probes.end(), L.warp, L.warp + kStreamWarps + 1);
+    for (int2_t d : L.gdesc) {
+      d.x += (int)(off[(size_t)b] / 128);
+      P.gdesc.push_back(d);
+    }
+    P.gcol.insert(P.gcol.end(), L.lane.begin(), L.lane.end());
+  }
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int b = 0; b < ctas; ++b) {
+    Local& L = loc[(size_t)b];
+    std::copy(L.ent.begin(), L.ent.end(), P.edges.begin() + (std::ptrdiff_t)off[(size_t)b]);
+    if (in.g) std::copy(L.g.begin(), L.g.end(), P.edge_g.begin() + (std::ptrdiff_t)off[(size_t)b]);
+    std::vector<uint16_t>().swap(L.ent);
+    std::vector<float>().swap(L.g);
+  }
+  P.tile_cap = share;
+  P.max_slots = max_slots;
+  P.shape = sh;
+  P.smem_bytes = stream_layout(sh).total;
+  return true;
+}
+
+// Auto mode's choice of a stream plan for edges that do not stay on chip.
+static bool stream_plan_wanted(const PlanInput& in) {
+  if (in.sync_mode != kSyncAuto || in.no_stream) return false;
+  const double n = (double)in.n, e = (double)in.row_ptr[in.n];
+  const size_t whole = (((size_t)in.n + 31) & ~(size_t)31) * sizeof(float) + kStreamThreads * 8 + 64;
+  if (whole <= in.smem_budget) return in.g || e < kStreamMaxDensity * n * n;
+  if (!in.g && e * kBitsMinDensityInv >= n * n) return false;
+  return e >= (double)kStreamMinDegree * n;
+}
+
 bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
   const int n = in.n;
   if (n <= 0 || !in.row_ptr || in.threads <= 0 || in.threads % 32 || in.grid_max <= 0) {
@@ -645,6 +1003,14 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
   if (in.sync_mode == kSyncGather) return make_gather_plan(in, out, err);
   if (in.sync_mode == kSyncTiledGather) return make_tgather_plan(in, out, err);
   if (in.sync_mode == kSyncBits) return make_bits_plan(in, out, err);
+  if (in.sync_mode == kSyncStream) return make_stream_plan(in, out, err);
+  // edges that cannot stay resident in shared memory (2 bytes, 6 with a
+  // conductance, per edge and CTA): no stamped plan is possible
+  if (in.sync_mode == kSyncAuto && stream_plan_wanted(in) &&
+      (E / std::max(1, in.grid_max)) * (int64_t)(sizeof(uint16_t) + (in.g ? sizeof(float) : 0)) >
+          (int64_t)in.smem_budget &&
+      make_stream_plan(in, out, err))
+    return true;
   // dense rows with one conductance whose edges cannot stay resident in shared
   // memory (2 bytes per edge per CTA): no stamped plan is possible, and auto
   // mode would pick the bitmask plan after building the tile plan; build it
@@ -972,6 +1338,13 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
   // instead of staging tiles (each row would be cut into a few edges per tile)
   // windows larger than shared memory: dense rows with one conductance walk
   // adjacency bits; short rows gather through staged tiles
+  if (!sh.stamped && stream_plan_wanted(in)) {
+    Plan st;
+    if (make_stream_plan(in, &st, err)) {
+      *out = std::move(st);
+      return true;
+    }
+  }
   if (!sh.stamped && in.sync_mode == kSyncAuto && !in.g &&
       E * kBitsMinDensityInv >= (int64_t)n * (int64_t)n)
     return make_bits_plan(in, out, err);
@@ -1267,14 +1640,80 @@ extern "C" int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t*
     ic_out = ic_plan.data();
   }
   const SmemLayout L = smem_layout(P.shape);
-  if (P.shape.gather >= 2 ? tgather_smem_bytes(P.shape) > (size_t)smem_budget
+  if (P.shape.gather == 4 && stream_layout(P.shape).total > (size_t)smem_budget) return -2;
+  if (P.shape.gather >= 2 && P.shape.gather < 4 ? tgather_smem_bytes(P.shape) > (size_t)smem_budget
                           : !P.shape.gather && L.total > (size_t)smem_budget)
     return -2;
   auto fexp = [](float V) { return 0.8f * std::exp(-(V * V) / 100.0f) + 0.2f; };
   std::vector<unsigned char> sm(P.shape.gather ? 0 : L.total);
   int64_t groups = 0, probes = 0, gather_waves = 0, gathers = 0;
   for (const CtaWork& w : P.cta) {
-    if (w.n_cells > threads || w.n_cells > P.shape.cells_cap) return -3;
+    if (w.n_cells > (P.shape.gather == 4 ? kStreamThreads : threads) || w.n_cells > P.shape.cells_cap) return -3;
+    if (P.shape.gather == 4) {
+      // one cluster at a time, at its first CTA: every CTA's image (share, rows),
+      // its groups into slots, then the owners' sums over the CTAs' slots
+      const int cs = P.shape.cluster, b0 = (int)(&w - P.cta.data());
+      if (w.pad1 != 0) continue;
+      std::vector<std::vector<float>> part((size_t)cs);
+      for (int k = 0; k < cs; ++k) {
+        const CtaWork& x = P.cta[(size_t)b0 + k];
+        if (x.pad1 != k || x.tile_begin != w.tile_begin || x.n_tiles != w.n_tiles) return -4;
+        const int lo = k * P.shape.tile_cap;
+        std::vector<float> img((size_t)P.shape.tile_cap + P.shape.rows_cap, 0.0f);
+        std::vector<char> set(img.size(), 0);
+        for (int i = lo; i < std::min(n, lo + P.shape.tile_cap); ++i) img[(size_t)(i - lo)] = vdend[i], set[(size_t)(i - lo)] = 1;
+        const int own = cs > 1 ? P.shape.tile_cap + (x.tile_begin & 3) : x.tile_begin;
+        if (cs > 1)
+          for (int r = 0; r < x.n_tiles; ++r) {
+            if ((size_t)(own + r) >= img.size()) return -4;
+            img[(size_t)(own + r)] = vdend[x.tile_begin + r];
+            set[(size_t)(own + r)] = 1;
+          }
+        part[(size_t)k].assign((size_t)P.shape.max_slots, 0.0f);
+        const int* wt = P.probes.data() + x.pad0;
+        if (wt[0] != 0 || wt[kStreamWarps] != x.n_groups) return -5;
+        for (int q = 0; q < kStreamWarps; ++q)
+          if (wt[q] > wt[q + 1]) return -5;
+        for (int gi = 0; gi < x.n_groups; ++gi) {
+          const int2_t d = P.gdesc[(size_t)x.group_begin + gi];
+          for (int kk = 0; kk < d.y * 4; ++kk) {
+            unsigned bank_words[32];
+            int bank_n[32] = {0}, worst = 1;
+            for (int l = 0; l < 32; ++l) {
+              const int64_t desc = (uint32_t)P.gcol[((size_t)x.group_begin + gi) * 32 + l];
+              const int row = (int)(desc & 0xffff), slot = (int)(desc >> 16);
+              if (row >= std::max(1, x.n_tiles) || slot >= P.shape.max_slots) return -6;
+              const size_t pairs = (size_t)d.y / 2;
+              const size_t at = (size_t)d.x * 128 + ((size_t)kk < pairs * 8 ? (size_t)(kk / 8) * 256 + l * 8 + kk % 8
+                                                                           : pairs * 256 + l * 4 + kk % 4);
+              const size_t ag = (size_t)d.x * 128 + (size_t)(kk / 4) * 128 + l * 4 + kk % 4;
+              if (at >= P.edges.size() || (g && ag >= P.edge_g.size())) return -8;
+              const unsigned o = P.edges[at];
+              if (o >= img.size() || !set[o]) return -7;
+              const float V = img[(size_t)(own + row)] - img[o];
+              part[(size_t)k][(size_t)slot] += (g ? P.edge_g[ag] : 1.0f) * fexp(V) * V;
+              if (bank_n[o & 31] == 0 || bank_words[o & 31] != o) bank_n[o & 31]++;
+              bank_words[o & 31] = o;
+              worst = std::max(worst, bank_n[o & 31]);
+            }
+            gather_waves += worst;
+            gathers += 1;
+          }
+          groups += 1;
+        }
+      }
+      for (int r = 0; r < w.n_tiles; ++r) {
+        const int c = w.tile_begin + r;
+        float acc = 0.0f;
+        for (int k = 0; k < cs; ++k) {
+          const CellSlots s = P.cell_slots[(size_t)c * cs + k];
+          if (s.begin < 0 || s.count < 0 || s.begin + s.count > P.cta[(size_t)b0 + k].n_slots) return -6;
+          for (int q = 0; q < s.count; ++q) acc += part[(size_t)k][(size_t)(s.begin + q)];
+        }
+        ic_out[c] = g ? acc : acc * g_uniform;
+      }
+      continue;
+    }
     if (P.shape.gather == 3) {
       const int wpr = w.pad0;
       for (int t = 0; t < w.n_cells; ++t) {
@@ -1433,7 +1872,7 @@ extern "C" int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t*
     info[0] = P.grid;
     info[1] = P.shape.gather ? 1 + P.shape.gather : P.shape.stamped;
     info[2] = P.shape.stamped ? (int64_t)!P.perm.empty() : (int64_t)P.tiles.size();
-    info[3] = P.shape.stamped ? groups : (int64_t)P.chunks.size();
+    info[3] = P.shape.stamped || P.shape.gather == 4 ? groups : (int64_t)P.chunks.size();
     info[4] = P.shape.max_slots;
     info[5] = (int64_t)P.smem_bytes;
     info[6] = probes;

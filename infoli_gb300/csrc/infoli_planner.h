@@ -37,6 +37,10 @@ struct PlanInput {
   int sync_mode = 0;               // kSyncAuto / kSyncBarrier / kSyncStamped
   int reorder = 1;                 // stamped plans: try a locality-preserving cell order
   const int* cta_starts = nullptr; // optional CTA cell ranges (grid + 1 entries; internal)
+  int no_stream = 0;               // auto mode: no stream plans
+  // stream plans over sender shares: most co-resident CTAs in clusters of 2
+  // and of 4 (0: none, -1: grid_max, rounded down to whole clusters)
+  int cluster_ctas[2] = {-1, -1};
 };
 
 // Locality reordering is tried for stamped plans whose largest window is at
@@ -46,7 +50,8 @@ struct PlanInput {
 enum { kReorderMinWindowRatio = 4, kReorderIters = 160 };
 constexpr int64_t kReorderMaxEdges = 32ll << 20;
 
-enum { kSyncAuto = 0, kSyncBarrier = 1, kSyncStamped = 2, kSyncGather = 3, kSyncTiledGather = 4, kSyncBits = 5 };
+enum { kSyncAuto = 0, kSyncBarrier = 1, kSyncStamped = 2, kSyncGather = 3, kSyncTiledGather = 4, kSyncBits = 5,
+       kSyncStream = 6 };
 
 // Auto mode picks a bitmask plan (uniform g only) over tile/gather plans when
 // the density is at least 1 / kBitsMinDensityInv.
@@ -55,6 +60,18 @@ enum { kBitsMinDensityInv = 16 };
 // Auto mode picks a tiled gather plan over a barrier plan when the mean degree
 // is at most this (rows too short to fill a warp per chunk once split by tiles).
 enum { kGatherMaxMeanDegree = 384 };
+
+// Stream plans are for edges that do not stay on chip.  Auto mode takes them
+//   - with the whole V_dend array as one share (up to about 50,000 cells), except
+//     for one conductance at a density of 1 / kStreamMaxDensityInv or more,
+//     where a bit per pair is shorter than 16 bits per edge by more than the
+//     walk of the bits costs;
+//   - with the senders shared by a cluster's CTAs for rows of at least
+//     kStreamMinDegree edges on average (shorter rows spend more on the
+//     exchange of partial sums than the tiles cost), unless they are dense
+//     with one conductance (bitmask plans).
+enum { kStreamMinDegree = 16 };
+constexpr double kStreamMaxDensity = 0.45;
 
 struct Plan {
   int grid = 0, threads = 0, tile_cap = 0, nbuf = 1, max_slots = 0;
