@@ -14,10 +14,11 @@
 // static __device__ array of fixed size (kNoAllocMaxCells cells, about 0.5
 // MiB), which every GPU that loads the library keeps until the process exits.
 //
-// The kernel is a variant of the persistent step kernel: one thread per cell
-// runs the coupling sum straight from the CSR lists (gathering V_dend from
-// the shared scratch buffer) and the fused compartment update with
-// register-resident state, with one grid barrier per step.  The barrier
+// The kernel walks the CSR lists as they are (nothing is planned, nothing is
+// kept between calls), a group of 4 to 32 lanes per receiver, with V_dend read
+// from the shared scratch buffer through L2; the cells are spread over up to
+// one CTA per SM, their state in shared memory, the gate units over all warps
+// and run while the step's grid barrier completes.  The barrier
 // counter is 64-bit, so one call may run any number of steps without it
 // wrapping.  Malformed topology (a sender id outside [0, n), a NULL column
 // array with edges, a decreasing or negative row_ptr) is recorded in the
@@ -26,6 +27,7 @@
 // against the length of the caller's arrays and is the caller's contract.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstdint>
 #include <cstring>
@@ -35,12 +37,18 @@
 #include "infoli_cell.cuh"
 #include "infoli_internal.h"
 #include "infoli_ptx.cuh"
+#include "infoli_step.cuh"
 
 namespace infoli {
 namespace {
 
 constexpr int kNoAllocMaxCells = 65536;  // largest network the static scratch holds
 constexpr int kNoAllocBlock = 512;
+constexpr int kNoAllocWarps = kNoAllocBlock / 32;
+// A CTA takes at least a warp's worth of cells (a small network stays on few
+// SMs, with a cheaper grid barrier) and at most its threads.
+constexpr int kNoAllocMinCells = 32;
+constexpr int kNoAllocLoads = 8;  // V_dend loads in flight per lane
 constexpr int kMaxDevices = 64;
 
 // Scratch layout: [0, 256) 64-bit barrier counter at 0 + error word at 64
@@ -50,8 +58,6 @@ constexpr int kErrBarrier = 1, kErrSender = 2, kErrRowPtr = 3;
 constexpr size_t kCtlBytes = 256;
 constexpr size_t kScratchBytes = kCtlBytes + 2 * sizeof(float) * (size_t)kNoAllocMaxCells;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
-
-constexpr float kNegLog2eOver100 = -0.014426950408889634f;  // -log2(e)/100
 
 struct NoAllocArgs {
   ModelParams P;
@@ -68,128 +74,167 @@ struct NoAllocArgs {
   unsigned long long timeout_ns;
 };
 
-__device__ __forceinline__ bool noalloc_barrier(const NoAllocArgs& a, unsigned long long* bar, int* err,
-                                                unsigned long long target) {
-  __shared__ int s_abort;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_abort = 0;
-    __threadfence();
-    red_release_gpu_add_u64(bar, 1ull);
-    const uint64_t t0 = globaltimer_ns();
-    while (ld_acquire_gpu_u64(bar) < target) {
-      if (ld_relaxed_gpu(err) != 0 || globaltimer_ns() - t0 > a.timeout_ns) {
-        atomicCAS(err, 0, kErrBarrier);
-        s_abort = 1;
-        break;
-      }
-    }
-  }
-  __syncthreads();
-  return s_abort == 0;
+// Shared memory of a CTA of `cap` cells: V_dend, V_soma, V_axon, nine unit
+// currents, the gap-junction current, the gate state, Ca2+, the edge ranges.
+enum { kNoAllocCellFloats = 13 };
+__host__ __device__ inline size_t noalloc_smem(int cap) {
+  return (size_t)cap * ((kNoAllocCellFloats + kGateFloats) * sizeof(float) + sizeof(double) + 2 * sizeof(int64_t));
 }
 
-__global__ void __launch_bounds__(kNoAllocBlock, 1) noalloc_step_kernel(const __grid_constant__ NoAllocArgs a) {
+// Sum over the edges of one receiver of g f(V) V by `width` lanes (a power of
+// two; `sub` is this lane's place among them), in all of them.
+__device__ __forceinline__ float noalloc_row(const NoAllocArgs& a, const float* vcur, int64_t e0, int64_t e1, float vc,
+                                             int sub, int width, int* err) {
+  float acc = 0.0f;
+  for (int64_t e = e0 + sub; e < e1; e += (int64_t)kNoAllocLoads * width) {
+    int s[kNoAllocLoads];
+    float vs[kNoAllocLoads], gg[kNoAllocLoads];
+#pragma unroll
+    for (int u = 0; u < kNoAllocLoads; ++u) {
+      const int64_t k = e + (int64_t)u * width;
+      s[u] = k < e1 ? __ldg(a.col + k) : -1;
+      gg[u] = a.g && k < e1 ? __ldg(a.g + k) : 1.0f;
+      if (k < e1 && (unsigned)s[u] >= (unsigned)a.n) {  // malformed topology: recorded, never read outside the buffer
+        atomicCAS(err, 0, kErrSender);
+        s[u] = -1;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kNoAllocLoads; ++u)
+      vs[u] = s[u] >= 0 ? __ldcg(vcur + s[u]) : vc;  // L2: written by other CTAs this launch
+#pragma unroll
+    for (int u = 0; u < kNoAllocLoads; ++u) {
+      const float V = vc - vs[u];
+      const float f = fmaf(0.8f, ex2_approx((V * V) * kNegLog2eOver100), 0.2f);
+      if (s[u] >= 0) acc += (gg[u] * f) * V;
+    }
+  }
+  for (int o = width >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
+
+// What bounds a step: the grid barrier and the L2 round trips to the senders'
+// V_dend, so a CTA has few cells and every lane eight loads in flight.
+// 5,003 cells x 60 senders, per-edge g, 200 steps: 1,264 us per call
+// against 5,180 with one thread per cell on 10 CTAs (the edges of a row one
+// after another, the gate units after them).
+__global__ void __launch_bounds__(kNoAllocBlock, 2) noalloc_step_kernel(const __grid_constant__ NoAllocArgs a,
+                                                                         int cells_per_cta, int cap) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_abort;
+  double* sCa = reinterpret_cast<double*>(smem_raw);
+  int64_t* sE0 = reinterpret_cast<int64_t*>(sCa + cap);
+  int64_t* sE1 = sE0 + cap;
+  float* sV = reinterpret_cast<float*>(sE1 + cap);
+  float* sI = sV + 3 * cap;   // nine unit currents
+  float* sIc = sI + 9 * cap;  // gap-junction current
+  float* sG = sIc + cap;      // gate state, field f of cell c at sG[f * cap + c]
   unsigned long long* bar = reinterpret_cast<unsigned long long*>(a.scratch);
   int* err = reinterpret_cast<int*>(a.scratch + 64);
   float* vd[2] = {reinterpret_cast<float*>(a.scratch + kCtlBytes),
                   reinterpret_cast<float*>(a.scratch + kCtlBytes) + kNoAllocMaxCells};
-  const int n = a.n;
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool own = c < n;
-  const size_t N = (size_t)n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int c0 = blockIdx.x * cells_per_cta;
+  const int nc = min(cells_per_cta, a.n - c0);
+  const bool own = tid < nc;
+  const size_t N = (size_t)a.n, c = (size_t)c0 + tid;
 
-  // reference state order: V_dend, Calcium_r, Potassium_s, Hcurrent_q,
-  // Ca2Plus, I_CaH, g_CaL, V_soma, Sodium_m, Sodium_h, Potassium_n,
-  // Potassium_p, Potassium_x_s, Calcium_k, Calcium_l, V_axon, Sodium_m_a,
-  // Sodium_h_a, Potassium_x_a
-  Volts v{};
-  Gates gs{};
+  // state order of the ABI's arrays, by device field
+  const int field[] = {-1, F_R, F_S, F_Q, -2, F_ICAH, F_GCAL, -3, F_M, F_H, F_N, F_P, F_XS, F_K, F_L, -4, F_MA, F_HA, F_XA};
   if (own) {
     const float* s = a.state;
-    v.Vd = s[0 * N + c];
-    gs.r = s[1 * N + c];
-    gs.s = s[2 * N + c];
-    gs.q = s[3 * N + c];
-    gs.Ca = (double)s[4 * N + c];
-    gs.ICaH = s[5 * N + c];
-    gs.gCaL = s[6 * N + c];
-    v.Vs = s[7 * N + c];
-    gs.m = s[8 * N + c];
-    gs.h = s[9 * N + c];
-    gs.n = s[10 * N + c];
-    gs.p = s[11 * N + c];
-    gs.xs = s[12 * N + c];
-    gs.k = s[13 * N + c];
-    gs.l = s[14 * N + c];
-    v.Va = s[15 * N + c];
-    gs.ma = s[16 * N + c];
-    gs.ha = s[17 * N + c];
-    gs.xa = s[18 * N + c];
-    vd[a.step0 & 1][c] = v.Vd;
-  }
-  unsigned long long target = gridDim.x;
-  bool ok = noalloc_barrier(a, bar, err, target);
-  // this thread's edge range, checked once (a bad row is recorded and skipped)
-  int64_t e_begin = 0, e_end = 0;
-  if (own) {
-    e_begin = a.row_ptr[c];
-    e_end = a.row_ptr[c + 1];
-    if (e_begin < 0 || e_end < e_begin) {
+    sV[tid] = s[0 * N + c];
+    sV[cap + tid] = s[7 * N + c];
+    sV[2 * cap + tid] = s[15 * N + c];
+    sCa[tid] = (double)s[4 * N + c];
+#pragma unroll
+    for (int k = 0; k < INFOLI_NSTATE; ++k)
+      if (field[k] >= 0) sG[field[k] * cap + tid] = s[k * N + c];
+    vd[a.step0 & 1][c] = sV[tid];
+    // this cell's edge range, checked once (a bad row is recorded and skipped)
+    int64_t e0 = a.row_ptr[c], e1 = a.row_ptr[c + 1];
+    if (e0 < 0 || e1 < e0) {
       atomicCAS(err, 0, kErrRowPtr);
-      e_end = e_begin;
-    } else if (e_end > e_begin && a.col == nullptr) {
+      e1 = e0 = 0;
+    } else if (e1 > e0 && a.col == nullptr) {
       atomicCAS(err, 0, kErrSender);
-      e_end = e_begin;
+      e1 = e0;
     }
+    sE0[tid] = e0;
+    sE1[tid] = e1;
   }
+  if (tid == 0) s_abort = 0;
+  // lanes per receiver: as many as the CTA has for each of its cells, at
+  // least 4 (rows then read in 16-byte pieces)
+  int width = 4;
+  while (width < 32 && width * 2 * nc <= kNoAllocBlock) width *= 2;
+  const int groups = kNoAllocBlock / width, sub = tid % width;
   const VoltCoef vk = volt_coef(a.P);
-  for (int t = 0; t < a.n_steps && ok; ++t) {
+  unsigned long long target = 0;
+  __syncthreads();
+  for (int t = 0; t < a.n_steps; ++t) {
     const int step = a.step0 + t;
-    if (own) {
-      const float* vcur = vd[step & 1];
-      float acc = 0.0f;
-      for (int64_t e = e_begin; e < e_end; ++e) {
-        const int s = a.col[e];
-        if ((unsigned)s >= (unsigned)n) {  // malformed topology: record, never read outside the buffer
-          atomicCAS(err, 0, kErrSender);
-          continue;
-        }
-        const float V = v.Vd - __ldcg(vcur + s);  // L2: written by other CTAs this launch
-        const float f = fmaf(0.8f, ex2_approx((V * V) * kNegLog2eOver100), 0.2f);
-        acc += a.g ? (a.g[e] * f) * V : f * V;
-      }
-      const float ic = a.g ? acc : acc * a.g_uniform;
-      const float iapp = (step >= a.pulse_start && step < a.pulse_end) ? a.pulse_amp : 0.0f;
-      Currents cur;
-      run_units(a.P, 0xffu, v, gs, cur);
-      voltage_step(a.P, vk, v, cur, ic, iapp);
-      vd[(step + 1) & 1][c] = v.Vd;
-      if (a.trace_axon) a.trace_axon[(size_t)t * N + c] = v.Va;
+    // V^step is written: arrive, run the gate units (own voltages only), wait
+    if (tid == 0) {
+      __threadfence();
+      red_release_gpu_add_u64(bar, 1ull);
     }
     target += gridDim.x;
-    ok = noalloc_barrier(a, bar, err, target);
+    const int items = ((nc + 31) >> 5) * kUnits;
+    for (int it = warp; it < items; it += kNoAllocWarps) {
+      const int k = (it / kUnits) * 32 + lane;
+      const unsigned m = 1u << (it % kUnits);
+      if (k < nc) {
+        const Volts u = {sV[k], sV[cap + k], sV[2 * cap + k]};
+        Currents cur;
+        Gates gs = load_gates(sG, sCa, cap, k, m);
+        run_units(a.P, m, u, gs, cur);
+        store_gates(sG, sCa, cap, k, m, gs);
+        store_currents(sI, cap, k, m, cur);
+      }
+    }
+    if (tid == kNoAllocBlock - 32) {
+      const uint64_t t0 = globaltimer_ns();
+      while (ld_acquire_gpu_u64(bar) < target) {
+        if (ld_relaxed_gpu(err) != 0 || globaltimer_ns() - t0 > a.timeout_ns) {
+          atomicCAS(err, 0, kErrBarrier);
+          s_abort = 1;
+          break;
+        }
+      }
+    }
+    __syncthreads();
+    if (s_abort) break;
+    const float* vcur = vd[step & 1];
+    for (int k0 = 0; k0 < nc; k0 += groups) {  // whole warps, with or without a receiver
+      const int k = k0 + tid / width;
+      const bool row = k < nc;
+      const float sum = noalloc_row(a, vcur, row ? sE0[k] : 0, row ? sE1[k] : 0, row ? sV[k] : 0.0f, sub, width, err);
+      if (row && sub == 0) sIc[k] = sum;
+    }
+    __syncthreads();
+    if (own) {
+      const float ic = a.g ? sIc[tid] : sIc[tid] * a.g_uniform;
+      const float iapp = (step >= a.pulse_start && step < a.pulse_end) ? a.pulse_amp : 0.0f;
+      Volts v = {sV[tid], sV[cap + tid], sV[2 * cap + tid]};
+      voltage_step(a.P, vk, v, load_currents(sI, cap, tid), ic, iapp);
+      vd[(step + 1) & 1][c] = v.Vd;
+      sV[tid] = v.Vd;
+      sV[cap + tid] = v.Vs;
+      sV[2 * cap + tid] = v.Va;
+      if (a.trace_axon) a.trace_axon[(size_t)t * N + c] = v.Va;
+    }
+    __syncthreads();
   }
   if (own) {
     float* s = a.state;
-    s[0 * N + c] = v.Vd;
-    s[1 * N + c] = gs.r;
-    s[2 * N + c] = gs.s;
-    s[3 * N + c] = gs.q;
-    s[4 * N + c] = (float)gs.Ca;
-    s[5 * N + c] = gs.ICaH;
-    s[7 * N + c] = v.Vs;
-    s[8 * N + c] = gs.m;
-    s[9 * N + c] = gs.h;
-    s[10 * N + c] = gs.n;
-    s[11 * N + c] = gs.p;
-    s[12 * N + c] = gs.xs;
-    s[13 * N + c] = gs.k;
-    s[14 * N + c] = gs.l;
-    s[15 * N + c] = v.Va;
-    s[16 * N + c] = gs.ma;
-    s[17 * N + c] = gs.ha;
-    s[18 * N + c] = gs.xa;
+    s[0 * N + c] = sV[tid];
+    s[7 * N + c] = sV[cap + tid];
+    s[15 * N + c] = sV[2 * cap + tid];
+    s[4 * N + c] = (float)sCa[tid];
+#pragma unroll
+    for (int k = 0; k < INFOLI_NSTATE; ++k)
+      if (field[k] >= 0 && field[k] != F_GCAL) s[k * N + c] = sG[field[k] * cap + tid];
   }
 }
 
@@ -234,9 +279,17 @@ extern "C" int infoli_run_noalloc(const float* params, int n_cells, const int64_
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess)
     return infoli__fail(INFOLI_ERR_CUDA, "run_noalloc: cudaDeviceGetAttribute: %s", cudaGetErrorString(e));
-  const int grid = (n_cells + kNoAllocBlock - 1) / kNoAllocBlock;
+  const int per_cta = std::max(kNoAllocMinCells, (n_cells + nsm - 1) / nsm);
+  const int grid = (n_cells + per_cta - 1) / per_cta, cap = (per_cta + 31) & ~31;
+  const size_t smem = noalloc_smem(cap);
+  if (per_cta > kNoAllocBlock)
+    return infoli__fail(INFOLI_ERR_CAPACITY, "run_noalloc: %d cells need more than one thread per cell on %d SMs",
+                        n_cells, nsm);
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_step_kernel, kNoAllocBlock, 0);
+  e = cudaFuncSetAttribute(noalloc_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)noalloc_smem(kNoAllocBlock));
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, noalloc_step_kernel, kNoAllocBlock, smem);
   if (e != cudaSuccess)
     return infoli__fail(INFOLI_ERR_CUDA, "run_noalloc: occupancy query: %s", cudaGetErrorString(e));
   if (grid > per_sm * nsm)
@@ -263,8 +316,9 @@ extern "C" int infoli_run_noalloc(const float* params, int n_cells, const int64_
   // the barrier counter and the error word must start at zero
   e = cudaMemsetAsync(scratch, 0, kCtlBytes, s);
   if (e != cudaSuccess) return infoli__fail(INFOLI_ERR_CUDA, "run_noalloc: cudaMemsetAsync: %s", cudaGetErrorString(e));
-  void* args[] = {&a};
-  e = cudaLaunchCooperativeKernel((const void*)noalloc_step_kernel, dim3(grid), dim3(kNoAllocBlock), args, 0, s);
+  int cells = per_cta, cap_arg = cap;
+  void* args[] = {&a, &cells, &cap_arg};
+  e = cudaLaunchCooperativeKernel((const void*)noalloc_step_kernel, dim3(grid), dim3(kNoAllocBlock), args, smem, s);
   if (e != cudaSuccess) return infoli__fail(INFOLI_ERR_CUDA, "run_noalloc: launch: %s", cudaGetErrorString(e));
   // the error word comes back on the caller's stream: a plain cudaMemcpy would
   // go to the legacy default stream and wait for every blocking stream

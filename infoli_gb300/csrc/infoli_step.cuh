@@ -68,6 +68,35 @@ __device__ __forceinline__ void store_gates(float* sG, double* sCa, int cap, int
   if (mask & 0x80u) sG[F_XA * cap + r] = g.xa;
 }
 
+// Unit currents of local cell r in shared memory (current k at sI[k * cap + r]).
+__device__ __forceinline__ void store_currents(float* sI, int cap, int r, unsigned mask, const Currents& c) {
+  if (mask & 0x01u) sI[0 * cap + r] = c.I_h;
+  if (mask & 0x02u) {
+    sI[1 * cap + r] = c.I_CaH;
+    sI[2 * cap + r] = c.I_K_Ca;
+  }
+  if (mask & 0x04u) sI[3 * cap + r] = c.I_CaL;
+  if (mask & 0x08u) sI[4 * cap + r] = c.I_Na_s;
+  if (mask & 0x10u) sI[5 * cap + r] = c.I_Kdr_s;
+  if (mask & 0x20u) sI[6 * cap + r] = c.I_K_s;
+  if (mask & 0x40u) sI[7 * cap + r] = c.I_Na_a;
+  if (mask & 0x80u) sI[8 * cap + r] = c.I_K_a;
+}
+
+__device__ __forceinline__ Currents load_currents(const float* sI, int cap, int r) {
+  Currents c;
+  c.I_h = sI[0 * cap + r];
+  c.I_CaH = sI[1 * cap + r];
+  c.I_K_Ca = sI[2 * cap + r];
+  c.I_CaL = sI[3 * cap + r];
+  c.I_Na_s = sI[4 * cap + r];
+  c.I_Kdr_s = sI[5 * cap + r];
+  c.I_K_s = sI[6 * cap + r];
+  c.I_Na_a = sI[7 * cap + r];
+  c.I_K_a = sI[8 * cap + r];
+  return c;
+}
+
 // Trace rows fall on the steps that are multiples of trace_every.  A
 // countdown per thread replaces a per-step integer division (it sat on the
 // voltage threads' path every step).
