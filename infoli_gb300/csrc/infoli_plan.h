@@ -128,6 +128,7 @@ typedef struct {
   int cluster;     // stream plan: CTAs per cluster (sender shares)
   int rows_cap;    // stream plan with cluster > 1: staged V_dend of the cluster's receivers
   int split_units; // stream plan: gate units over all warps, gate state in shared memory
+  int byte_off;    // stream plan: entries are byte offsets (the staged floats fit in 64 KB), else float indices
 } SmemShape;
 
 static inline INFOLI_HD size_t tgather_smem_bytes(SmemShape s) {
@@ -207,16 +208,23 @@ static inline INFOLI_HD SmemLayout smem_layout(SmemShape s) {
 // lies at (first * 128) + (k / 8) * 256 + l * 8 + k % 8 in the edge array while
 // whole 8-entry pairs last (16-byte loads), the odd quad after them at
 // + l * 4 + k % 4; its conductance at (first * 128) + (k / 4) * 128 + l * 4 + k % 4.
-// An entry is the index of a float from the start of dynamic shared memory;
-// padding entries name the row's own V_dend (a term of exactly 0).  Partial
+// An entry is the place of a float from the start of dynamic shared memory, in
+// bytes where all of them lie within 64 KB (one instruction less per entry),
+// else in floats; padding entries name the row's own V_dend (a term of exactly 0).  Partial
 // sums: cell_slots[cell * cluster + k] = its slots in CTA k of the cluster.
 //   [share of V_dend][cluster > 1: the rows' V_dend][partial sums, with KAHAN
-//   as (sum, compensation) pairs][mbarrier][split_units: 12 cell arrays, Ca2+,
-//   gate state]
-enum { kStreamThreads = 1024, kStreamWarps = 32, kStreamMaxCluster = 4, kStreamCellArrays = 12 };
+//   as (sum, compensation) pairs][mbarrier][split_units: 16 cell arrays (three
+//   voltages, nine currents, the first half of the voltage step), Ca2+, gate
+//   state]
+enum { kStreamThreads = 1024, kStreamWarps = 32, kStreamMaxCluster = 4, kStreamCellArrays = 16 };
 typedef struct {
   size_t rows, part, mbar, cells, gca, gates, total;
 } StreamLayout;
+
+// Entries per lane by which groups are padded: the kernel's block (16, with
+// conductances 8), or a quad after blocks of 8 where the cells' gate state
+// leaves few registers.
+static inline INFOLI_HD int stream_unit(SmemShape s) { return !s.split_units ? 4 : s.edge_g ? 8 : 16; }
 
 static inline INFOLI_HD StreamLayout stream_layout(SmemShape s) {
   StreamLayout L;

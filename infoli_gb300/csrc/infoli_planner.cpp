@@ -633,7 +633,8 @@ struct StreamCut {
 // the write of 32 partial sums), kSlotCost: a slot's in the owner's sum.
 constexpr double kStreamGroupCost = 8.0, kStreamSlotCost = 0.4;
 
-StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, std::vector<int>& hist) {
+// A group's length is a multiple of `unit` entries.
+StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, int unit, std::vector<int>& hist) {
   StreamCut c;
   c.len = len;
   hist.assign((size_t)std::min(len, max_len) + 2, 0);
@@ -652,7 +653,7 @@ StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, st
     int best = 0;
     for (int w = 1; w < kStreamWarps; ++w)
       if (load[w] < load[best]) best = w;
-    load[best] += ((l + 3) & ~3) + kStreamGroupCost;
+    load[best] += (l + unit - 1) / unit * unit + kStreamGroupCost;
   };
   for (int l = (int)hist.size() - 1; l > 0; --l) {
     int left = hist[(size_t)l];
@@ -714,6 +715,7 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     *err = "make_plan: the senders' shares do not fit in shared memory";
     return false;
   }
+  sh.byte_off = (size_t)(sh.tile_cap + sh.rows_cap) * sizeof(float) <= 65536;
   const int cs = sh.cluster, share = sh.tile_cap;
   const int nclus = (int)starts.size() - 1, ctas = nclus * cs;
   sh.cells_cap = 32;
@@ -728,6 +730,8 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     sh.split_units = 1;
     if (stream_layout(sh).total > in.smem_budget) sh.split_units = 0;
   }
+  // groups are whole blocks of the entries that the kernel takes at a time
+  const int unit = stream_unit(sh);
   sh.max_slots = 0;
   const int slots_cap = (int)std::min<size_t>(65535, (in.smem_budget - stream_layout(sh).total) / slot_bytes);
 
@@ -772,12 +776,18 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
       cnt[(size_t)r] = (int)(at[(size_t)r + 1] - at[(size_t)r]);
       max_len = std::max(max_len, cnt[(size_t)r]);
     }
-    // lane-chunk length: the cheapest of a few whose slots fit
-    std::vector<int> hist;
+    // lane-chunk length: the cheapest of those that give the warps about 1 to 4
+    // groups each, and of a few fixed ones, whose slots fit
+    std::vector<int> hist, lens;
+    for (int k = 1; k <= 4; ++k)
+      for (double f : {1.0, 1.02, 1.04, 1.06, 1.08, 1.11, 1.15, 1.2, 1.3})
+        lens.push_back(std::max(16, (int)std::ceil(f * (double)idx.size() / (1024.0 * k))));
+    for (int len : {16, 24, 32, 48, 64, 96, 128, 256, 512, 1024, 4096, 1 << 30}) lens.push_back(len);
+    std::sort(lens.begin(), lens.end());
+    lens.erase(std::unique(lens.begin(), lens.end()), lens.end());
     StreamCut best;
-    for (int len : {16, 20, 24, 28, 32, 40, 48, 56, 64, 80, 96, 112, 128, 160, 192, 224, 256, 320, 384, 512, 768, 1024,
-                    2048, 4096, 1 << 30}) {
-      const StreamCut c = stream_cut_cost(cnt, len, max_len, hist);
+    for (int len : lens) {
+      const StreamCut c = stream_cut_cost(cnt, len, max_len, unit, hist);
       if (c.slots < slots_cap && (best.len == 0 || c.cost < best.cost)) best = c;
       if (len >= max_len) break;
     }
@@ -813,29 +823,34 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
         int w = 0;
         for (int q = 1; q < kStreamWarps; ++q)
           if (load[q] < load[w]) w = q;
-        load[w] += ((pc[(size_t)g * 32].len + 3) & ~3) + kStreamGroupCost;
+        load[w] += (pc[(size_t)g * 32].len + unit - 1) / unit * unit + kStreamGroupCost;
         of_warp[(size_t)g] = w;
       }
     }
     std::vector<int> next;
     std::vector<int> head(32 * 32);
+    std::vector<uint16_t> count(32 * 32);
     int placed = 0;
     for (int w = 0; w < kStreamWarps; ++w) {
       L.warp[w] = placed;
       for (int g = 0; g < ng; ++g) {
         if (of_warp[(size_t)g] != w) continue;
         ++placed;
-        const int quads = (pc[(size_t)g * 32].len + 3) / 4, pairs = quads / 2, len = quads * 4;
+        const int quads = (pc[(size_t)g * 32].len + unit - 1) / unit * (unit / 4), pairs = quads / 2, len = quads * 4;
         const size_t base = L.ent.size();
         L.gdesc.push_back(int2_t{(int)(base / 128), quads});
         L.ent.resize(base + (size_t)quads * 128);
         if (in.g) L.g.resize(base + (size_t)quads * 128);
         // Lanes reading position k of a group should hit different banks: the
         // entries of each lane are bucketed by bank, and position by position
-        // every lane takes one from a bank no other lane has taken, where it
-        // has such an entry left (banks tried from a start that rotates).
+        // every lane takes one from a bank no other lane has taken, the fuller
+        // buckets first, so that all buckets last (tried from a start that
+        // rotates); lanes without such a bank share one taken once where they
+        // can.  Wavefronts per gather: 1.41 for lanes of 132 entries, 1.7 for
+        // 52, 2.2 for 28 (3.5 in any order).
         std::fill(head.begin(), head.end(), -1);
-        unsigned avail[32];
+        std::fill(count.begin(), count.end(), (uint16_t)0);
+        unsigned avail[32], full[32], fuller[32];
         int left[32], pad[32];
         size_t lb[32];
         next.assign((size_t)32 * len, -1);
@@ -855,13 +870,23 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
               const int bank = idx[lb[l] + (size_t)q] & 31;
               next[(size_t)l * len + q] = head[(size_t)l * 32 + bank];
               head[(size_t)l * 32 + bank] = q;
+              ++count[(size_t)l * 32 + bank];
               avail[l] |= 1u << bank;
             }
           }
           L.lane.push_back(desc);
         }
         for (int q = 0; q < len; ++q) {
-          unsigned taken = 0;
+          if (q % 16 == 0)  // which buckets are at or above a lane's average, and well above it
+            for (int l = 0; l < 32; ++l) {
+              const int avg = (left[l] + 31) / 32;
+              full[l] = fuller[l] = 0;
+              for (int bk = 0; bk < 32; ++bk) {
+                full[l] |= (unsigned)(count[(size_t)l * 32 + bk] >= avg) << bk;
+                fuller[l] |= (unsigned)(count[(size_t)l * 32 + bk] > avg) << bk;
+              }
+            }
+          unsigned taken = 0, twice = 0;
           int late[32], nlate = 0;
           int pick[32];
           for (int l = 0; l < 32; ++l) {
@@ -869,13 +894,22 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
             if (left[l] == 0) taken |= 1u << (pad[l] & 31);
           }
           auto take = [&](int l, unsigned cand) {
+            if (cand & fuller[l])
+              cand &= fuller[l];
+            else if (cand & full[l])
+              cand &= full[l];
             const int rot = (l + q) & 31;
             const unsigned c = rot ? (cand >> rot) | (cand << (32 - rot)) : cand;
             const int bank = (__builtin_ctz(c) + rot) & 31;
             int& h = head[(size_t)l * 32 + bank];
             pick[l] = h;
             h = next[(size_t)l * len + h];
-            if (h < 0) avail[l] &= ~(1u << bank);
+            if (--count[(size_t)l * 32 + bank] == 0) {
+              avail[l] &= ~(1u << bank);
+              full[l] &= avail[l];
+              fuller[l] &= avail[l];
+            }
+            twice |= taken & (1u << bank);
             taken |= 1u << bank;
             --left[l];
           };
@@ -888,11 +922,15 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
             else
               late[nlate++] = l;
           }
-          for (int j = 0; j < nlate; ++j) take(late[j], avail[late[j]]);
+          for (int j = 0; j < nlate; ++j) {
+            const int l = late[j];
+            take(l, avail[l] & ~twice ? avail[l] & ~twice : avail[l]);
+          }
           for (int l = 0; l < 32; ++l) {
             const size_t e = q < pairs * 8 ? base + (size_t)(q / 8) * 256 + l * 8 + q % 8
                                            : base + (size_t)pairs * 256 + l * 4 + q % 4;
-            L.ent[e] = pick[l] < 0 ? (uint16_t)pad[l] : idx[lb[l] + (size_t)pick[l]];
+            const unsigned at = pick[l] < 0 ? (unsigned)pad[l] : idx[lb[l] + (size_t)pick[l]];
+            L.ent[e] = (uint16_t)(sh.byte_off ? at * sizeof(float) : at);
             if (in.g)
               L.g[base + (size_t)(q / 4) * 128 + l * 4 + q % 4] = pick[l] < 0 ? 0.0f : gv[lb[l] + (size_t)pick[l]];
           }
@@ -1676,6 +1714,7 @@ extern "C" int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t*
           if (wt[q] > wt[q + 1]) return -5;
         for (int gi = 0; gi < x.n_groups; ++gi) {
           const int2_t d = P.gdesc[(size_t)x.group_begin + gi];
+          if (d.y * 4 % stream_unit(P.shape)) return -5;
           for (int kk = 0; kk < d.y * 4; ++kk) {
             unsigned bank_words[32];
             int bank_n[32] = {0}, worst = 1;
@@ -1688,7 +1727,8 @@ extern "C" int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t*
                                                                            : pairs * 256 + l * 4 + kk % 4);
               const size_t ag = (size_t)d.x * 128 + (size_t)(kk / 4) * 128 + l * 4 + kk % 4;
               if (at >= P.edges.size() || (g && ag >= P.edge_g.size())) return -8;
-              const unsigned o = P.edges[at];
+              if (P.shape.byte_off && P.edges[at] % sizeof(float)) return -7;
+              const unsigned o = P.shape.byte_off ? P.edges[at] / sizeof(float) : P.edges[at];
               if (o >= img.size() || !set[o]) return -7;
               const float V = img[(size_t)(own + row)] - img[o];
               part[(size_t)k][(size_t)slot] += (g ? P.edge_g[ag] : 1.0f) * fexp(V) * V;

@@ -86,26 +86,47 @@ __device__ __forceinline__ float4 ld_streamg(const float4* p, uint64_t pol) {
   return v;
 }
 
-// Four entries of a lane: -(their terms) into nt (two accumulators: entries
-// 0, 2 and 1, 3), in V_dend x kVScale (the exponent is -(dV')^2).
-template <bool EDGE_G>
-__device__ __forceinline__ void stream_quad(const float* sm, uint2 o, float4 g4, float2 nvc2, float2& nt) {
-  const float2 c08 = make_float2(0.8f, 0.8f), c02 = make_float2(0.2f, 0.2f);
-  const unsigned i[4] = {o.x & 0xffffu, o.x >> 16, o.y & 0xffffu, o.y >> 16};
-  const float2 gg[2] = {make_float2(g4.x, g4.y), make_float2(g4.z, g4.w)};
+// N entries of a lane (two per word of o): -(their terms) into nt (two
+// accumulators: even and odd entries), in V_dend x kVScale (the exponent is
+// -(dV')^2).  All gathers first, then the arithmetic in stages: a warp then
+// waits once per block and not once per pair of entries (2.03 against 2.7
+// cycles of an SM per warp and entry in a loop over shared memory without bank
+// conflicts; the SFU and the FMA pipe take about one each).
+template <int N, bool BYTE>
+__device__ __forceinline__ void stream_gather(const float* sm, const uint4* o, float2* x) {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float2 nv = __fadd2_rn(make_float2(sm[i[2 * h]], sm[i[2 * h + 1]]), nvc2);  // -V
-    const float2 sq = __fmul2_rn(nv, nv);
-    const float2 e = make_float2(ex2_approx(-sq.x), ex2_approx(-sq.y));
-    float2 f = __ffma2_rn(c08, e, c02);
-    if (EDGE_G) f = __fmul2_rn(gg[h], f);
-    nt = __ffma2_rn(f, nv, nt);
+  for (int k = 0; k < N / 2; ++k) {
+    const unsigned w = k % 4 == 0 ? o[k / 4].x : k % 4 == 1 ? o[k / 4].y : k % 4 == 2 ? o[k / 4].z : o[k / 4].w;
+    if (BYTE) {
+      const unsigned char* b = reinterpret_cast<const unsigned char*>(sm);
+      x[k] = make_float2(*reinterpret_cast<const float*>(b + (w & 0xffffu)), *reinterpret_cast<const float*>(b + (w >> 16)));
+    } else {
+      x[k] = make_float2(sm[w & 0xffffu], sm[w >> 16]);
+    }
+  }
+}
+
+template <int N, bool EDGE_G>
+__device__ __forceinline__ void stream_terms(float2* x, const float4* g, float2 nvc2, float2& nt) {
+  const float2 c08 = make_float2(0.8f, 0.8f), c02 = make_float2(0.2f, 0.2f);
+#pragma unroll
+  for (int k = 0; k < N / 2; ++k) x[k] = __fadd2_rn(x[k], nvc2);  // -V
+  float2 e[N / 2];
+#pragma unroll
+  for (int k = 0; k < N / 2; ++k) {
+    const float2 sq = __fmul2_rn(x[k], x[k]);
+    e[k] = make_float2(ex2_approx(-sq.x), ex2_approx(-sq.y));
+  }
+#pragma unroll
+  for (int k = 0; k < N / 2; ++k) {
+    float2 f = __ffma2_rn(c08, e[k], c02);
+    if (EDGE_G) f = __fmul2_rn(k % 2 ? make_float2(g[k / 2].z, g[k / 2].w) : make_float2(g[k / 2].x, g[k / 2].y), f);
+    nt = __ffma2_rn(f, x[k], nt);
   }
 }
 
 // Running sum of a lane-chunk, negated.  With KAHAN every block of up to
-// eight entries (summed per accumulator first) is added compensated.
+// sixteen entries (summed per accumulator first) is added compensated.
 template <bool KAHAN>
 struct StreamSum {
   float2 acc = make_float2(-0.0f, -0.0f), cmp = make_float2(0.0f, 0.0f);
@@ -125,62 +146,91 @@ struct StreamSum {
 };
 
 // A warp's groups of lane-chunks, partial sums into `part` (pairs of sum and
-// compensation with KAHAN).
-template <bool KAHAN, bool EDGE_G>
+// compensation with KAHAN), in blocks of N entries per lane (whole blocks
+// only, except with N = 8 a last quad, when QUAD).  The next block's entries
+// are loaded before this one's arithmetic, across groups too, and the first
+// group's before `wait` (the wait for V_dend): no load latency stands between
+// blocks.  G_EARLY: the next conductances as well, where registers allow.
+template <bool KAHAN, bool EDGE_G, bool BYTE, int N, bool QUAD, bool G_EARLY, class Wait>
 __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& w, int warp, int lane, const float* sm,
-                                              const float* rows, float* part, uint64_t pol) {
+                                              const float* rows, float* part, uint64_t pol, Wait wait) {
   const int* wt = a.probes + w.pad0 + warp;
   const int g0 = w.group_begin + __ldg(wt), g1 = w.group_begin + __ldg(wt + 1);
+  const uint4* ent = reinterpret_cast<const uint4*>(a.edges) + lane;
+  const float4* eg = EDGE_G ? reinterpret_cast<const float4*>(a.edge_g) + lane : nullptr;
+  uint4 c[N / 8];
+  float4 gc[EDGE_G ? N / 4 : 1];
+  auto load_c = [&](int quad_row) {
+#pragma unroll
+    for (int i = 0; i < N / 8; ++i) c[i] = ld_stream4(ent + (size_t)quad_row * 16 + i * 32, pol);
+  };
+  auto load_g = [&](int quad_row, float4* d) {
+#pragma unroll
+    for (int i = 0; i < N / 4; ++i) d[i] = ld_streamg(eg + (size_t)(quad_row + i) * 32, pol);
+  };
+  int2 gd = make_int2(0, 0);  // {first quad row, quads per lane}
+  unsigned ld = 0;
+  if (g0 < g1) {
+    gd = __ldg(a.gdesc + g0);
+    ld = (unsigned)__ldg(a.gcol + (size_t)g0 * 32 + lane);
+    if (gd.y >= N / 4) {
+      load_c(gd.x);
+      if (EDGE_G) load_g(gd.x, gc);
+    }
+  }
+  wait();
   for (int g = g0; g < g1; ++g) {
-    const int2 gd = __ldg(a.gdesc + g);  // {first quad row, quads per lane}
-    const unsigned ld = (unsigned)__ldg(a.gcol + (size_t)g * 32 + lane);
-    const uint4* pe = reinterpret_cast<const uint4*>(a.edges) + (size_t)gd.x * 16 + lane;
-    const float4* pg = EDGE_G ? reinterpret_cast<const float4*>(a.edge_g) + (size_t)gd.x * 32 + lane : nullptr;
-    const int np = gd.y >> 1;
-    const bool odd = gd.y & 1;
-    const float4 one = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-    uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
-    float4 ga = one, gb = one;
+    int2 gn = make_int2(0, 0);
+    unsigned ln = 0;
+    if (g + 1 < g1) {
+      gn = __ldg(a.gdesc + g + 1);
+      ln = (unsigned)__ldg(a.gcol + (size_t)(g + 1) * 32 + lane);
+    }
+    const int end = gd.x + gd.y / (N / 4) * (N / 4);
+    const bool odd = QUAD && (gd.y & 1);
     uint2 tail = make_uint2(0, 0);
-    float4 gt = one;
-    if (np > 0) {
-      c0 = ld_stream4(pe, pol);
-      if (EDGE_G) {
-        ga = ld_streamg(pg, pol);
-        gb = ld_streamg(pg + 32, pol);
-      }
-    }
-    if (!EDGE_G && np > 1) c1 = ld_stream4(pe + 32, pol);
-    if (odd) {
-      tail = ld_stream2(reinterpret_cast<const uint2*>(pe - lane + np * 32) + lane, pol);
-      if (EDGE_G) gt = ld_streamg(pg + np * 64, pol);
-    }
+    float4 gt = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     const float nvc = -rows[ld & 0xffffu];
     const float2 nvc2 = make_float2(nvc, nvc);
     StreamSum<KAHAN> s;
-    for (int p = 0; p < np; ++p) {
-      const uint4 c = c0;
-      const float4 g_a = ga, g_b = gb;
-      // the next pair's loads are in flight while this one is computed (two
-      // pairs ahead without conductances)
-      if (EDGE_G) {
-        if (p + 1 < np) {
-          c0 = ld_stream4(pe + (p + 1) * 32, pol);
-          ga = ld_streamg(pg + (p + 1) * 64, pol);
-          gb = ld_streamg(pg + (p + 1) * 64 + 32, pol);
-        }
-      } else {
-        c0 = c1;
-        if (p + 2 < np) c1 = ld_stream4(pe + (p + 2) * 32, pol);
+    auto next_group = [&]() {  // what follows this group's whole blocks
+      if (odd) {
+        tail = ld_stream2(reinterpret_cast<const uint2*>(ent - lane + (size_t)end * 16) + lane, pol);
+        if (EDGE_G) gt = ld_streamg(eg + (size_t)end * 32, pol);
       }
+      if (gn.y >= N / 4) load_c(gn.x);
+    };
+    if (end == gd.x) {
+      next_group();
+      if (EDGE_G && gn.y >= N / 4) load_g(gn.x, gc);
+    }
+    for (int q = gd.x; q < end; q += N / 4) {
+      float2 x[N / 2];
+      stream_gather<N, BYTE>(sm, c, x);
+      const bool more = q + N / 4 < end;
+      const int nq = more ? q + N / 4 : gn.y >= N / 4 ? gn.x : -1;
+      if (more)
+        load_c(q + N / 4);
+      else
+        next_group();
       float2 nt = s.start();
-      stream_quad<EDGE_G>(sm, make_uint2(c.x, c.y), g_a, nvc2, nt);
-      stream_quad<EDGE_G>(sm, make_uint2(c.z, c.w), g_b, nvc2, nt);
+      if (EDGE_G && G_EARLY) {
+        float4 now[N / 4];
+#pragma unroll
+        for (int i = 0; i < N / 4; ++i) now[i] = gc[i];
+        if (nq >= 0) load_g(nq, gc);
+        stream_terms<N, EDGE_G>(x, now, nvc2, nt);
+      } else {
+        stream_terms<N, EDGE_G>(x, gc, nvc2, nt);
+        if (EDGE_G && nq >= 0) load_g(nq, gc);
+      }
       s.add(nt);
     }
     if (odd) {
-      float2 nt = s.start();
-      stream_quad<EDGE_G>(sm, tail, gt, nvc2, nt);
+      float2 x[2], nt = s.start();
+      const uint4 o = make_uint4(tail.x, tail.y, 0u, 0u);
+      stream_gather<4, BYTE>(sm, &o, x);
+      stream_terms<4, EDGE_G>(x, &gt, nvc2, nt);
       s.add(nt);
     }
     const unsigned slot = ld >> 16;
@@ -194,34 +244,54 @@ __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& 
     } else {
       part[slot] = -(s.acc.x + s.acc.y);
     }
+    gd = gn;
+    ld = ln;
   }
 }
 
-// Sum of an owned receiver's partial sums over the cluster's CTAs, in sender
+// Sum of an owned receiver's partial sums over the cluster's CTAs by `width`
+// lanes (`sub`: this lane's place; all lanes of the warp call it), in a fixed
 // order (TwoSum per addition with KAHAN, the errors and compensations applied
-// once).
-template <bool KAHAN>
-__device__ __forceinline__ float combine_stream(const int2* slots, int cs, const float* part) {
+// once).  The first AHEAD CTAs' slot ranges are in `ahead`.  The result is valid in the lanes with sub == 0.
+template <bool KAHAN, int AHEAD>
+__device__ __forceinline__ float combine_stream(const int2* ahead, const int2* slots, bool own, int cs,
+                                                const float* part, int sub, int width) {
   const uint32_t base = smem_u32(part);
-  float s = 0.0f, e = 0.0f, c = 0.0f;
+  float s = 0.0f, e = 0.0f;
+  auto add = [&](float x) {
+    const float t = s + x;
+    const float bp = t - s;
+    e += (s - (t - bp)) + (x - bp);
+    s = t;
+  };
+#pragma unroll 1
   for (int k = 0; k < cs; ++k) {
-    const int2 sl = __ldg(slots + k);
+    int2 sl = ahead[0];
+    if (AHEAD > 1 && k == 1) sl = ahead[AHEAD - 1];
+    if (k >= AHEAD) sl = own ? __ldg(slots + k) : make_int2(0, 0);
     const uint32_t pa = cs > 1 ? peer_addr(base, (unsigned)k) : base;
 #pragma unroll 4
-    for (int q = 0; q < sl.y; ++q) {
+    for (int q = sub; q < sl.y; q += width) {
       if (KAHAN) {
         const float2 p = cs > 1 ? ld_peer2(pa + 8u * (uint32_t)(sl.x + q)) : reinterpret_cast<const float2*>(part)[sl.x + q];
-        const float t = s + p.x;
-        const float bp = t - s;
-        e += (s - (t - bp)) + (p.x - bp);
-        c += p.y;
-        s = t;
+        add(p.x);
+        e -= p.y;
       } else {
         s += cs > 1 ? ld_peer(pa + 4u * (uint32_t)(sl.x + q)) : part[sl.x + q];
       }
     }
   }
-  return KAHAN ? s + (e - c) : s;
+  for (int o = 1; o < width; o <<= 1) {
+    const float s2 = __shfl_down_sync(0xffffffffu, s, o);
+    if (KAHAN) {
+      const float e2 = __shfl_down_sync(0xffffffffu, e, o);
+      add(s2);
+      e += e2;
+    } else {
+      s += s2;
+    }
+  }
+  return KAHAN ? s + e : s;
 }
 
 __device__ __forceinline__ bool stream_wait(const StepArgs& a, uint64_t* bar, unsigned parity, volatile int* s_abort) {
@@ -237,7 +307,7 @@ __device__ __forceinline__ bool stream_wait(const StepArgs& a, uint64_t* bar, un
   return true;
 }
 
-template <bool KAHAN, bool EDGE_G, bool SPLIT>
+template <bool KAHAN, bool EDGE_G, bool SPLIT, bool BYTE>
 __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_abort;
@@ -249,6 +319,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   const int cs = a.shape.cluster, share = a.shape.tile_cap, cap = a.shape.cells_cap;
   float* sV = reinterpret_cast<float*>(smem_raw + L.cells);  // SPLIT: V_dend, V_soma, V_axon, nine currents
   float* sI = sV + 3 * cap;
+  float* sH = sV + 12 * cap;  // SPLIT: VoltHalf of every cell
   double* sCa = reinterpret_cast<double*>(smem_raw + L.gca);
   float* sG = reinterpret_cast<float*>(smem_raw + L.gates);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -260,8 +331,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     return;
   }
   const CtaWork w = a.cta[blockIdx.x];
-  const bool owner = tid < w.n_cells;
-  const int cell = w.cell_begin + tid;
+  // Owned cells: one thread each, or (SPLIT, few cells per CTA) `width` lanes
+  // that add the partial sums together, the first of them the owner; the last
+  // warp, which waits for the grid barrier, owns none then.
+  int width = 1;
+  if (SPLIT)
+    while (width < 8 && width * 2 * w.n_cells <= kStreamThreads - 32) width *= 2;
+  const int r = tid / width, sub = tid % width;
+  const bool mine = r < w.n_cells, owner = mine && sub == 0;
+  const int cell = w.cell_begin + r;
   const long long np = a.n_pad;
   // this CTA's share of V_dend: cells [lo, lo + nshare), and with cluster > 1
   // the cluster's rows (copies of whole 16-byte units)
@@ -286,11 +364,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     v.Vs = st[F_VS * np + cell];
     v.Va = st[F_VA * np + cell];
     if (SPLIT) {
-      for (int f = F_Q; f < F_COUNT; ++f) sG[f * cap + tid] = st[f * np + cell];
-      sCa[tid] = a.ca[cell];
-      sV[tid] = v.Vd;
-      sV[cap + tid] = v.Vs;
-      sV[2 * cap + tid] = v.Va;
+      for (int f = F_Q; f < F_COUNT; ++f) sG[f * cap + r] = st[f * np + cell];
+      sCa[r] = a.ca[cell];
+      sV[r] = v.Vd;
+      sV[cap + r] = v.Vs;
+      sV[2 * cap + r] = v.Va;
     } else {
       g.q = st[F_Q * np + cell];
       g.r = st[F_R * np + cell];
@@ -336,11 +414,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   for (int st = 0; st < a.n_steps; ++st) {
     const int step = a.step0 + st;
     const bool trace_now = tclock.take();
-    // V^step is written (and every thread past a CTA barrier): arrive
-    if (tid == 0) {
-      __threadfence();
-      if ((int)blockIdx.x != a.stall_cta) red_release_gpu_add(a.bar, 1u);
-    }
+    // V^step is written and every thread past a CTA barrier: arrive (the
+    // release covers the CTA's writes)
+    if (producer && (int)blockIdx.x != a.stall_cta) red_release_gpu_add(a.bar, 1u);
     bar_target += gridDim.x;
 
     // ---------------- gate units (own voltages only), first half of the voltage step
@@ -356,17 +432,20 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
           Gates gs = load_gates(sG, sCa, cap, c, m);
           run_units(a.P, m, u, gs, cur);
           store_gates(sG, sCa, cap, c, m, gs);
-          if (m & 0x01u) sI[0 * cap + c] = cur.I_h;
-          if (m & 0x02u) {
-            sI[1 * cap + c] = cur.I_CaH;
-            sI[2 * cap + c] = cur.I_K_Ca;
-          }
-          if (m & 0x04u) sI[3 * cap + c] = cur.I_CaL;
-          if (m & 0x08u) sI[4 * cap + c] = cur.I_Na_s;
-          if (m & 0x10u) sI[5 * cap + c] = cur.I_Kdr_s;
-          if (m & 0x20u) sI[6 * cap + c] = cur.I_K_s;
-          if (m & 0x40u) sI[7 * cap + c] = cur.I_Na_a;
-          if (m & 0x80u) sI[8 * cap + c] = cur.I_K_a;
+          store_currents(sI, cap, c, m, cur);
+        }
+      }
+      __syncwarp();
+      if (warp == kStreamWarps - 1) {
+        asm volatile("bar.arrive 1, %0;" ::"r"((int)kStreamThreads) : "memory");
+      } else {
+        asm volatile("bar.sync 1, %0;" ::"r"((int)kStreamThreads) : "memory");
+        if (owner) {
+          vh = voltage_first(a.P, vk, v, load_currents(sI, cap, r));
+          sH[r] = vh.dend;
+          sH[cap + r] = vh.I_h;
+          sH[2 * cap + r] = vh.Vs;
+          sH[3 * cap + r] = vh.Va;
         }
       }
     } else if (owner) {
@@ -404,9 +483,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     __syncwarp();
 
     // ---------------- coupling
-    if (!stream_wait(a, mbar, (unsigned)st & 1u, &s_abort)) s_abort = 1;
-    mark(1);
-    couple_stream<KAHAN, EDGE_G>(a, w, warp, lane, sm, rows, part, pol);
+    constexpr int kBlockEntries = SPLIT && !EDGE_G ? 16 : 8;
+    couple_stream<KAHAN, EDGE_G, BYTE, kBlockEntries, !SPLIT, SPLIT>(a, w, warp, lane, sm, rows, part, pol, [&]() {
+      if (!stream_wait(a, mbar, (unsigned)st & 1u, &s_abort)) s_abort = 1;
+      mark(1);
+    });
+    // the owners' slot ranges, in flight while the other warps finish
+    int2 slots[SPLIT ? 1 : 2];
+#pragma unroll
+    for (int k = 0; k < (SPLIT ? 1 : 2); ++k)
+      slots[k] = mine && k < cs ? __ldg(a.cell_slots + (size_t)cell * cs + k) : make_int2(0, 0);
     if (cs > 1)
       cluster_sync_all();  // every CTA's partial sums (and abort flags) are there
     else
@@ -414,8 +500,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     mark(2);
 
     // ---------------- owners: the receiver's sum, second half of the voltage step
+    float ic = 0.0f;
+    if (SPLIT || mine)
+      ic = combine_stream<KAHAN, (SPLIT ? 1 : 2)>(slots, a.cell_slots + (size_t)cell * cs, mine, cs, part, sub, width) *
+           kInvVScale;
     if (owner) {
-      float ic = combine_stream<KAHAN>(a.cell_slots + (size_t)cell * cs, cs, part) * kInvVScale;
       if (!EDGE_G) ic *= a.g_uniform;
       const int ls = step + my_off;
       float iapp;
@@ -425,27 +514,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
         iapp = (ls >= my_onset && ls < my_onset + a.stim_dur) ? my_amp : 0.0f;
       else
         iapp = a.stim_table[(size_t)st * np + cell];
-      if (SPLIT) {
-        Currents cur;
-        cur.I_h = sI[0 * cap + tid];
-        cur.I_CaH = sI[1 * cap + tid];
-        cur.I_K_Ca = sI[2 * cap + tid];
-        cur.I_CaL = sI[3 * cap + tid];
-        cur.I_Na_s = sI[4 * cap + tid];
-        cur.I_Kdr_s = sI[5 * cap + tid];
-        cur.I_K_s = sI[6 * cap + tid];
-        cur.I_Na_a = sI[7 * cap + tid];
-        cur.I_K_a = sI[8 * cap + tid];
-        vh = voltage_first(a.P, vk, v, cur);
-      }
+      if (SPLIT) vh = {sH[r], sH[cap + r], sH[2 * cap + r], sH[3 * cap + r]};
       v.Vd = voltage_second(a.P, vk, v.Vd, vh, ic, iapp);
       v.Vs = vh.Vs;
       v.Va = vh.Va;
       a.vds[(step + 1) & 1][cell] = v.Vd * kVScale;
       if (SPLIT) {
-        sV[tid] = v.Vd;
-        sV[cap + tid] = v.Vs;
-        sV[2 * cap + tid] = v.Va;
+        sV[r] = v.Vd;
+        sV[cap + r] = v.Vs;
+        sV[2 * cap + r] = v.Va;
       }
       if (trace_now) {
         float* tr = a.trace + (size_t)row * a.trace_nq * np + cell;
@@ -485,8 +562,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     st[F_VS * np + cell] = v.Vs;
     st[F_VA * np + cell] = v.Va;
     if (SPLIT) {
-      for (int f = F_Q; f < F_COUNT; ++f) st[f * np + cell] = sG[f * cap + tid];
-      a.ca[cell] = sCa[tid];
+      for (int f = F_Q; f < F_COUNT; ++f) st[f * np + cell] = sG[f * cap + r];
+      a.ca[cell] = sCa[r];
     } else {
       st[F_Q * np + cell] = g.q;
       st[F_R * np + cell] = g.r;
@@ -508,12 +585,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   }
 }
 
-const void* stream_fn(bool kahan, bool edge_g, bool split) {
-#define INFOLI_STREAM_FN(K, G) \
-  (split ? (const void*)stream_kernel<K, G, true> : (const void*)stream_kernel<K, G, false>)
-  if (kahan) return edge_g ? INFOLI_STREAM_FN(true, true) : INFOLI_STREAM_FN(true, false);
-  return edge_g ? INFOLI_STREAM_FN(false, true) : INFOLI_STREAM_FN(false, false);
-#undef INFOLI_STREAM_FN
+template <bool K, bool G>
+const void* stream_fn2(bool split, bool byte_off) {
+  if (split) return byte_off ? (const void*)stream_kernel<K, G, true, true> : (const void*)stream_kernel<K, G, true, false>;
+  return byte_off ? (const void*)stream_kernel<K, G, false, true> : (const void*)stream_kernel<K, G, false, false>;
+}
+
+const void* stream_fn(bool kahan, bool edge_g, bool split, bool byte_off) {
+  if (kahan) return edge_g ? stream_fn2<true, true>(split, byte_off) : stream_fn2<true, false>(split, byte_off);
+  return edge_g ? stream_fn2<false, true>(split, byte_off) : stream_fn2<false, false>(split, byte_off);
 }
 
 void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, int cluster, size_t smem,
@@ -537,7 +617,7 @@ void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, i
 
 cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t stream) {
   const size_t smem = stream_layout(a.shape).total;
-  const void* fn = stream_fn(a.shape.kahan != 0, a.edge_g != nullptr, a.shape.split_units != 0);
+  const void* fn = stream_fn(a.shape.kahan != 0, a.edge_g != nullptr, a.shape.split_units != 0, a.shape.byte_off != 0);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg;
@@ -548,7 +628,7 @@ cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t strea
 }
 
 int max_stream_ctas(int cluster, size_t smem) {
-  const void* fn = stream_fn(true, true, false);
+  const void* fn = stream_fn(true, true, false, false);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
