@@ -127,7 +127,7 @@ typedef struct {
                    // senders + progress probes); picks the poll batch size
   int cluster;     // stream plan: CTAs per cluster (sender shares)
   int rows_cap;    // stream plan with cluster > 1: staged V_dend of the cluster's receivers
-  int split_units; // stream plan: gate units over all warps, gate state in shared memory
+  int block;       // stream plan: entries per lane taken at a time (8, or 16 for long lane-chunks)
   int byte_off;    // stream plan: entries are byte offsets (the staged floats fit in 64 KB), else float indices
 } SmemShape;
 
@@ -212,19 +212,12 @@ static inline INFOLI_HD SmemLayout smem_layout(SmemShape s) {
 // bytes where all of them lie within 64 KB (one instruction less per entry),
 // else in floats; padding entries name the row's own V_dend (a term of exactly 0).  Partial
 // sums: cell_slots[cell * cluster + k] = its slots in CTA k of the cluster.
-//   [share of V_dend][cluster > 1: the rows' V_dend][partial sums, with KAHAN
-//   as (sum, compensation) pairs][mbarrier][split_units: 16 cell arrays (three
-//   voltages, nine currents, the first half of the voltage step), Ca2+, gate
-//   state]
-enum { kStreamThreads = 1024, kStreamWarps = 32, kStreamMaxCluster = 4, kStreamCellArrays = 16 };
+//   [share of V_dend][cluster > 1: the rows' V_dend][partial sums][the own
+//   cells' sums by CTA of the cluster][mbarrier]
+enum { kStreamThreads = 1024, kStreamWarps = 32, kStreamMaxCluster = 4 };
 typedef struct {
-  size_t rows, part, mbar, cells, gca, gates, total;
+  size_t rows, part, sums, mbar, total;
 } StreamLayout;
-
-// Entries per lane by which groups are padded: the kernel's block (16, with
-// conductances 8), or a quad after blocks of 8 where the cells' gate state
-// leaves few registers.
-static inline INFOLI_HD int stream_unit(SmemShape s) { return !s.split_units ? 4 : s.edge_g ? 8 : 16; }
 
 static inline INFOLI_HD StreamLayout stream_layout(SmemShape s) {
   StreamLayout L;
@@ -233,20 +226,12 @@ static inline INFOLI_HD StreamLayout stream_layout(SmemShape s) {
   off += (size_t)s.rows_cap * sizeof(float);
   off = (off + 15) & ~(size_t)15;
   L.part = off;
-  off += (size_t)s.max_slots * sizeof(float) * (s.kahan ? 2 : 1);
+  off += (size_t)s.max_slots * sizeof(float);
+  L.sums = off;
+  off += (size_t)s.cluster * (size_t)s.cells_cap * sizeof(float);
   off = (off + 15) & ~(size_t)15;
   L.mbar = off;
   off += 16;
-  L.cells = off;
-  L.gca = off;
-  L.gates = off;
-  if (s.split_units) {
-    off += (size_t)kStreamCellArrays * (size_t)s.cells_cap * sizeof(float);
-    L.gca = off;
-    off += (size_t)s.cells_cap * sizeof(double);
-    L.gates = off;
-    off += (size_t)kGateFloats * (size_t)s.cells_cap * sizeof(float);
-  }
   L.total = off;
   return L;
 }

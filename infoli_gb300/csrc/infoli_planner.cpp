@@ -22,7 +22,7 @@ size_t plan_smem_bytes(int tile_cap, int nbuf, int threads, int cells_cap, int m
 namespace {
 
 constexpr int kCellCost = 8;  // edge-equivalents charged per cell when balancing CTAs
-constexpr int kStreamSplitCells = 256;  // stream plans: gate units over all warps up to this many cells per CTA
+constexpr int kStreamLongChunk = 64;    // entries per lane and group from which stream plans take 16 at a time
 constexpr int kSmallNetworkCtas = 100;  // the most CTAs the small-network floor asks for
 
 // Contiguous partition of cells into at most `grid` CTAs, each at most
@@ -633,8 +633,7 @@ struct StreamCut {
 // the write of 32 partial sums), kSlotCost: a slot's in the owner's sum.
 constexpr double kStreamGroupCost = 8.0, kStreamSlotCost = 0.4;
 
-// A group's length is a multiple of `unit` entries.
-StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, int unit, std::vector<int>& hist) {
+StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, std::vector<int>& hist) {
   StreamCut c;
   c.len = len;
   hist.assign((size_t)std::min(len, max_len) + 2, 0);
@@ -653,7 +652,7 @@ StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, in
     int best = 0;
     for (int w = 1; w < kStreamWarps; ++w)
       if (load[w] < load[best]) best = w;
-    load[best] += (l + unit - 1) / unit * unit + kStreamGroupCost;
+    load[best] += ((l + 3) & ~3) + kStreamGroupCost;
   };
   for (int l = (int)hist.size() - 1; l > 0; --l) {
     int left = hist[(size_t)l];
@@ -677,7 +676,6 @@ StreamCut stream_cut_cost(const std::vector<int>& rows, int len, int max_len, in
 
 static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
   const int n = in.n;
-  const size_t slot_bytes = in.kahan ? 2 * sizeof(float) : sizeof(float);
   // ---- cluster size: the fewest sender shares whose V_dend fits
   SmemShape sh{};
   sh.threads = kStreamThreads;
@@ -706,6 +704,7 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     sh.tile_cap = share;
     sh.rows_cap = cs > 1 ? ((mr + 3) & ~3) + 8 : 0;
     sh.max_slots = mr;
+    sh.cells_cap = ((mr + cs - 1) / cs + 31) & ~31;
     if (stream_layout(sh).total > in.smem_budget) continue;
     starts.swap(st);
     max_rows = mr;
@@ -723,17 +722,8 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     const int per = (starts[b + 1] - starts[b] + cs - 1) / cs;
     sh.cells_cap = std::max(sh.cells_cap, (per + 31) & ~31);
   }
-  // gate units over all warps with the gate state in shared memory, where few
-  // cells per CTA leave most warps without an own cell and the state fits
-  sh.max_slots = max_rows;
-  if (sh.cells_cap <= kStreamSplitCells) {
-    sh.split_units = 1;
-    if (stream_layout(sh).total > in.smem_budget) sh.split_units = 0;
-  }
-  // groups are whole blocks of the entries that the kernel takes at a time
-  const int unit = stream_unit(sh);
   sh.max_slots = 0;
-  const int slots_cap = (int)std::min<size_t>(65535, (in.smem_budget - stream_layout(sh).total) / slot_bytes);
+  const int slots_cap = (int)std::min<size_t>(65535, (in.smem_budget - stream_layout(sh).total - 16) / sizeof(float));
 
   Plan& P = *out;
   P = Plan();
@@ -787,7 +777,7 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     lens.erase(std::unique(lens.begin(), lens.end()), lens.end());
     StreamCut best;
     for (int len : lens) {
-      const StreamCut c = stream_cut_cost(cnt, len, max_len, unit, hist);
+      const StreamCut c = stream_cut_cost(cnt, len, max_len, hist);
       if (c.slots < slots_cap && (best.len == 0 || c.cost < best.cost)) best = c;
       if (len >= max_len) break;
     }
@@ -823,7 +813,7 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
         int w = 0;
         for (int q = 1; q < kStreamWarps; ++q)
           if (load[q] < load[w]) w = q;
-        load[w] += (pc[(size_t)g * 32].len + unit - 1) / unit * unit + kStreamGroupCost;
+        load[w] += ((pc[(size_t)g * 32].len + 3) & ~3) + kStreamGroupCost;
         of_warp[(size_t)g] = w;
       }
     }
@@ -836,7 +826,7 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
       for (int g = 0; g < ng; ++g) {
         if (of_warp[(size_t)g] != w) continue;
         ++placed;
-        const int quads = (pc[(size_t)g * 32].len + unit - 1) / unit * (unit / 4), pairs = quads / 2, len = quads * 4;
+        const int quads = (pc[(size_t)g * 32].len + 3) / 4, pairs = quads / 2, len = quads * 4;
         const size_t base = L.ent.size();
         L.gdesc.push_back(int2_t{(int)(base / 128), quads});
         L.ent.resize(base + (size_t)quads * 128);
@@ -951,6 +941,9 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     groups += L.gdesc.size();
   }
   sh.max_slots = max_slots;
+  // blocks of 16 entries where lane-chunks are long (fewer waits per entry);
+  // blocks of 8 where what is left of a chunk after whole blocks would weigh
+  sh.block = !in.g && total >= (size_t)kStreamLongChunk * 32 * std::max<size_t>(1, groups) ? 16 : 8;
   if (stream_layout(sh).total > in.smem_budget) {
     *err = "make_plan: could not fit shared memory";
     return false;
@@ -1099,6 +1092,18 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
     std::sort(u.begin(), u.end());
     u.erase(std::unique(u.begin(), u.end()), u.end());
     if (!u.empty()) max_window = std::max(max_window, ((u.back() + 4) & ~3) - (u.front() & ~3));
+  }
+  if (!in.cta_starts && stream_plan_wanted(in)) {
+    // decided before the stamped plan is packed where it cannot turn out
+    // better: many cells per CTA, or wide windows that no order narrows
+    int words = 0, cells = 0;
+    for (int b = 0; b < ctas; ++b) {
+      words = std::max(words, (int)uniq[b].size());
+      cells = std::max(cells, starts[b + 1] - starts[b]);
+    }
+    if (cells > kStampedMaxCells || (words > kStampedMaxWords && words > n / 2)) {
+      if (make_stream_plan(in, out, err)) return true;
+    }
   }
 
   // ---- tile capacity: one buffer holding the whole window when it fits,
@@ -1587,7 +1592,7 @@ std::vector<int> locality_order(const PlanInput& in, int parts, int threads, std
 // Plans the network as given; for stamped plans with wide windows, also
 // plans it in a locality-preserving cell order and keeps that plan when its
 // largest window is at least a fifth smaller.
-bool make_plan(const PlanInput& in, Plan* out, std::string* err) {
+static bool make_plan_ordered(const PlanInput& in, Plan* out, std::string* err) {
   if (!make_plan_base(in, out, err)) return false;
   if (!in.reorder || in.cta_starts || !out->shape.stamped || out->cta.size() < 2) return true;
   const int n = in.n;
@@ -1630,6 +1635,18 @@ bool make_plan(const PlanInput& in, Plan* out, std::string* err) {
   if ((int64_t)max_window(P2) * 5 > (int64_t)w0 * 4) return true;
   P2.perm.assign(order.begin(), order.end());
   *out = std::move(P2);
+  return true;
+}
+
+// The plan for a launch: a stamped plan whose windows stay wide in any order
+// gives way to a stream plan.
+bool make_plan(const PlanInput& in, Plan* out, std::string* err) {
+  if (!make_plan_ordered(in, out, err)) return false;
+  if (out->shape.stamped && out->shape.poll_words > kStampedMaxWords && stream_plan_wanted(in)) {
+    Plan st;
+    std::string e2;
+    if (make_stream_plan(in, &st, &e2)) *out = std::move(st);
+  }
   return true;
 }
 
@@ -1714,7 +1731,6 @@ extern "C" int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t*
           if (wt[q] > wt[q + 1]) return -5;
         for (int gi = 0; gi < x.n_groups; ++gi) {
           const int2_t d = P.gdesc[(size_t)x.group_begin + gi];
-          if (d.y * 4 % stream_unit(P.shape)) return -5;
           for (int kk = 0; kk < d.y * 4; ++kk) {
             unsigned bank_words[32];
             int bank_n[32] = {0}, worst = 1;

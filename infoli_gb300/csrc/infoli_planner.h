@@ -70,6 +70,16 @@ enum { kGatherMaxMeanDegree = 384 };
 //     kStreamMinDegree edges on average (shorter rows spend more on the
 //     exchange of partial sums than the tiles cost), unless they are dense
 //     with one conductance (bitmask plans).
+// A stamped plan (edges on chip, V_dend word by word from its publishers) gives
+// way to a stream plan when a CTA polls more than kStampedMaxWords words or owns
+// more than kStampedMaxCells cells.  Microseconds per step, stamped against
+// stream: 6,000 cells x 60 senders (2,800 words) 2.85 / 3.5; 10,000 x 40 (3,300)
+// 3.30 / 3.53; 20,000 x 30 (132 cells, 3,900) 3.73 / 3.65; 4,000 at 20 % (4,000)
+// 3.85 / 4.52; 10,000 x 100 (4,850) 4.29 / 3.86; 6,000 x 200 (5,300) 3.97 / 3.79;
+// 20,000 x 100 (9,700) 6.82 / 4.30; 30,000 x 8 (198 cells, 1,600 words) 4.56 /
+// 3.51; 150 x 150 grid (148 cells) 4.33 / 4.94; 200 x 200 grid (264 cells) 5.33 /
+// 4.95; 48,000 x 33 (316 cells, 9,400) 7.84 / 4.66.
+enum { kStampedMaxWords = 4500, kStampedMaxCells = 192 };
 enum { kStreamMinDegree = 16 };
 constexpr double kStreamMaxDensity = 0.45;
 

@@ -44,15 +44,8 @@ __device__ __forceinline__ uint32_t peer_addr(uint32_t local, unsigned peer) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(local), "r"(peer));
   return ra;
 }
-__device__ __forceinline__ float ld_peer(uint32_t a) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ float2 ld_peer2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-  return v;
+__device__ __forceinline__ void st_peer(uint32_t a, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
 
 // The entries are read once per step: past L1, and in L2 with a policy that
@@ -145,13 +138,12 @@ struct StreamSum {
   }
 };
 
-// A warp's groups of lane-chunks, partial sums into `part` (pairs of sum and
-// compensation with KAHAN), in blocks of N entries per lane (whole blocks
-// only, except with N = 8 a last quad, when QUAD).  The next block's entries
-// are loaded before this one's arithmetic, across groups too, and the first
-// group's before `wait` (the wait for V_dend): no load latency stands between
-// blocks.  G_EARLY: the next conductances as well, where registers allow.
-template <bool KAHAN, bool EDGE_G, bool BYTE, int N, bool QUAD, bool G_EARLY, class Wait>
+// A warp's groups of lane-chunks, partial sums into `part`, in blocks of N
+// entries per lane, then what is left of a group: with N = 16 up to a pair of
+// quads, and a quad.  The next block's entries are loaded before this one's
+// arithmetic, across groups too, and the first group's before `wait` (the wait
+// for V_dend): no load latency stands between blocks.
+template <bool KAHAN, bool EDGE_G, bool BYTE, int N, class Wait>
 __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& w, int warp, int lane, const float* sm,
                                               const float* rows, float* part, uint64_t pol, Wait wait) {
   const int* wt = a.probes + w.pad0 + warp;
@@ -187,16 +179,19 @@ __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& 
       ln = (unsigned)__ldg(a.gcol + (size_t)(g + 1) * 32 + lane);
     }
     const int end = gd.x + gd.y / (N / 4) * (N / 4);
-    const bool odd = QUAD && (gd.y & 1);
-    uint2 tail = make_uint2(0, 0);
+    const bool pair = N == 16 && (gd.y & 2), odd = gd.y & 1;
+    uint4 left_pair = make_uint4(0, 0, 0, 0);
+    uint2 left_quad = make_uint2(0, 0);
     float4 gt = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     const float nvc = -rows[ld & 0xffffu];
     const float2 nvc2 = make_float2(nvc, nvc);
     StreamSum<KAHAN> s;
     auto next_group = [&]() {  // what follows this group's whole blocks
+      if (pair) left_pair = ld_stream4(ent + (size_t)end * 16, pol);
       if (odd) {
-        tail = ld_stream2(reinterpret_cast<const uint2*>(ent - lane + (size_t)end * 16) + lane, pol);
-        if (EDGE_G) gt = ld_streamg(eg + (size_t)end * 32, pol);
+        const int q = end + (pair ? 2 : 0);
+        left_quad = ld_stream2(reinterpret_cast<const uint2*>(ent - lane + (size_t)q * 16) + lane, pol);
+        if (EDGE_G) gt = ld_streamg(eg + (size_t)q * 32, pol);
       }
       if (gn.y >= N / 4) load_c(gn.x);
     };
@@ -214,7 +209,7 @@ __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& 
       else
         next_group();
       float2 nt = s.start();
-      if (EDGE_G && G_EARLY) {
+      if (EDGE_G) {
         float4 now[N / 4];
 #pragma unroll
         for (int i = 0; i < N / 4; ++i) now[i] = gc[i];
@@ -222,74 +217,56 @@ __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& 
         stream_terms<N, EDGE_G>(x, now, nvc2, nt);
       } else {
         stream_terms<N, EDGE_G>(x, gc, nvc2, nt);
-        if (EDGE_G && nq >= 0) load_g(nq, gc);
       }
+      s.add(nt);
+    }
+    if (pair) {
+      float2 x[4], nt = s.start();
+      stream_gather<8, BYTE>(sm, &left_pair, x);
+      stream_terms<8, false>(x, &gt, nvc2, nt);
       s.add(nt);
     }
     if (odd) {
       float2 x[2], nt = s.start();
-      const uint4 o = make_uint4(tail.x, tail.y, 0u, 0u);
+      const uint4 o = make_uint4(left_quad.x, left_quad.y, 0u, 0u);
       stream_gather<4, BYTE>(sm, &o, x);
       stream_terms<4, EDGE_G>(x, &gt, nvc2, nt);
       s.add(nt);
     }
-    const unsigned slot = ld >> 16;
-    if (KAHAN) {
-      // error-free sum of the two accumulators; its error joins the compensation
-      const float a0 = -s.acc.x, a1 = -s.acc.y;
-      const float sum = a0 + a1;
+    const float a0 = -s.acc.x, a1 = -s.acc.y;
+    float sum = a0 + a1;
+    if (KAHAN) {  // the rounding of this addition and the compensations, applied once
       const float bb = sum - a0;
-      const float err = (a0 - (sum - bb)) + (a1 - bb);
-      reinterpret_cast<float2*>(part)[slot] = make_float2(sum, (s.cmp.x + s.cmp.y) - err);
-    } else {
-      part[slot] = -(s.acc.x + s.acc.y);
+      sum += ((a0 - (sum - bb)) + (a1 - bb)) - (s.cmp.x + s.cmp.y);
     }
+    part[ld >> 16] = sum;
     gd = gn;
     ld = ln;
   }
 }
 
-// Sum of an owned receiver's partial sums over the cluster's CTAs by `width`
-// lanes (`sub`: this lane's place; all lanes of the warp call it), in a fixed
-// order (TwoSum per addition with KAHAN, the errors and compensations applied
-// once).  The first AHEAD CTAs' slot ranges are in `ahead`.  The result is valid in the lanes with sub == 0.
-template <bool KAHAN, int AHEAD>
-__device__ __forceinline__ float combine_stream(const int2* ahead, const int2* slots, bool own, int cs,
-                                                const float* part, int sub, int width) {
-  const uint32_t base = smem_u32(part);
+// Sum of a receiver's partial sums by `width` lanes (`sub`: this lane's place;
+// with width > 1 all lanes of the warp call it), in a fixed order, with KAHAN
+// an error-free sum per addition whose errors are applied once.  Valid in the
+// lanes with sub == 0.
+template <bool KAHAN>
+__device__ __forceinline__ float sum_slots(int2 sl, const float* part, int sub, int width) {
   float s = 0.0f, e = 0.0f;
   auto add = [&](float x) {
     const float t = s + x;
-    const float bp = t - s;
-    e += (s - (t - bp)) + (x - bp);
+    if (KAHAN) {
+      const float bp = t - s;
+      e += (s - (t - bp)) + (x - bp);
+    }
     s = t;
   };
-#pragma unroll 1
-  for (int k = 0; k < cs; ++k) {
-    int2 sl = ahead[0];
-    if (AHEAD > 1 && k == 1) sl = ahead[AHEAD - 1];
-    if (k >= AHEAD) sl = own ? __ldg(slots + k) : make_int2(0, 0);
-    const uint32_t pa = cs > 1 ? peer_addr(base, (unsigned)k) : base;
 #pragma unroll 4
-    for (int q = sub; q < sl.y; q += width) {
-      if (KAHAN) {
-        const float2 p = cs > 1 ? ld_peer2(pa + 8u * (uint32_t)(sl.x + q)) : reinterpret_cast<const float2*>(part)[sl.x + q];
-        add(p.x);
-        e -= p.y;
-      } else {
-        s += cs > 1 ? ld_peer(pa + 4u * (uint32_t)(sl.x + q)) : part[sl.x + q];
-      }
-    }
-  }
+  for (int q = sub; q < sl.y; q += width) add(part[sl.x + q]);
   for (int o = 1; o < width; o <<= 1) {
     const float s2 = __shfl_down_sync(0xffffffffu, s, o);
-    if (KAHAN) {
-      const float e2 = __shfl_down_sync(0xffffffffu, e, o);
-      add(s2);
-      e += e2;
-    } else {
-      s += s2;
-    }
+    const float e2 = KAHAN ? __shfl_down_sync(0xffffffffu, e, o) : 0.0f;
+    add(s2);
+    e += e2;
   }
   return KAHAN ? s + e : s;
 }
@@ -307,21 +284,18 @@ __device__ __forceinline__ bool stream_wait(const StepArgs& a, uint64_t* bar, un
   return true;
 }
 
-template <bool KAHAN, bool EDGE_G, bool SPLIT, bool BYTE>
+template <bool KAHAN, bool EDGE_G, bool BYTE, int N>
 __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_abort;
+  __shared__ float s_peer[kStreamMaxCluster];  // set by a CTA of the cluster that gave up
   __shared__ unsigned long long s_prof[4];  // cycles: gate units, wait for the share, coupling, rest
   const StreamLayout L = stream_layout(a.shape);
   const float* sm = reinterpret_cast<const float*>(smem_raw);
   float* part = reinterpret_cast<float*>(smem_raw + L.part);
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + L.mbar);
+  float* sums = reinterpret_cast<float*>(smem_raw + L.sums);
   const int cs = a.shape.cluster, share = a.shape.tile_cap, cap = a.shape.cells_cap;
-  float* sV = reinterpret_cast<float*>(smem_raw + L.cells);  // SPLIT: V_dend, V_soma, V_axon, nine currents
-  float* sI = sV + 3 * cap;
-  float* sH = sV + 12 * cap;  // SPLIT: VoltHalf of every cell
-  double* sCa = reinterpret_cast<double*>(smem_raw + L.gca);
-  float* sG = reinterpret_cast<float*>(smem_raw + L.gates);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // A launch whose clusters are not the plan's (a tool that relaunches the
   // kernel without its attributes) would read shared memory of CTAs that are
@@ -331,15 +305,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     return;
   }
   const CtaWork w = a.cta[blockIdx.x];
-  // Owned cells: one thread each, or (SPLIT, few cells per CTA) `width` lanes
-  // that add the partial sums together, the first of them the owner; the last
-  // warp, which waits for the grid barrier, owns none then.
-  int width = 1;
-  if (SPLIT)
-    while (width < 8 && width * 2 * w.n_cells <= kStreamThreads - 32) width *= 2;
-  const int r = tid / width, sub = tid % width;
-  const bool mine = r < w.n_cells, owner = mine && sub == 0;
-  const int cell = w.cell_begin + r;
+  const bool owner = tid < w.n_cells;  // one thread per owned cell
+  const int cell = w.cell_begin + tid;
+  // Lanes that add a receiver's partial sums: one, or with few cells of many
+  // slots each (dense rows) as many as the CTA has for each of its cells, up
+  // to 8; the sums then go through shared memory to the owners.
+  int wlog = 0;
+  if (cs == 1 && w.n_slots > 4 * w.n_cells)
+    while (wlog < 3 && (2 * w.n_cells << wlog) <= kStreamThreads) ++wlog;
+  const int width = 1 << wlog;
   const long long np = a.n_pad;
   // this CTA's share of V_dend: cells [lo, lo + nshare), and with cluster > 1
   // the cluster's rows (copies of whole 16-byte units)
@@ -353,45 +327,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     mbar_init(mbar, 1);
     fence_mbar_init();
     s_abort = 0;
+    for (int k = 0; k < kStreamMaxCluster; ++k) s_peer[k] = 0.0f;
   }
   Volts v{};
-  Gates g{};
-  float my_amp = 0.0f;
-  int my_onset = 0, my_off = 0;
   if (owner) {
     const float* st = a.st;
     v.Vd = a.vd[a.step0 & 1][cell];
     v.Vs = st[F_VS * np + cell];
     v.Va = st[F_VA * np + cell];
-    if (SPLIT) {
-      for (int f = F_Q; f < F_COUNT; ++f) sG[f * cap + r] = st[f * np + cell];
-      sCa[r] = a.ca[cell];
-      sV[r] = v.Vd;
-      sV[cap + r] = v.Vs;
-      sV[2 * cap + r] = v.Va;
-    } else {
-      g.q = st[F_Q * np + cell];
-      g.r = st[F_R * np + cell];
-      g.s = st[F_S * np + cell];
-      g.Ca = a.ca[cell];
-      g.ICaH = st[F_ICAH * np + cell];
-      g.gCaL = st[F_GCAL * np + cell];
-      g.k = st[F_K * np + cell];
-      g.l = st[F_L * np + cell];
-      g.m = st[F_M * np + cell];
-      g.h = st[F_H * np + cell];
-      g.n = st[F_N * np + cell];
-      g.p = st[F_P * np + cell];
-      g.xs = st[F_XS * np + cell];
-      g.ma = st[F_MA * np + cell];
-      g.ha = st[F_HA * np + cell];
-      g.xa = st[F_XA * np + cell];
-    }
-    if (a.stim_kind == STIM_CELL) {
-      my_amp = a.cell_amp[cell];
-      my_onset = a.cell_onset[cell];
-    }
-    if (a.cell_step_off) my_off = a.cell_step_off[cell];
     a.vds[a.step0 & 1][cell] = v.Vd * kVScale;
   }
   const VoltCoef vk = volt_coef(a.P);
@@ -411,8 +354,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     s_prof[k] += t - t_prev;
     t_prev = t;
   };
-  for (int st = 0; st < a.n_steps; ++st) {
-    const int step = a.step0 + st;
+  for (int st_i = 0; st_i < a.n_steps; ++st_i) {
+    const int step = a.step0 + st_i;
     const bool trace_now = tclock.take();
     // V^step is written and every thread past a CTA barrier: arrive (the
     // release covers the CTA's writes)
@@ -421,36 +364,49 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
 
     // ---------------- gate units (own voltages only), first half of the voltage step
     VoltHalf vh{};
-    if (SPLIT) {
-      const int items = ((w.n_cells + 31) >> 5) * kUnits;
-      for (int it = warp; it < items; it += kStreamWarps) {
-        const int c = (it / kUnits) * 32 + lane;
-        const unsigned m = 1u << (it % kUnits);
-        if (c < w.n_cells) {
-          const Volts u = {sV[c], sV[cap + c], sV[2 * cap + c]};
-          Currents cur;
-          Gates gs = load_gates(sG, sCa, cap, c, m);
-          run_units(a.P, m, u, gs, cur);
-          store_gates(sG, sCa, cap, c, m, gs);
-          store_currents(sI, cap, c, m, cur);
-        }
-      }
-      __syncwarp();
-      if (warp == kStreamWarps - 1) {
-        asm volatile("bar.arrive 1, %0;" ::"r"((int)kStreamThreads) : "memory");
-      } else {
-        asm volatile("bar.sync 1, %0;" ::"r"((int)kStreamThreads) : "memory");
-        if (owner) {
-          vh = voltage_first(a.P, vk, v, load_currents(sI, cap, r));
-          sH[r] = vh.dend;
-          sH[cap + r] = vh.I_h;
-          sH[2 * cap + r] = vh.Vs;
-          sH[3 * cap + r] = vh.Va;
-        }
-      }
-    } else if (owner) {
+    if (owner) {
+      // The gate state stays in global memory (L2) between steps, so that the
+      // coupling has the registers; its loads and stores, like the units, run
+      // while the barrier and the copy complete.  (In registers: 15.9 against
+      // 12.9 us per step at 100,000 cells, with spills and no room for loads
+      // in flight; in shared memory with the units spread over all warps: 4.7
+      // against 3.5 us at 10,000 cells x 40 senders, through two more waits
+      // inside the CTA.)
+      float* st = a.st + cell;
+      Gates g;
+      g.q = st[F_Q * np];
+      g.r = st[F_R * np];
+      g.s = st[F_S * np];
+      g.Ca = a.ca[cell];
+      g.ICaH = st[F_ICAH * np];
+      g.gCaL = st[F_GCAL * np];
+      g.k = st[F_K * np];
+      g.l = st[F_L * np];
+      g.h = st[F_H * np];
+      g.n = st[F_N * np];
+      g.p = st[F_P * np];
+      g.xs = st[F_XS * np];
+      g.ha = st[F_HA * np];
+      g.xa = st[F_XA * np];
       Currents cur;
       run_units(a.P, 0xffu, v, g, cur);
+      st[F_Q * np] = g.q;
+      st[F_R * np] = g.r;
+      st[F_S * np] = g.s;
+      a.ca[cell] = g.Ca;
+      st[F_ICAH * np] = g.ICaH;
+      st[F_K * np] = g.k;
+      st[F_L * np] = g.l;
+      st[F_H * np] = g.h;
+      st[F_N * np] = g.n;
+      st[F_P * np] = g.p;
+      st[F_XS * np] = g.xs;
+      st[F_HA * np] = g.ha;
+      st[F_XA * np] = g.xa;
+      if (st_i + 1 == a.n_steps) {  // m and m_a follow from the voltages alone
+        st[F_M * np] = g.m;
+        st[F_MA * np] = g.ma;
+      }
       vh = voltage_first(a.P, vk, v, cur);
     }
 
@@ -483,47 +439,64 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     __syncwarp();
 
     // ---------------- coupling
-    constexpr int kBlockEntries = SPLIT && !EDGE_G ? 16 : 8;
-    couple_stream<KAHAN, EDGE_G, BYTE, kBlockEntries, !SPLIT, SPLIT>(a, w, warp, lane, sm, rows, part, pol, [&]() {
-      if (!stream_wait(a, mbar, (unsigned)st & 1u, &s_abort)) s_abort = 1;
+    couple_stream<KAHAN, EDGE_G, BYTE, N>(a, w, warp, lane, sm, rows, part, pol, [&]() {
+      if (!stream_wait(a, mbar, (unsigned)st_i & 1u, &s_abort)) s_abort = 1;
       mark(1);
     });
-    // the owners' slot ranges, in flight while the other warps finish
-    int2 slots[SPLIT ? 1 : 2];
-#pragma unroll
-    for (int k = 0; k < (SPLIT ? 1 : 2); ++k)
-      slots[k] = mine && k < cs ? __ldg(a.cell_slots + (size_t)cell * cs + k) : make_int2(0, 0);
-    if (cs > 1)
-      cluster_sync_all();  // every CTA's partial sums (and abort flags) are there
-    else
-      __syncthreads();
+    // what the update reads from global memory, in flight while the other warps finish
+    const int2 none = make_int2(0, 0);
+    const int per = cs > 1 ? (w.n_tiles + cs - 1) / cs : 0;  // rows of a CTA of the cluster
+    int2 slots = none;
+    const int sr = tid >> wlog;  // the receiver that this thread adds slots of
+    if (sr < (cs == 1 ? w.n_cells : w.n_tiles))
+      slots = __ldg(a.cell_slots + (size_t)((cs == 1 ? w.cell_begin : w.tile_begin) + sr) * cs + w.pad1);
+    float my_amp = 0.0f;
+    int my_onset = 0;
+    if (owner && a.stim_kind == STIM_CELL) {
+      my_amp = __ldg(a.cell_amp + cell);
+      my_onset = __ldg(a.cell_onset + cell);
+    }
+    __syncthreads();
+    if (cs > 1) {
+      // every row's sum over this share goes to its owner's CTA (a store: a
+      // remote load would stand in the update's way)
+      for (int q = tid; q < w.n_tiles; q += kStreamThreads) {
+        if (q >= kStreamThreads) slots = __ldg(a.cell_slots + (size_t)(w.tile_begin + q) * cs + w.pad1);
+        const float s = sum_slots<KAHAN>(slots, part, 0, 1);
+        const int k = (q >= per) + (q >= 2 * per) + (q >= 3 * per);
+        st_peer(peer_addr(smem_u32(sums + w.pad1 * cap + (q - k * per)), (unsigned)k), s);
+      }
+      if (s_abort && tid < cs) st_peer(peer_addr(smem_u32(s_peer + w.pad1), (unsigned)tid), 1.0f);
+      cluster_sync_all();
+    }
     mark(2);
 
     // ---------------- owners: the receiver's sum, second half of the voltage step
     float ic = 0.0f;
-    if (SPLIT || mine)
-      ic = combine_stream<KAHAN, (SPLIT ? 1 : 2)>(slots, a.cell_slots + (size_t)cell * cs, mine, cs, part, sub, width) *
-           kInvVScale;
+    if (width > 1) {
+      const float s = sum_slots<KAHAN>(slots, part, (tid & (width - 1)), width);
+      if (sr < w.n_cells && (tid & (width - 1)) == 0) sums[sr] = s;
+      __syncthreads();
+      if (owner) ic = sums[tid];
+    } else if (cs == 1) {
+      if (owner) ic = sum_slots<KAHAN>(slots, part, 0, 1);
+    } else if (owner) {
+      for (int k = 0; k < cs; ++k) ic += sums[k * cap + tid];
+    }
     if (owner) {
+      ic *= kInvVScale;
       if (!EDGE_G) ic *= a.g_uniform;
-      const int ls = step + my_off;
       float iapp;
       if (a.stim_kind == STIM_PULSE)
-        iapp = (ls >= a.stim_start && ls < a.stim_end) ? a.stim_amp : 0.0f;
+        iapp = (step >= a.stim_start && step < a.stim_end) ? a.stim_amp : 0.0f;
       else if (a.stim_kind == STIM_CELL)
-        iapp = (ls >= my_onset && ls < my_onset + a.stim_dur) ? my_amp : 0.0f;
+        iapp = (step >= my_onset && step < my_onset + a.stim_dur) ? my_amp : 0.0f;
       else
-        iapp = a.stim_table[(size_t)st * np + cell];
-      if (SPLIT) vh = {sH[r], sH[cap + r], sH[2 * cap + r], sH[3 * cap + r]};
+        iapp = a.stim_table[(size_t)st_i * np + cell];
       v.Vd = voltage_second(a.P, vk, v.Vd, vh, ic, iapp);
       v.Vs = vh.Vs;
       v.Va = vh.Va;
       a.vds[(step + 1) & 1][cell] = v.Vd * kVScale;
-      if (SPLIT) {
-        sV[r] = v.Vd;
-        sV[cap + r] = v.Vs;
-        sV[2 * cap + r] = v.Va;
-      }
       if (trace_now) {
         float* tr = a.trace + (size_t)row * a.trace_nq * np + cell;
         int qi = 0;
@@ -533,13 +506,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
       }
     }
     if (trace_now) ++row;
-    if (cs > 1 && tid == kStreamThreads - 1) {
-      // a CTA that gave up takes its cluster with it (no CTA may leave while
-      // another reads its shared memory)
-      int ab = 0;
-      for (int k = 0; k < cs; ++k) ab |= __float_as_int(ld_peer(peer_addr(smem_u32(&s_abort), (unsigned)k)));
-      if (ab) s_abort = 1;
-    }
+    // a CTA that gave up takes its cluster with it (no CTA may leave while
+    // another writes to its shared memory)
+    if (cs > 1 && tid < cs && s_peer[tid] != 0.0f) s_abort = 1;
     __syncthreads();
     mark(3);
     if (s_abort) break;
@@ -561,39 +530,18 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     a.vd[(a.step0 + a.n_steps) & 1][cell] = v.Vd;
     st[F_VS * np + cell] = v.Vs;
     st[F_VA * np + cell] = v.Va;
-    if (SPLIT) {
-      for (int f = F_Q; f < F_COUNT; ++f) st[f * np + cell] = sG[f * cap + r];
-      a.ca[cell] = sCa[r];
-    } else {
-      st[F_Q * np + cell] = g.q;
-      st[F_R * np + cell] = g.r;
-      st[F_S * np + cell] = g.s;
-      a.ca[cell] = g.Ca;
-      st[F_ICAH * np + cell] = g.ICaH;
-      st[F_GCAL * np + cell] = g.gCaL;
-      st[F_K * np + cell] = g.k;
-      st[F_L * np + cell] = g.l;
-      st[F_M * np + cell] = g.m;
-      st[F_H * np + cell] = g.h;
-      st[F_N * np + cell] = g.n;
-      st[F_P * np + cell] = g.p;
-      st[F_XS * np + cell] = g.xs;
-      st[F_MA * np + cell] = g.ma;
-      st[F_HA * np + cell] = g.ha;
-      st[F_XA * np + cell] = g.xa;
-    }
   }
 }
 
-template <bool K, bool G>
-const void* stream_fn2(bool split, bool byte_off) {
-  if (split) return byte_off ? (const void*)stream_kernel<K, G, true, true> : (const void*)stream_kernel<K, G, true, false>;
-  return byte_off ? (const void*)stream_kernel<K, G, false, true> : (const void*)stream_kernel<K, G, false, false>;
+template <bool K, bool G, int N>
+const void* stream_fn2(bool byte_off) {
+  return byte_off ? (const void*)stream_kernel<K, G, true, N> : (const void*)stream_kernel<K, G, false, N>;
 }
 
-const void* stream_fn(bool kahan, bool edge_g, bool split, bool byte_off) {
-  if (kahan) return edge_g ? stream_fn2<true, true>(split, byte_off) : stream_fn2<true, false>(split, byte_off);
-  return edge_g ? stream_fn2<false, true>(split, byte_off) : stream_fn2<false, false>(split, byte_off);
+const void* stream_fn(bool kahan, bool edge_g, bool byte_off, int block) {
+  if (edge_g) return kahan ? stream_fn2<true, true, 8>(byte_off) : stream_fn2<false, true, 8>(byte_off);
+  if (block == 8) return kahan ? stream_fn2<true, false, 8>(byte_off) : stream_fn2<false, false, 8>(byte_off);
+  return kahan ? stream_fn2<true, false, 16>(byte_off) : stream_fn2<false, false, 16>(byte_off);
 }
 
 void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, int cluster, size_t smem,
@@ -617,7 +565,7 @@ void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, i
 
 cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t stream) {
   const size_t smem = stream_layout(a.shape).total;
-  const void* fn = stream_fn(a.shape.kahan != 0, a.edge_g != nullptr, a.shape.split_units != 0, a.shape.byte_off != 0);
+  const void* fn = stream_fn(a.shape.kahan != 0, a.edge_g != nullptr, a.shape.byte_off != 0, a.shape.block);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg;
@@ -628,7 +576,7 @@ cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t strea
 }
 
 int max_stream_ctas(int cluster, size_t smem) {
-  const void* fn = stream_fn(true, true, false, false);
+  const void* fn = stream_fn(true, true, false, 8);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
