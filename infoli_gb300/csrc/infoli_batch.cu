@@ -10,12 +10,17 @@
 // needing the same number of CTAs form one launch with that cluster size, so
 // clusters have no idle CTA; the launches run concurrently.
 //
-// Coupling is read from per-network adjacency bitmasks with one conductance
-// per network (the reference's uniform CONDUCTANCE, src/openmp/infoli.c:320):
-// a receiver walks the set bits of its row (src/openmp/infoli.c:512-518 for
-// the arithmetic).  Rows are stored word-major so consecutive receivers read
-// consecutive words; a network whose rows fit keeps them in shared memory for
-// the launch, otherwise they are streamed from global memory every step.
+// Networks come as adjacency bitmasks with one conductance per network (the
+// reference's uniform CONDUCTANCE, src/openmp/infoli.c:320; :512-518 for the
+// coupling's arithmetic).  Two ways to run them:
+//   - entry lists (list_kernel, batches): the rows are turned into 16-bit
+//     entries on the device when the batch is made, and streamed every step,
+//     one receiver per lane;
+//   - bitmask rows (batch_kernel: the serving lane, and batches whose lists
+//     would take more than half of the free memory): a receiver walks the set
+//     bits of its row.  Rows are stored word-major so consecutive receivers
+//     read consecutive words; a network whose rows fit keeps them in shared
+//     memory for the launch, otherwise they are streamed every step.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,15 +32,8 @@
 #include "../../include/infoli_gpu.h"
 #include "infoli_cell.cuh"
 #include "infoli_internal.h"
+#include "infoli_list.cuh"
 #include "infoli_ptx.cuh"
-
-namespace infoli {
-namespace {
-
-constexpr float kNegLog2eOver100 = -0.014426950408889634f;  // -log2(e)/100
-
-}  // namespace
-}  // namespace infoli
 
 #include "infoli_lane.h"
 
@@ -49,6 +47,7 @@ struct BatchArgs {
   int res_words;     // shared words for resident rows (per CTA)
   const int* step;   // current step index of the batch (device), for CTAs whose step0 < 0
   int n_steps;       // steps of the launch, for CTAs whose n_steps < 0
+  float l2_keep;     // entry lists: share of their lines that L2 should keep
   unsigned long long* cta_ns;  // [2 * grid]: globaltimer at start and end of every CTA
 };
 
@@ -278,6 +277,244 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batch_kernel(const __grid
   }
 }
 
+// ------------------------------------------------------------- entry lists
+
+// A receiver's row as entries: one warp per row, lane i taking bank b = (r + i)
+// % 32, the senders with that remainder.  Entry j of lane i goes to position 32
+// j + i, so the 32 consecutive receivers of a warp, at one position, read 32
+// different banks; positions whose bank has run out are filled with what other
+// banks have too much of, the rest follows.  The order depends on the row
+// alone, so results do not depend on how receivers fall into warps.
+constexpr int kPackWarps = 8;
+
+__global__ void __launch_bounds__(kPackWarps * 32) batch_pack_kernel(const uint32_t* __restrict__ bits, int n, int per,
+                                                                      int gstride, const int2* __restrict__ grp,
+                                                                      uint16_t* __restrict__ ent) {
+  __shared__ int s_hole[kPackWarps][33], s_count[kPackWarps][32];
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+  const int r = blockIdx.x * kPackWarps + wi;
+  if (r >= n) return;
+  const int wpr = (n + 31) / 32, bank = (r + lane) & 31;
+  const uint32_t* row = bits + (size_t)r * wpr;
+  auto word = [&](int w) {  // this row's word w without self and the bits past the network
+    uint32_t x = w < wpr ? __ldg(row + w) : 0u;
+    if (w == r / 32) x &= ~(1u << (r & 31));
+    if (w == wpr - 1 && (n & 31)) x &= (1u << (n & 31)) - 1u;
+    return x;
+  };
+  int count = 0;
+  for (int w0 = 0; w0 < wpr; w0 += 32) {
+    const uint32_t mine = word(w0 + lane);
+    for (int j = 0; j < 32; ++j) count += (__shfl_sync(0xffffffffu, mine, j) >> bank) & 1u;
+  }
+  int total = count;
+  for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  const int full = total / 32;  // rounds of 32 positions
+  const int holes = max(0, full - count), spare = max(0, count - full);
+  int hs = holes, ss = spare;  // inclusive scans
+  for (int o = 1; o < 32; o <<= 1) {
+    const int h = __shfl_up_sync(0xffffffffu, hs, o), q = __shfl_up_sync(0xffffffffu, ss, o);
+    if (lane >= o) {
+      hs += h;
+      ss += q;
+    }
+  }
+  const int all_holes = __shfl_sync(0xffffffffu, hs, 31);
+  s_hole[wi][lane] = hs - holes;
+  if (lane == 31) s_hole[wi][32] = hs;
+  s_count[wi][lane] = count;
+  __syncwarp();
+  const int k = r / per, local = r - k * per;
+  const int2 gd = grp[k * gstride + local / 32];  // {first pair row, pairs}
+  uint16_t* out = ent + (size_t)gd.x * 256 + (local & 31) * 8;
+  auto put = [&](int pos, int sender) { out[(size_t)(pos >> 3) * 256 + (pos & 7)] = (uint16_t)(sender * 4); };
+  int j = 0;
+  for (int w0 = 0; w0 < wpr; w0 += 32) {
+    const uint32_t mine = word(w0 + lane);
+    for (int q = 0; q < 32; ++q) {
+      const uint32_t x = __shfl_sync(0xffffffffu, mine, q);
+      if (!((x >> bank) & 1u)) continue;
+      int pos;
+      if (j < full) {
+        pos = 32 * j + lane;
+      } else {
+        const int s = ss - spare + (j - full);  // among all spare entries
+        if (s < all_holes) {
+          int lo = 0, hi = 31;  // the lane whose holes contain the s-th
+          while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_hole[wi][mid] <= s)
+              lo = mid;
+            else
+              hi = mid - 1;
+          }
+          pos = 32 * (s_count[wi][lo] + s - s_hole[wi][lo]) + lo;
+        } else {
+          pos = 32 * full + (s - all_holes);
+        }
+      }
+      put(pos, 32 * (w0 + q) + bank);
+      ++j;
+    }
+  }
+  for (int pos = total + lane; pos < gd.y * 8; pos += 32) put(pos, r);  // the receiver itself: a term of 0
+}
+
+// Gate state in shared memory (13 floats and Ca2+ per cell; m and m_a follow
+// from the voltages), so the coupling has the registers.
+constexpr int kListGateFloats = 13;
+constexpr int kListDepth = 4;  // pair rows in flight per lane
+
+size_t list_smem(int block, int vcap) {
+  return 2 * sizeof(float) * (size_t)vcap + (size_t)block * (kListGateFloats * sizeof(float) + sizeof(double));
+}
+
+// What bounds it: HBM (2 bytes per edge and step: 3.7e12 edges/s at 7.4 TB/s)
+// while every SM has a network, else an SM's SFU, FMA and issue rates (about
+// 2.2 cycles per warp and entry).  The bit walk takes 16 instructions per lane
+// and lockstep iteration, lanes waiting for the fullest word.
+template <int BLOCK, bool KAHAN>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) list_kernel(const __grid_constant__ BatchArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* vbuf = reinterpret_cast<float*>(smem_raw);  // [2][vcap]
+  double* sCa = reinterpret_cast<double*>(vbuf + 2 * a.vcap);
+  float* sG = reinterpret_cast<float*>(sCa + BLOCK);
+  const unsigned long long t_start = globaltimer_ns();
+  const BatchCta* wp = a.cta + blockIdx.x;
+  const int ncell = wp->ncell, ncta = wp->ncta, rank0 = wp->rank0;
+  const bool cl_sync = wp->cl_sync != 0;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const unsigned me = cluster_rank();
+  const bool own = tid < ncell, walker = (tid & ~31) < ncell;
+  const int r = wp->cbeg + tid;
+  const int step0 = wp->step0 >= 0 ? wp->step0 : *a.step;
+  const int n_steps = wp->n_steps >= 0 ? wp->n_steps : a.n_steps;
+  const uint64_t pol = l2_policy(a.l2_keep);
+  const int2 gd = walker ? __ldg(wp->grp + (tid >> 5)) : make_int2(0, 0);
+  const uint4* ent = wp->ent + (size_t)gd.x * 32 + lane;
+  const int np = gd.y;
+  uint4 c[kListDepth];
+  auto first = [&]() {
+#pragma unroll
+    for (int i = 0; i < kListDepth; ++i)
+      if (i < np) c[i] = ld_stream4(ent + i * 32, pol);
+  };
+  first();
+  Volts v{};
+  if (own) {
+    const long long T = wp->T;
+    const float* s = wp->st + wp->cell_base + r;
+    v.Vd = s[0 * T];
+    v.Vs = s[7 * T];
+    v.Va = s[15 * T];
+    const int f[kListGateFloats] = {1, 2, 3, 5, 6, 9, 10, 11, 12, 13, 14, 17, 18};
+#pragma unroll
+    for (int k = 0; k < kListGateFloats; ++k) sG[k * BLOCK + tid] = s[f[k] * T];
+    sCa[tid] = wp->ca[wp->cell_base + r];
+  }
+  cluster_sync_all();  // every CTA of the cluster is running before peers write into it
+  if (own) {
+    vbuf[r] = v.Vd * kVScale;
+    for (int p = 0; p < ncta; ++p)
+      if (rank0 + p != (int)me) st_peer(vbuf + r, (unsigned)(rank0 + p), v.Vd * kVScale);
+  }
+  cluster_sync_all();
+
+  const VoltCoef vk = volt_coef(a.P);
+  for (int t = 0; t < n_steps; ++t) {
+    const int step = step0 + t;
+    const float* vcur = vbuf + (t & 1) * a.vcap;
+    float* vnxt = vbuf + ((t + 1) & 1) * a.vcap;
+    // ---- coupling: this lane's row, kListDepth pairs of quads in flight
+    float sum = 0.0f;
+    if (walker) {
+      const float nvc = -v.Vd * kVScale;
+      const float2 nvc2 = make_float2(nvc, nvc);
+      StreamSum<KAHAN> s;
+      for (int p = 0; p < np; p += kListDepth) {
+#pragma unroll
+        for (int i = 0; i < kListDepth; ++i) {
+          if (p + i < np) {
+            float2 x[4];
+            stream_gather<8, true>(vcur, &c[i], x);
+            if (p + i + kListDepth < np) c[i] = ld_stream4(ent + (p + i + kListDepth) * 32, pol);
+            float2 nt = s.start();
+            stream_terms<8, false>(x, nullptr, nvc2, nt);
+            s.add(nt);
+          }
+        }
+      }
+      first();  // the next step's, in flight over the update and the barrier
+      sum = s.total();
+    }
+    if (own) {
+      const float ic = sum * (wp->g * kInvVScale);
+      const float iapp = (step >= wp->pulse_start && step < wp->pulse_end) ? wp->pulse_amp : 0.0f;
+      Gates g;
+      float* sg = sG + tid;
+      g.r = sg[0 * BLOCK];
+      g.s = sg[1 * BLOCK];
+      g.q = sg[2 * BLOCK];
+      g.ICaH = sg[3 * BLOCK];
+      g.gCaL = sg[4 * BLOCK];
+      g.h = sg[5 * BLOCK];
+      g.n = sg[6 * BLOCK];
+      g.p = sg[7 * BLOCK];
+      g.xs = sg[8 * BLOCK];
+      g.k = sg[9 * BLOCK];
+      g.l = sg[10 * BLOCK];
+      g.ha = sg[11 * BLOCK];
+      g.xa = sg[12 * BLOCK];
+      g.Ca = sCa[tid];
+      Currents cur;
+      run_units(a.P, 0xffu, v, g, cur);
+      voltage_step(a.P, vk, v, cur, ic, iapp);
+      const float vds = v.Vd * kVScale;
+      vnxt[r] = vds;
+      for (int p = 0; p < ncta; ++p)
+        if (rank0 + p != (int)me) st_peer(vnxt + r, (unsigned)(rank0 + p), vds);
+      sg[0 * BLOCK] = g.r;
+      sg[1 * BLOCK] = g.s;
+      sg[2 * BLOCK] = g.q;
+      sg[3 * BLOCK] = g.ICaH;
+      sg[5 * BLOCK] = g.h;
+      sg[6 * BLOCK] = g.n;
+      sg[7 * BLOCK] = g.p;
+      sg[8 * BLOCK] = g.xs;
+      sg[9 * BLOCK] = g.k;
+      sg[10 * BLOCK] = g.l;
+      sg[11 * BLOCK] = g.ha;
+      sg[12 * BLOCK] = g.xa;
+      sCa[tid] = g.Ca;
+      if (t + 1 == n_steps) {
+        float* s = wp->st + wp->cell_base + r;
+        s[8 * wp->T] = g.m;
+        s[16 * wp->T] = g.ma;
+      }
+    }
+    if (cl_sync)
+      cluster_sync_all();
+    else
+      __syncthreads();
+  }
+
+  if (own) {
+    const long long T = wp->T;
+    float* s = wp->st + wp->cell_base + r;
+    s[0 * T] = v.Vd;
+    s[7 * T] = v.Vs;
+    s[15 * T] = v.Va;
+    const int f[kListGateFloats] = {1, 2, 3, 5, 6, 9, 10, 11, 12, 13, 14, 17, 18};
+#pragma unroll
+    for (int k = 0; k < kListGateFloats; ++k) s[f[k] * T] = sG[k * BLOCK + tid];
+    wp->ca[wp->cell_base + r] = sCa[tid];
+  }
+  if (tid == 0) {
+    a.cta_ns[2 * blockIdx.x] = t_start;
+    a.cta_ns[2 * blockIdx.x + 1] = globaltimer_ns();
+  }
+}
+
 __global__ void batch_advance(int* step, int n) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *step += n;
 }
@@ -298,6 +535,7 @@ struct BatchGroup {
   int cs = 1;             // CTAs per cluster = CTAs per network
   int cta_off = 0, grid = 0;
   int vcap = 0, res_words = 0;
+  float l2_keep = 1.0f;
   size_t smem = 0;
   int max_active = 0;     // clusters of this group the device runs at once
   int priority = 0;
@@ -314,11 +552,14 @@ struct infoli_batch {
   ModelParams P{};
   int kahan = 0;
   int block = 1024;
+  bool lists = false;  // entry lists (else bitmask rows)
   std::vector<BatchGroup> groups;
   std::vector<BatchCta> cta;
   std::vector<long long> cell_base;
   BatchCta* d_cta = nullptr;
   uint32_t* d_bits = nullptr;
+  uint16_t* d_ent = nullptr;
+  int2* d_grp = nullptr;
   float* d_st = nullptr;
   double* d_ca = nullptr;
   int* d_step = nullptr;
@@ -344,6 +585,11 @@ namespace {
                           __LINE__);                                                               \
   } while (0)
 
+// Of the entry lists that the CTAs on the device read, what L2 (129 MB) is
+// asked to keep from step to step (more was slower for one network's lists).
+constexpr double kBatchL2Bytes = 70e6;
+constexpr int kBatchSms = 152;
+
 uint32_t reverse_bits(uint32_t x) {
   x = ((x >> 1) & 0x55555555u) | ((x & 0x55555555u) << 1);
   x = ((x >> 2) & 0x33333333u) | ((x & 0x33333333u) << 2);
@@ -359,7 +605,7 @@ void batch_release(infoli_batch* b) {
   if (b->graph_exec) cudaGraphExecDestroy(b->graph_exec);
   if (b->graph) cudaGraphDestroy(b->graph);
   for (void* p : {(void*)b->d_cta, (void*)b->d_bits, (void*)b->d_st, (void*)b->d_ca, (void*)b->d_step,
-                  (void*)b->d_cta_ns})
+                  (void*)b->d_cta_ns, (void*)b->d_ent, (void*)b->d_grp})
     if (p) cudaFree(p);
   for (BatchGroup& g : b->groups) {
     if (g.done) cudaEventDestroy(g.done);
@@ -372,7 +618,9 @@ void batch_release(infoli_batch* b) {
   delete b;
 }
 
-const void* kernel_ptr(int block, bool kahan) {
+const void* kernel_ptr(int block, bool kahan, bool lists) {
+  if (lists && block == 512) return kahan ? (const void*)list_kernel<512, true> : (const void*)list_kernel<512, false>;
+  if (lists) return kahan ? (const void*)list_kernel<1024, true> : (const void*)list_kernel<1024, false>;
   if (block == 512) return kahan ? (const void*)batch_kernel<512, true> : (const void*)batch_kernel<512, false>;
   return kahan ? (const void*)batch_kernel<1024, true> : (const void*)batch_kernel<1024, false>;
 }
@@ -380,8 +628,8 @@ const void* kernel_ptr(int block, bool kahan) {
 // Kernel attributes are set before any capture (cudaFuncSetAttribute is not a
 // stream operation).
 cudaError_t set_attrs(int block, size_t smem, int cluster) {
-  for (int k = 0; k < 2; ++k) {
-    const void* fn = kernel_ptr(block, k == 1);
+  for (int k = 0; k < 4; ++k) {
+    const void* fn = kernel_ptr(block, (k & 1) != 0, (k & 2) != 0);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
@@ -406,13 +654,13 @@ void fill_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, int
   cfg.numAttrs = 2;
 }
 
-int max_clusters(int block, int cluster, size_t smem) {
+int max_clusters(int block, int cluster, size_t smem, bool lists) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
   fill_config(cfg, at, cluster, block, cluster, smem, 0, nullptr);
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kernel_ptr(block, false), &cfg) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel_ptr(block, false, lists), &cfg) != cudaSuccess) return 0;
   return n;
 }
 
@@ -424,11 +672,9 @@ cudaError_t launch_group(const infoli_batch* b, const BatchGroup& g, BatchArgs a
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
   fill_config(cfg, at, g.grid, b->block, g.cs, g.smem, g.priority, g.stream);
-  if (b->block == 512)
-    return b->kahan ? cudaLaunchKernelEx(&cfg, batch_kernel<512, true>, a)
-                    : cudaLaunchKernelEx(&cfg, batch_kernel<512, false>, a);
-  return b->kahan ? cudaLaunchKernelEx(&cfg, batch_kernel<1024, true>, a)
-                  : cudaLaunchKernelEx(&cfg, batch_kernel<1024, false>, a);
+  a.l2_keep = g.l2_keep;
+  void* args[] = {&a};
+  return cudaLaunchKernelExC(&cfg, kernel_ptr(b->block, b->kahan != 0, b->lists), args);
 }
 
 }  // namespace
@@ -479,15 +725,48 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
   }
   // time per step of a network ~ its mean row weight (set bits per receiver)
   // plus a constant for the cell update: heavy networks are launched first
+  // and the pair rows of every warp's entry list: its longest row in eights
   std::vector<double> weight(d->n_nets);
+  std::vector<std::vector<int2>> groups(d->n_nets);  // first pair row within the network, pairs
+  std::vector<long long> pair_rows(d->n_nets);
 #pragma omp parallel for schedule(dynamic, 1)
   for (int i = 0; i < d->n_nets; ++i) {
     const int n = d->n_cells[i], wpr = (n + 31) / 32;
+    const int cs = (n + b->block - 1) / b->block, per = (n + cs - 1) / cs, gstride = (per + 31) / 32;
     const uint32_t* src = d->bits + in_base[i];
+    groups[i].assign((size_t)cs * gstride, int2{0, 0});
     long long ones = 0;
-    for (long long k = 0; k < (long long)n * wpr; ++k) ones += __builtin_popcount(src[k]);
+    for (int r = 0; r < n; ++r) {
+      const uint32_t* row = src + (size_t)r * wpr;
+      int deg = 0;
+      for (int w = 0; w < wpr; ++w) deg += __builtin_popcount(row[w]);
+      if (n % 32) deg -= __builtin_popcount(row[wpr - 1] >> (n % 32));
+      if (row[r / 32] >> (r % 32) & 1u) --deg;
+      ones += deg;
+      int& most = groups[i][(size_t)(r / per) * gstride + (r % per) / 32].y;
+      most = std::max(most, (deg + 7) / 8);
+    }
     weight[i] = (double)ones / n + 64.0;
+    long long at = 0;
+    for (int2& g : groups[i]) {
+      g.x = (int)at;
+      at += g.y;
+    }
+    pair_rows[i] = at;
   }
+  long long rows_total = 0, groups_total = 0;
+  std::vector<long long> row_base(d->n_nets), group_base(d->n_nets);
+  for (int i = 0; i < d->n_nets; ++i) {
+    row_base[i] = rows_total;
+    group_base[i] = groups_total;
+    rows_total += pair_rows[i];
+    groups_total += (long long)groups[i].size();
+  }
+  // Entry lists (16 bits per edge, 512 bytes per pair row) unless they would
+  // take more than half of the free memory: then the rows as bits.
+  size_t mem_free = 0, mem_total = 0;
+  cudaMemGetInfo(&mem_free, &mem_total);
+  b->lists = (double)rows_total * 512.0 <= 0.5 * (double)mem_free && rows_total <= INT32_MAX;
   int smem_optin = 0, smem_sm = 0, prio_lo = 0, prio_hi = 0;
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
   cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->device);
@@ -518,11 +797,11 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
       const int wr = (d->n_cells[i] + 31) / 32 + 2;
       if (vbytes + sizeof(uint32_t) * (size_t)wr * b->block <= res_budget) res_rows = std::max(res_rows, wr);
     }
-    g.res_words = res_rows * b->block;
-    g.smem = vbytes + sizeof(uint32_t) * (size_t)g.res_words;
+    g.res_words = b->lists ? 0 : res_rows * b->block;
+    g.smem = b->lists ? list_smem(b->block, g.vcap) : vbytes + sizeof(uint32_t) * (size_t)g.res_words;
     if (g.smem > budget)
       return fail(infoli__fail(INFOLI_ERR_CAPACITY, "batch_create: %zu bytes of shared memory needed", g.smem));
-    if (set_attrs(b->block, budget, max_cs) != cudaSuccess || (g.max_active = max_clusters(b->block, cs, g.smem)) <= 0)
+    if (set_attrs(b->block, budget, max_cs) != cudaSuccess || (g.max_active = max_clusters(b->block, cs, g.smem, b->lists)) <= 0)
       return fail(infoli__fail(INFOLI_ERR_CAPACITY, "batch_create: clusters of %d CTAs of %d threads cannot run",
                                cs, b->block));
     // greatest priority for the largest networks
@@ -548,7 +827,7 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
         w.pulse_start = b->pulse_start;
         w.pulse_end = b->pulse_end;
         w.pulse_amp = b->pulse_amp;
-        w.resident = (w.wpr + 2) * b->block <= g.res_words ? 1 : 0;
+        w.resident = !b->lists && (w.wpr + 2) * b->block <= g.res_words ? 1 : 0;
         w.cl_sync = cs > 1 ? 1 : 0;
         b->cta.push_back(w);
       }
@@ -557,21 +836,32 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
     b->groups.push_back(g);
   }
 
-  // Device bitmasks, word-major (word w of receiver r at base + w * n + r),
-  // most-significant bit first, two zero words after every row.
-  std::vector<uint32_t> tb((size_t)bits_total, 0u);
+  // Bitmask rows on the device: as given for the lists' packing, else
+  // word-major (word w of receiver r at base + w * n + r), most-significant bit
+  // first, two zero words after every row.
+  std::vector<uint32_t> tb(b->lists ? 0 : (size_t)bits_total, 0u);
+  if (!b->lists) {
 #pragma omp parallel for schedule(dynamic, 1)
-  for (int i = 0; i < d->n_nets; ++i) {
-    const int n = d->n_cells[i], wpr = (n + 31) / 32;
-    const uint32_t* src = d->bits + in_base[i];
-    uint32_t* dst = tb.data() + bits_base[i];
-    for (int r = 0; r < n; ++r)
-      for (int wd = 0; wd < wpr; ++wd) {
-        uint32_t x = src[(size_t)r * wpr + wd];
-        if (wd == r / 32) x &= ~(1u << (r % 32));  // no self-coupling
-        if (wd == wpr - 1 && n % 32) x &= (1u << (n % 32)) - 1u;
-        dst[(size_t)wd * n + r] = reverse_bits(x);
-      }
+    for (int i = 0; i < d->n_nets; ++i) {
+      const int n = d->n_cells[i], wpr = (n + 31) / 32;
+      const uint32_t* src = d->bits + in_base[i];
+      uint32_t* dst = tb.data() + bits_base[i];
+      for (int r = 0; r < n; ++r)
+        for (int wd = 0; wd < wpr; ++wd) {
+          uint32_t x = src[(size_t)r * wpr + wd];
+          if (wd == r / 32) x &= ~(1u << (r % 32));  // no self-coupling
+          if (wd == wpr - 1 && n % 32) x &= (1u << (n % 32)) - 1u;
+          dst[(size_t)wd * n + r] = reverse_bits(x);
+        }
+    }
+  }
+  const uint32_t* up_bits = b->lists ? d->bits : tb.data();
+  const size_t up_words = b->lists ? (size_t)in_total : tb.size();
+  std::vector<int2> grp;
+  if (b->lists) {
+    grp.reserve((size_t)groups_total);
+    for (int i = 0; i < d->n_nets; ++i)
+      for (int2 g : groups[i]) grp.push_back(int2{(int)(g.x + row_base[i]), g.y});
   }
   std::vector<float> st((size_t)INFOLI_NSTATE * b->total);
   if (d->init_state) {
@@ -582,7 +872,9 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
   }
   std::vector<double> ca(st.begin() + 4 * b->total, st.begin() + 5 * b->total);
   if (cudaMalloc((void**)&b->d_cta, sizeof(BatchCta) * b->cta.size()) != cudaSuccess ||
-      cudaMalloc((void**)&b->d_bits, sizeof(uint32_t) * std::max<size_t>(1, tb.size())) != cudaSuccess ||
+      cudaMalloc((void**)&b->d_bits, sizeof(uint32_t) * std::max<size_t>(1, up_words)) != cudaSuccess ||
+      (b->lists && (cudaMalloc((void**)&b->d_ent, (size_t)std::max(1LL, rows_total) * 512) != cudaSuccess ||
+                    cudaMalloc((void**)&b->d_grp, sizeof(int2) * grp.size()) != cudaSuccess)) ||
       cudaMalloc((void**)&b->d_st, sizeof(float) * st.size()) != cudaSuccess ||
       cudaMalloc((void**)&b->d_ca, sizeof(double) * b->total) != cudaSuccess ||
       cudaMalloc((void**)&b->d_step, sizeof(int)) != cudaSuccess ||
@@ -591,16 +883,40 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
   for (BatchCta& w : b->cta) {
     w.st = b->d_st;
     w.ca = b->d_ca;
-    w.bits = b->d_bits + bits_base[w.net];
+    w.bits = b->lists ? nullptr : b->d_bits + bits_base[w.net];
     w.T = b->total;
+    if (b->lists) {
+      const int per = (w.n + w.ncta - 1) / w.ncta, gstride = (per + 31) / 32;
+      w.ent = reinterpret_cast<const uint4*>(b->d_ent);
+      w.grp = b->d_grp + group_base[w.net] + (size_t)w.rank * gstride;
+    }
   }
+  // the CTAs on the device at a time read their lists from L2 where they fit
+  const double in_flight = (double)rows_total * 512.0 * std::min(1.0, (double)kBatchSms / (double)b->cta.size());
+  for (BatchGroup& g : b->groups) g.l2_keep = (float)std::min(1.0, kBatchL2Bytes / std::max(1.0, in_flight));
   if (cudaMemcpy(b->d_cta, b->cta.data(), sizeof(BatchCta) * b->cta.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b->d_bits, tb.data(), sizeof(uint32_t) * tb.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(b->d_bits, up_bits, sizeof(uint32_t) * up_words, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(b->d_st, st.data(), sizeof(float) * st.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(b->d_ca, ca.data(), sizeof(double) * ca.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(b->d_step, 0, sizeof(int)) != cudaSuccess ||
       cudaMemset(b->d_cta_ns, 0, sizeof(unsigned long long) * 2 * b->cta.size()) != cudaSuccess)
     return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: upload failed"));
+  if (b->lists) {
+    cudaError_t e = cudaMemcpy(b->d_grp, grp.data(), sizeof(int2) * grp.size(), cudaMemcpyHostToDevice);
+    // lanes without a receiver read entry 0
+    if (e == cudaSuccess) e = cudaMemset(b->d_ent, 0, (size_t)std::max(1LL, rows_total) * 512);
+    for (int i = 0; i < d->n_nets && e == cudaSuccess; ++i) {
+      const int n = d->n_cells[i], cs = (n + b->block - 1) / b->block, per = (n + cs - 1) / cs;
+      batch_pack_kernel<<<(n + kPackWarps - 1) / kPackWarps, kPackWarps * 32>>>(
+          b->d_bits + in_base[i], n, per, (per + 31) / 32, b->d_grp + group_base[i], b->d_ent);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess)
+      return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: entry lists: %s", cudaGetErrorString(e)));
+    cudaFree(b->d_bits);
+    b->d_bits = nullptr;
+  }
   if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess)

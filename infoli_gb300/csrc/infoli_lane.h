@@ -4,6 +4,7 @@
 // steps.  Internal to libinfoli_gpu.so (infoli_batch.cu, infoli_serve.cu).
 #pragma once
 #include <cstdint>
+#include <vector_types.h>
 
 namespace infoli {
 
@@ -20,6 +21,11 @@ struct alignas(16) BatchCta {
   int wpr;           // bitmask words per receiver row, ceil(n / 32)
   float* st;         // state: field f of the network's cell c at st[f * T + cell_base + c]
   double* ca;        // Ca2+ of the network's cell c at ca[cell_base + c] (FP64 between launches)
+  // entry lists (batches): group g of the CTA (receivers 32 g ..) is grp[g] =
+  // {first pair row, pairs}, a pair row being 32 lanes x 8 entries of ent (16-bit
+  // byte offsets into the V_dend buffer); null: bitmask rows
+  const uint4* ent;
+  const int2* grp;
   const uint32_t* bits;  // word w of receiver r at bits[w * n + r] (two zero words after each row)
   long long T;       // SoA stride of st
   long long cell_base;
