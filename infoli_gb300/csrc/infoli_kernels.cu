@@ -531,8 +531,6 @@ __global__ void __launch_bounds__(BLOCK, 1) step_kernel(const __grid_constant__ 
   const bool unit_warp = warp < ngroups * U;
   const int ucell_l = (warp / U) * 32 + lane;  // local cell of this unit lane
   const bool unit_lane = unit_warp && ucell_l < w.n_cells;
-  unsigned umask = 0;
-  for (int u = warp % U; u < kUnits; u += U) umask |= 1u << u;
   // stamped mode: threads from poll_first on gather the neighbours' words --
   // the warps left over by the gate units when they can take every word in
   // one batch of loads (they poll while the units compute), else every thread
@@ -693,27 +691,8 @@ __global__ void __launch_bounds__(BLOCK, 1) step_kernel(const __grid_constant__ 
     if (poll_early) poll_issue_lean(a, a.vll[step & 1], pw, tid, (int)blockDim.x, tbuf, shp.dup_words, early);
 
     // ---------------- gate units (old voltages only)
-    if (unit_lane) {
-      Volts v;
-      v.Vd = sVd[ucell_l];
-      v.Vs = sVs[ucell_l];
-      v.Va = sVa[ucell_l];
-      Currents cur;
-      Gates gs = load_gates(sG, sCa, cap, ucell_l, umask);
-      run_units(a.P, umask, v, gs, cur);
-      store_gates(sG, sCa, cap, ucell_l, umask, gs);
-      if (umask & 0x01u) sI[0 * cap + ucell_l] = cur.I_h;
-      if (umask & 0x02u) {
-        sI[1 * cap + ucell_l] = cur.I_CaH;
-        sI[2 * cap + ucell_l] = cur.I_K_Ca;
-      }
-      if (umask & 0x04u) sI[3 * cap + ucell_l] = cur.I_CaL;
-      if (umask & 0x08u) sI[4 * cap + ucell_l] = cur.I_Na_s;
-      if (umask & 0x10u) sI[5 * cap + ucell_l] = cur.I_Kdr_s;
-      if (umask & 0x20u) sI[6 * cap + ucell_l] = cur.I_K_s;
-      if (umask & 0x40u) sI[7 * cap + ucell_l] = cur.I_Na_a;
-      if (umask & 0x80u) sI[8 * cap + ucell_l] = cur.I_K_a;
-    }
+    if (unit_lane)
+      for (int u = warp % U; u < kUnits; u += U) unit_step(a.P, u, sVd, sG, sCa, sI, cap, ucell_l);
     const uint64_t t_units = prof ? clock64() : 0;
 
     // ---------------- phase A: gap-junction coupling
@@ -845,16 +824,7 @@ __global__ void __launch_bounds__(BLOCK, 1) step_kernel(const __grid_constant__ 
         iapp = (ls >= my_onset && ls < my_onset + a.stim_dur) ? my_amp : 0.0f;
       else
         iapp = a.stim_table[(size_t)t * np + ocell];
-      Currents cur;
-      cur.I_h = sI[0 * cap + tid];
-      cur.I_CaH = sI[1 * cap + tid];
-      cur.I_K_Ca = sI[2 * cap + tid];
-      cur.I_CaL = sI[3 * cap + tid];
-      cur.I_Na_s = sI[4 * cap + tid];
-      cur.I_Kdr_s = sI[5 * cap + tid];
-      cur.I_K_s = sI[6 * cap + tid];
-      cur.I_Na_a = sI[7 * cap + tid];
-      cur.I_K_a = sI[8 * cap + tid];
+      const Currents cur = load_currents(sI, cap, tid);
       Volts v;
       v.Vd = sVd[tid];
       v.Vs = sVs[tid];

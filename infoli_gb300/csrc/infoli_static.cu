@@ -183,15 +183,7 @@ __global__ void __launch_bounds__(kNoAllocBlock, 2) noalloc_step_kernel(const __
     const int items = ((nc + 31) >> 5) * kUnits;
     for (int it = warp; it < items; it += kNoAllocWarps) {
       const int k = (it / kUnits) * 32 + lane;
-      const unsigned m = 1u << (it % kUnits);
-      if (k < nc) {
-        const Volts u = {sV[k], sV[cap + k], sV[2 * cap + k]};
-        Currents cur;
-        Gates gs = load_gates(sG, sCa, cap, k, m);
-        run_units(a.P, m, u, gs, cur);
-        store_gates(sG, sCa, cap, k, m, gs);
-        store_currents(sI, cap, k, m, cur);
-      }
+      if (k < nc) unit_step(a.P, it % kUnits, sV, sG, sCa, sI, cap, k);
     }
     if (tid == kNoAllocBlock - 32) {
       const uint64_t t0 = globaltimer_ns();

@@ -13,74 +13,89 @@ constexpr float kNegLog2eOver100 = -0.014426950408889634f;  // -log2(e)/100
 constexpr float kVScale = 0.12011224087864497f;
 constexpr float kInvVScale = 8.325546111576978f;
 
-// Gate state of local cell r from / to shared memory (field f at
-// sG[f * cap + r]), only the fields the units in `mask` use.
-__device__ __forceinline__ Gates load_gates(const float* sG, const double* sCa, int cap, int r, unsigned mask) {
-  Gates g;
-  if (mask & 0x01u) g.q = sG[F_Q * cap + r];
-  if (mask & 0x02u) {
-    g.r = sG[F_R * cap + r];
-    g.s = sG[F_S * cap + r];
-    g.Ca = sCa[r];
-    g.ICaH = sG[F_ICAH * cap + r];
+// One gate unit of local cell r on shared-memory state: its gates (field f at
+// sG[f * cap + r], Ca2+ in sCa), the compartment's voltage (sV: V_dend, V_soma,
+// V_axon, cap apart) in, its currents (current k at sI[k * cap + r]) out.  One
+// block of code per unit behind one switch: with loads, arithmetic and stores
+// each behind eight tests of a unit mask, a warp went through 32 branches for
+// one unit.
+__device__ __forceinline__ void unit_step(const ModelParams& P, int u, const float* sV, float* sG, double* sCa,
+                                          float* sI, int cap, int r) {
+  Volts v{};
+  Gates g{};
+  Currents c{};
+  switch (u) {
+    case 0:
+      v.Vd = sV[r];
+      g.q = sG[F_Q * cap + r];
+      unit_q(P, v, g, c);
+      sG[F_Q * cap + r] = g.q;
+      sI[0 * cap + r] = c.I_h;
+      break;
+    case 1:
+      v.Vd = sV[r];
+      g.r = sG[F_R * cap + r];
+      g.s = sG[F_S * cap + r];
+      g.Ca = sCa[r];
+      g.ICaH = sG[F_ICAH * cap + r];
+      unit_rs(P, v, g, c);
+      sG[F_R * cap + r] = g.r;
+      sG[F_S * cap + r] = g.s;
+      sCa[r] = g.Ca;
+      sG[F_ICAH * cap + r] = g.ICaH;
+      sI[1 * cap + r] = c.I_CaH;
+      sI[2 * cap + r] = c.I_K_Ca;
+      break;
+    case 2:
+      v.Vs = sV[cap + r];
+      g.k = sG[F_K * cap + r];
+      g.l = sG[F_L * cap + r];
+      g.gCaL = sG[F_GCAL * cap + r];
+      unit_kl(P, v, g, c);
+      sG[F_K * cap + r] = g.k;
+      sG[F_L * cap + r] = g.l;
+      sI[3 * cap + r] = c.I_CaL;
+      break;
+    case 3:
+      v.Vs = sV[cap + r];
+      g.h = sG[F_H * cap + r];
+      unit_mh(P, v, g, c);
+      sG[F_M * cap + r] = g.m;
+      sG[F_H * cap + r] = g.h;
+      sI[4 * cap + r] = c.I_Na_s;
+      break;
+    case 4:
+      v.Vs = sV[cap + r];
+      g.n = sG[F_N * cap + r];
+      g.p = sG[F_P * cap + r];
+      unit_np(P, v, g, c);
+      sG[F_N * cap + r] = g.n;
+      sG[F_P * cap + r] = g.p;
+      sI[5 * cap + r] = c.I_Kdr_s;
+      break;
+    case 5:
+      v.Vs = sV[cap + r];
+      g.xs = sG[F_XS * cap + r];
+      unit_xs(P, v, g, c);
+      sG[F_XS * cap + r] = g.xs;
+      sI[6 * cap + r] = c.I_K_s;
+      break;
+    case 6:
+      v.Va = sV[2 * cap + r];
+      g.ha = sG[F_HA * cap + r];
+      unit_mha(P, v, g, c);
+      sG[F_MA * cap + r] = g.ma;
+      sG[F_HA * cap + r] = g.ha;
+      sI[7 * cap + r] = c.I_Na_a;
+      break;
+    default:
+      v.Va = sV[2 * cap + r];
+      g.xa = sG[F_XA * cap + r];
+      unit_xa(P, v, g, c);
+      sG[F_XA * cap + r] = g.xa;
+      sI[8 * cap + r] = c.I_K_a;
+      break;
   }
-  if (mask & 0x04u) {
-    g.k = sG[F_K * cap + r];
-    g.l = sG[F_L * cap + r];
-    g.gCaL = sG[F_GCAL * cap + r];
-  }
-  if (mask & 0x08u) g.h = sG[F_H * cap + r];
-  if (mask & 0x10u) {
-    g.n = sG[F_N * cap + r];
-    g.p = sG[F_P * cap + r];
-  }
-  if (mask & 0x20u) g.xs = sG[F_XS * cap + r];
-  if (mask & 0x40u) g.ha = sG[F_HA * cap + r];
-  if (mask & 0x80u) g.xa = sG[F_XA * cap + r];
-  return g;
-}
-
-__device__ __forceinline__ void store_gates(float* sG, double* sCa, int cap, int r, unsigned mask, const Gates& g) {
-  if (mask & 0x01u) sG[F_Q * cap + r] = g.q;
-  if (mask & 0x02u) {
-    sG[F_R * cap + r] = g.r;
-    sG[F_S * cap + r] = g.s;
-    sCa[r] = g.Ca;
-    sG[F_ICAH * cap + r] = g.ICaH;
-  }
-  if (mask & 0x04u) {
-    sG[F_K * cap + r] = g.k;
-    sG[F_L * cap + r] = g.l;
-  }
-  if (mask & 0x08u) {
-    sG[F_M * cap + r] = g.m;
-    sG[F_H * cap + r] = g.h;
-  }
-  if (mask & 0x10u) {
-    sG[F_N * cap + r] = g.n;
-    sG[F_P * cap + r] = g.p;
-  }
-  if (mask & 0x20u) sG[F_XS * cap + r] = g.xs;
-  if (mask & 0x40u) {
-    sG[F_MA * cap + r] = g.ma;
-    sG[F_HA * cap + r] = g.ha;
-  }
-  if (mask & 0x80u) sG[F_XA * cap + r] = g.xa;
-}
-
-// Unit currents of local cell r in shared memory (current k at sI[k * cap + r]).
-__device__ __forceinline__ void store_currents(float* sI, int cap, int r, unsigned mask, const Currents& c) {
-  if (mask & 0x01u) sI[0 * cap + r] = c.I_h;
-  if (mask & 0x02u) {
-    sI[1 * cap + r] = c.I_CaH;
-    sI[2 * cap + r] = c.I_K_Ca;
-  }
-  if (mask & 0x04u) sI[3 * cap + r] = c.I_CaL;
-  if (mask & 0x08u) sI[4 * cap + r] = c.I_Na_s;
-  if (mask & 0x10u) sI[5 * cap + r] = c.I_Kdr_s;
-  if (mask & 0x20u) sI[6 * cap + r] = c.I_K_s;
-  if (mask & 0x40u) sI[7 * cap + r] = c.I_Na_a;
-  if (mask & 0x80u) sI[8 * cap + r] = c.I_K_a;
 }
 
 __device__ __forceinline__ Currents load_currents(const float* sI, int cap, int r) {
