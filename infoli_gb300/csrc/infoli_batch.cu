@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batch_kernel(const __grid
       const float iapp = (step >= wp->pulse_start && step < wp->pulse_end) ? wp->pulse_amp : 0.0f;
       // ---- fused compartment update
       Currents cur;
-      run_units(a.P, 0xffu, v, gs, cur);
+      run_units(a.P, v, gs, cur);
       voltage_step(a.P, vk, v, cur, ic, iapp);
       const float vds = v.Vd * kVScale;
       vnxt[r] = vds;
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) list_kernel(const __grid_
       g.xa = sg[12 * BLOCK];
       g.Ca = sCa[tid];
       Currents cur;
-      run_units(a.P, 0xffu, v, g, cur);
+      run_units(a.P, v, g, cur);
       voltage_step(a.P, vk, v, cur, ic, iapp);
       const float vds = v.Vd * kVScale;
       vnxt[r] = vds;

@@ -423,7 +423,7 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
   // INFOLI_THREADS=512|1024 overrides.
   int want_threads = 0;
   if (const char* ts = getenv("INFOLI_THREADS")) want_threads = atoi(ts) == 512 ? 512 : 1024;
-  // stream plans run 1024 threads; their clusters only where the simulation may
+  // stream plans have a CTA size of their own; their clusters only where the simulation may
   // have the whole GPU (a share of the SMs need not come in whole clusters)
   pin.no_stream = want_threads == 512 ? 1 : 0;
   for (int i = 0; i < 2; ++i) pin.cluster_ctas[i] = d->grid > 0 ? 0 : max_stream_ctas(2 << i, pin.smem_budget);
@@ -447,7 +447,8 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
   }
   if (!planned) return fail(infoli__fail(INFOLI_ERR_ARG, "%s", perr.c_str()));
   cudaError_t occ_err = cudaSuccess;
-  const int cores = max_coresident_ctas(s->plan.threads, s->plan.smem_bytes, &occ_err);
+  const int cores = s->plan.shape.gather == 4 ? max_stream_ctas(s->plan.shape.cluster, s->plan.smem_bytes)
+                                              : max_coresident_ctas(s->plan.threads, s->plan.smem_bytes, &occ_err);
   if (cores < s->plan.grid)
     return fail(infoli__fail(INFOLI_ERR_CUDA, "plan needs %d co-resident CTAs of %d threads and %lld bytes of shared "
                              "memory, device allows %d (%s)", s->plan.grid, s->plan.threads,

@@ -1055,7 +1055,7 @@ __global__ void __launch_bounds__(BLOCK, 1) gather_kernel(const __grid_constant_
         iapp = a.stim_table[(size_t)t * np + cell];
       Gates g = gather_load_gates(sGt, sCa, BLOCK, tid);
       Currents cur;
-      run_units(a.P, 0xffu, v, g, cur);
+      run_units(a.P, v, g, cur);
       voltage_step(a.P, vk, v, cur, ic, iapp);
       gather_store_gates(sGt, sCa, BLOCK, tid, g);
       a.vd[(step + 1) & 1][cell] = v.Vd;
@@ -1221,7 +1221,7 @@ __global__ void __launch_bounds__(BLOCK, 1) tgather_kernel(const __grid_constant
       else
         iapp = a.stim_table[(size_t)t * np + cell];
       Currents cur;
-      run_units(a.P, 0xffu, v, g, cur);
+      run_units(a.P, v, g, cur);
       voltage_step(a.P, vk, v, cur, ic, iapp);
       a.vd[(step + 1) & 1][cell] = v.Vd;
       if (trace_now) {
@@ -1463,7 +1463,7 @@ __global__ void __launch_bounds__(BLOCK, 1) bits_kernel(const __grid_constant__ 
       else
         iapp = a.stim_table[(size_t)st * np + cell];
       Currents cur;
-      run_units(a.P, 0xffu, v, g, cur);
+      run_units(a.P, v, g, cur);
       voltage_step(a.P, vk, v, cur, ic, iapp);
       a.vd[(step + 1) & 1][cell] = v.Vd;
       a.vds[(step + 1) & 1][cell] = v.Vd * kVScale;

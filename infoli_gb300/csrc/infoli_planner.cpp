@@ -771,7 +771,7 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     std::vector<int> hist, lens;
     for (int k = 1; k <= 4; ++k)
       for (double f : {1.0, 1.02, 1.04, 1.06, 1.08, 1.11, 1.15, 1.2, 1.3})
-        lens.push_back(std::max(16, (int)std::ceil(f * (double)idx.size() / (1024.0 * k))));
+        lens.push_back(std::max(16, (int)std::ceil(f * (double)idx.size() / ((double)kStreamThreads * k))));
     for (int len : {16, 24, 32, 48, 64, 96, 128, 256, 512, 1024, 4096, 1 << 30}) lens.push_back(len);
     std::sort(lens.begin(), lens.end());
     lens.erase(std::unique(lens.begin(), lens.end()), lens.end());

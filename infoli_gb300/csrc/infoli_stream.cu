@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
       g.ha = st[F_HA * np];
       g.xa = st[F_XA * np];
       Currents cur;
-      run_units(a.P, 0xffu, v, g, cur);
+      run_units(a.P, v, g, cur);
       st[F_Q * np] = g.q;
       st[F_R * np] = g.r;
       st[F_S * np] = g.s;
