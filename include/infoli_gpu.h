@@ -230,8 +230,8 @@ int infoli_sim_set_stimulus_table(infoli_sim* s, const float* table, int rows, i
  * n_steps explicit-Euler steps.  When trace_every > 0, the selected
  * quantities are recorded after every step whose index is a multiple of
  * trace_every (the reference's print rule, :682) and delivered to cb, in step
- * order, from the calling thread; device->host trace copies run on a side
- * stream while the next steps compute. */
+ * order, from the calling thread; the kernel writes the rows to pinned host
+ * memory, and long traces are delivered while the next steps compute. */
 int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, infoli_trace_cb cb,
                    void* user);
 

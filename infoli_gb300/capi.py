@@ -485,12 +485,14 @@ class Simulation:
             _check(self._L.infoli_sim_run_into(self._h, int(n_steps), 0, 0, None, 0, None))
             return {}
         s0 = self.step
-        rows = sum(1 for t in range(s0, s0 + n_steps) if t % trace_every == 0)
-        out = np.zeros((max(rows, 1), len(names), self.n), dtype=np.float32)
+        rows = max(0, (s0 + n_steps - 1) // trace_every - (s0 - 1) // trace_every)  # multiples in [s0, s0 + n_steps)
+        out = np.empty((max(rows, 1), len(names), self.n), dtype=np.float32)
         got = C.c_int(0)
         _check(self._L.infoli_sim_run_into(self._h, int(n_steps), int(trace_every), int(what), _p(out),
                                            out.size, C.byref(got)))
         assert got.value == rows
+        if len(names) == 1:
+            return {names[0]: out[:rows, 0]}
         return {nm: out[:rows, i, :].copy() for i, nm in enumerate(names)}
 
     def launch(self, n_steps):

@@ -1,6 +1,12 @@
 // C ABI of libinfoli_gpu.so: simulation handles, device memory, the chunked
-// launch loop and trace streaming (pinned host slots filled by
-// cudaMemcpyAsync on a side stream while the next chunk of steps computes).
+// launch loop and trace streaming (pinned host slots that the kernel writes;
+// one is delivered while the next launch fills the other).  A call's own
+// costs count most where a run is short: 20 steps of 50 cells with one trace
+// row took 73 us, 30 of them steps, with the trace copied from the device on
+// a side stream, three memsets per launch and the error word fetched by a
+// copy of its own; 49 us without these.  Rows written across the link at every
+// step cost less than the copies did (200 rows of 100,000 cells: 15.3 -> 8.1
+// ms; of 1,000 cells: 480 -> 400 us).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,7 +48,7 @@ constexpr int kMaxStepsPerLaunch = 8192;
 // step.  16,000 cells at 30 % (154 MB of entries): 38.1 us per step with 70 MB,
 // 38.3 with 50, 39.8 with 85, 42.2 with 100.
 constexpr double kStreamL2Bytes = 70e6;
-constexpr size_t kTraceSlotBytes = 64u << 20;
+constexpr size_t kTraceSlotBytes = 64u << 20;  // pinned host memory, written by the kernel
 
 // Device memory of simulation handles comes from one stream-ordered pool per
 // device (cudaMallocFromPoolAsync / cudaFreeAsync on the handle's stream).
@@ -137,11 +143,12 @@ struct infoli_sim {
   int* d_err = nullptr;
   unsigned long long* d_prof = nullptr;  // per-CTA phase timers when profiling is on
   // trace ring
-  float* d_trace[2] = {nullptr, nullptr};
   float* h_trace[2] = {nullptr, nullptr};
-  size_t trace_slot_floats = 0;
-  cudaStream_t stream = nullptr, side = nullptr;
-  cudaEvent_t ev_kernel[2] = {nullptr, nullptr}, ev_copy[2] = {nullptr, nullptr};
+  size_t trace_floats[2] = {0, 0};  // room in each slot
+  int* h_err = nullptr;             // pinned: where a run's kernels report an error, or null
+  bool stamps_valid = false;  // the stamped words are those of the current state and step
+  cudaStream_t stream = nullptr;
+  cudaEvent_t ev_kernel[2] = {nullptr, nullptr};
   cudaEvent_t ev_t0 = nullptr, ev_t1 = nullptr;
   float last_ms = 0.0f;
   int last_launches = 0;
@@ -155,10 +162,9 @@ namespace {
 void release(infoli_sim* s) {
   if (!s) return;
   cudaSetDevice(s->device);
-  if (s->side) cudaStreamSynchronize(s->side);
   void* dptrs[] = {s->d_cta,   s->d_tiles,  s->d_chunks, s->d_cell_slots, s->d_edges,
                    s->d_edge_g, s->d_vd[0], s->d_vd[1],  s->d_st,         s->d_ca,
-                   s->d_cell_amp, s->d_cell_onset, s->d_bar, s->d_err, s->d_trace[0], s->d_trace[1],
+                   s->d_cell_amp, s->d_cell_onset, s->d_bar, s->d_err,
                    s->d_prof, s->d_probes, s->d_vll[0], s->d_vll[1], s->d_gdesc, s->d_stim_table,
                    s->d_gcol, s->d_perm, s->d_io, s->d_vds[0], s->d_vds[1]};
   if (s->stream) {
@@ -166,12 +172,11 @@ void release(infoli_sim* s) {
       if (p) cudaFreeAsync(p, s->stream);
     cudaStreamSynchronize(s->stream);
   }
-  for (float* h : s->h_trace)
+  for (void* h : {(void*)s->h_trace[0], (void*)s->h_trace[1], (void*)s->h_err})
     if (h) cudaFreeHost(h);
-  for (cudaEvent_t e : {s->ev_kernel[0], s->ev_kernel[1], s->ev_copy[0], s->ev_copy[1], s->ev_t0, s->ev_t1})
+  for (cudaEvent_t e : {s->ev_kernel[0], s->ev_kernel[1], s->ev_t0, s->ev_t1})
     if (e) cudaEventDestroy(e);
   if (s->stream) cudaStreamDestroy(s->stream);
-  if (s->side) cudaStreamDestroy(s->side);
   delete s;
 }
 
@@ -230,6 +235,7 @@ int state_io_buffer(infoli_sim* s) {
 // caller's buffer is pinned), then the scatter on the device.  Returns after
 // the copy has completed, so the caller may reuse its buffer.
 int upload_state(infoli_sim* s, const float* state /*19 x n*/) {
+  s->stamps_valid = false;
   const int n = s->n;
   const long long total = (long long)INFOLI_NSTATE * n;
   if (int rc = state_io_buffer(s)) return rc;
@@ -327,11 +333,9 @@ int count_rows(int step0, int n_steps, int every) {
 
 int nq_of(int what) { return !!(what & INFOLI_TRACE_AXON) + !!(what & INFOLI_TRACE_SOMA) + !!(what & INFOLI_TRACE_DEND); }
 
-int check_device_error(infoli_sim* s) {
-  int err = 0;
-  CK(cudaMemcpyAsync(&err, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  CK(cudaStreamSynchronize(s->stream));
+int report_device_error(infoli_sim* s, int err) {
   if (err != DEV_OK) {
+    s->stamps_valid = false;
     cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream);
     if (err == DEV_ERR_CONFIG)
       return infoli__fail(INFOLI_ERR_CUDA, "the step kernel was launched without the clusters of its plan");
@@ -340,6 +344,40 @@ int check_device_error(infoli_sim* s) {
                         : err == DEV_ERR_STAMP_TIMEOUT ? "stamped V_dend exchange timeout"
                                                        : "tile copy timeout");
   }
+  return INFOLI_OK;
+}
+
+int check_device_error(infoli_sim* s) {
+  int err = 0;
+  CK(cudaMemcpyAsync(&err, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CK(cudaStreamSynchronize(s->stream));
+  return report_device_error(s, err);
+}
+
+// Before a launch: the barrier count back to zero; the stamped words wiped,
+// so that no stale stamp can match a step of the launch.  A launch leaves its
+// last voltages under the stamp of the step that the next one begins with, and
+// that one publishes the same words again, so they are wiped only where the
+// state was set or a launch failed since.
+int reset_exchange(infoli_sim* s) {
+  if (!s->plan.shape.stamped) {
+    CK(cudaMemsetAsync(s->d_bar, 0, sizeof(unsigned), s->stream));
+  } else if (!s->stamps_valid) {
+    CK(cudaMemsetAsync(s->d_vll[0], 0xff, (size_t)s->n_pad * sizeof(unsigned long long), s->stream));
+    CK(cudaMemsetAsync(s->d_vll[1], 0xff, (size_t)s->n_pad * sizeof(unsigned long long), s->stream));
+  }
+  return INFOLI_OK;
+}
+
+// Trace slot i with room for `floats`.
+int trace_slot(infoli_sim* s, int i, size_t floats) {
+  if (s->trace_floats[i] >= floats) return INFOLI_OK;
+  CK(cudaStreamSynchronize(s->stream));
+  if (s->h_trace[i]) cudaFreeHost(s->h_trace[i]);
+  s->h_trace[i] = nullptr;
+  s->trace_floats[i] = 0;
+  CK(cudaMallocHost((void**)&s->h_trace[i], floats * sizeof(float)));
+  s->trace_floats[i] = floats;
   return INFOLI_OK;
 }
 
@@ -388,8 +426,7 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
     return rc;
   };
   if (cudaSetDevice(s->device) != cudaSuccess) return fail(infoli__fail(INFOLI_ERR_CUDA, "cudaSetDevice failed"));
-  if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess)
+  if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(infoli__fail(INFOLI_ERR_CUDA, "stream creation failed"));
 
   // ---- plan
@@ -508,8 +545,7 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
   }
   if ((rc = upload_state_copies(s, st))) return fail(rc);
   for (int i = 0; i < 2; ++i)
-    if (cudaEventCreateWithFlags(&s->ev_kernel[i], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&s->ev_copy[i], cudaEventDisableTiming) != cudaSuccess)
+    if (cudaEventCreateWithFlags(&s->ev_kernel[i], cudaEventDisableTiming) != cudaSuccess)
       return fail(infoli__fail(INFOLI_ERR_CUDA, "event creation failed"));
   if (cudaEventCreate(&s->ev_t0) != cudaSuccess || cudaEventCreate(&s->ev_t1) != cudaSuccess)
     return fail(infoli__fail(INFOLI_ERR_CUDA, "event creation failed"));
@@ -620,27 +656,21 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
     const size_t need = (size_t)rows_cap * row_floats;
     const int rows_needed = count_rows(0, launch_steps + trace_every, trace_every) + 1;
     const size_t want = std::min(need, (size_t)rows_needed * row_floats);
-    if (s->trace_slot_floats < want) {
-      CK(cudaStreamSynchronize(s->stream));
-      for (int i = 0; i < 2; ++i) {
-        if (s->d_trace[i]) cudaFreeAsync(s->d_trace[i], s->stream);
-        if (s->h_trace[i]) cudaFreeHost(s->h_trace[i]);
-        s->d_trace[i] = nullptr;
-        s->h_trace[i] = nullptr;
-      }
-      for (int i = 0; i < 2; ++i) {
-        CK(pool_alloc(&s->d_trace[i], want * sizeof(float), s->device, s->stream));
-        CK(cudaMallocHost((void**)&s->h_trace[i], want * sizeof(float)));
-      }
-      s->trace_slot_floats = want;
-    }
+    for (int i = 0; i < (n_steps > launch_steps ? 2 : 1); ++i)
+      if (int rc = trace_slot(s, i, want)) return rc;
   }
+  if (!s->h_err && cudaMallocHost((void**)&s->h_err, sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    s->h_err = nullptr;
+  }
+  if (s->h_err) *s->h_err = DEV_OK;
 
   StepArgs a;
   fill_args(s, &a);
   a.trace_every = trace_every > 0 ? trace_every : 0;
   a.trace_mask = trace_what;
   a.trace_nq = nq;
+  a.err_host = s->h_err;
 
   struct Pending {
     int slot, step0, rows;
@@ -650,7 +680,7 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
   CK(cudaEventRecord(s->ev_t0, s->stream));
   int done = 0, li = 0;
   auto drain = [&](const Pending& p) -> int {
-    CK(cudaEventSynchronize(s->ev_copy[p.slot]));
+    CK(cudaEventSynchronize(s->ev_kernel[p.slot]));
     // rows are the multiples of trace_every in the launch's step range
     int st = ((p.step0 + trace_every - 1) / trace_every) * trace_every;
     for (int row = 0; row < p.rows; ++row, st += trace_every) {
@@ -667,27 +697,20 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
     a.step0 = s->step + done;
     a.n_steps = len;
     a.stim_table = table_at(s, a.step0);
-    a.trace = nq ? s->d_trace[slot] : nullptr;
+    a.trace = nq ? s->h_trace[slot] : nullptr;
     const int rows = count_rows(a.step0, len, trace_every);
-    // the slot's previous contents must have been copied and consumed
+    // the slot's previous contents must have been consumed
     if (pend.size() >= 2) {
       int rc = drain(pend.front());
       if (rc) return rc;
       pend.erase(pend.begin());
     }
-    CK(cudaMemsetAsync(s->d_bar, 0, sizeof(unsigned), s->stream));
-    if (s->plan.shape.stamped) {  // no stale stamp may match a step of this launch
-      CK(cudaMemsetAsync(s->d_vll[0], 0xff, (size_t)s->n_pad * sizeof(unsigned long long), s->stream));
-      CK(cudaMemsetAsync(s->d_vll[1], 0xff, (size_t)s->n_pad * sizeof(unsigned long long), s->stream));
-    }
+    if (int rc = reset_exchange(s)) return rc;
     CK(launch_step_kernel(a, s->plan.grid, s->plan.threads, s->stream));
+    s->stamps_valid = true;
     ++launches;
     if (rows > 0) {
       CK(cudaEventRecord(s->ev_kernel[slot], s->stream));
-      CK(cudaStreamWaitEvent(s->side, s->ev_kernel[slot], 0));
-      CK(cudaMemcpyAsync(s->h_trace[slot], s->d_trace[slot], (size_t)rows * row_floats * sizeof(float),
-                         cudaMemcpyDeviceToHost, s->side));
-      CK(cudaEventRecord(s->ev_copy[slot], s->side));
       pend.push_back({slot, a.step0, rows});
     }
     done += len;
@@ -704,7 +727,7 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
   CK(cudaEventElapsedTime(&ms, s->ev_t0, s->ev_t1));
   s->last_ms = ms;
   s->last_launches = launches;
-  int rc = check_device_error(s);
+  int rc = s->h_err ? report_device_error(s, *s->h_err) : check_device_error(s);
   if (rc) return rc;
   s->step += n_steps;
   return INFOLI_OK;
@@ -728,12 +751,9 @@ int infoli_sim_launch(infoli_sim* s, int n_steps) {
     a.step0 = s->step + done;
     a.n_steps = len;
     a.stim_table = table_at(s, a.step0);
-    CK(cudaMemsetAsync(s->d_bar, 0, sizeof(unsigned), s->stream));
-    if (s->plan.shape.stamped) {
-      CK(cudaMemsetAsync(s->d_vll[0], 0xff, (size_t)s->n_pad * sizeof(unsigned long long), s->stream));
-      CK(cudaMemsetAsync(s->d_vll[1], 0xff, (size_t)s->n_pad * sizeof(unsigned long long), s->stream));
-    }
+    if (int rc = reset_exchange(s)) return rc;
     CK(launch_step_kernel(a, s->plan.grid, s->plan.threads, s->stream));
+    s->stamps_valid = true;
     done += len;
   }
   CK(cudaEventRecord(s->ev_t1, s->stream));
@@ -819,7 +839,6 @@ int infoli_sim_get_state(infoli_sim* s, float* out) {
   infoli__clear_error();
   if (!s || !out) return infoli__fail(INFOLI_ERR_ARG, "get_state: bad argument");
   CK(cudaSetDevice(s->device));
-  CK(cudaStreamSynchronize(s->stream));
   // gather on the device into the ABI layout, then one device->host copy
   const int n = s->n;
   const long long total = (long long)INFOLI_NSTATE * n;

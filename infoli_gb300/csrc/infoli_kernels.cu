@@ -32,7 +32,7 @@ __device__ __forceinline__ bool wait_tile(const StepArgs& a, uint64_t* bar, unsi
   const uint64_t t0 = globaltimer_ns();
   while (!mbar_try_wait(bar, parity)) {
     if (globaltimer_ns() - t0 > a.timeout_ns) {
-      atomicCAS(a.err, 0, DEV_ERR_COPY_TIMEOUT);
+      device_error(a, DEV_ERR_COPY_TIMEOUT);
       return false;
     }
   }
@@ -64,7 +64,7 @@ __device__ __forceinline__ bool grid_sync(const StepArgs& a, unsigned target, vo
           break;
         }
         if (globaltimer_ns() - t0 > a.timeout_ns) {
-          atomicCAS(a.err, 0, DEV_ERR_BARRIER_TIMEOUT);
+          device_error(a, DEV_ERR_BARRIER_TIMEOUT);
           *s_abort = 1;
           break;
         }
@@ -227,7 +227,7 @@ __device__ __forceinline__ bool poll_finish_lean(const StepArgs& a, const unsign
     if (t0 == 0) {
       t0 = now;
     } else if (now - t0 > a.timeout_ns || ld_relaxed_gpu(a.err) != 0) {
-      atomicCAS(a.err, 0, DEV_ERR_STAMP_TIMEOUT);
+      device_error(a, DEV_ERR_STAMP_TIMEOUT);
       return false;
     }
 #pragma unroll
@@ -267,7 +267,7 @@ __device__ __forceinline__ bool poll_retry(const StepArgs& a, const unsigned lon
     if (t0 == 0) {
       t0 = now;
     } else if (now - t0 > a.timeout_ns || ld_relaxed_gpu(a.err) != 0) {
-      atomicCAS(a.err, 0, DEV_ERR_STAMP_TIMEOUT);
+      device_error(a, DEV_ERR_STAMP_TIMEOUT);
       return false;
     }
 #pragma unroll
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(BLOCK, 1) step_kernel(const __grid_constant__ 
   int row = 0;
   unsigned bar_target = 0;
   if (LL && owner) {
-    // publish V^step0 with its stamp (the host cleared both slots before launch)
+    // publish V^step0 with its stamp (the slots hold that same word or none of this launch's stamps)
     if ((int)blockIdx.x != a.stall_cta)
       st_relaxed_gpu_u64(a.vll[a.step0 & 1] + cell, pack_stamp(sVd[tid], (unsigned)a.step0));
   }

@@ -71,6 +71,7 @@ struct StepArgs {
   // synchronisation
   unsigned* bar;              // grid barrier counter (zeroed before launch)
   int* err;                   // device error word
+  int* err_host;              // pinned host memory that learns of an error too, or null
   unsigned long long timeout_ns;
   int stall_cta;              // failure-detection test hook: this CTA never arrives at grid
                               // barriers and never publishes stamped words (-1: none), so
@@ -89,6 +90,12 @@ enum {
   PROF_STAGE = 0, PROF_COUPLE, PROF_UPDATE, PROF_BARRIER, PROF_STEPS, PROF_UNITS, PROF_SPAN_NS,
   PROF_SPAN_CYCLES, kProfSlots = 8
 };
+
+// Records the launch's first error.
+__device__ __forceinline__ void device_error(const StepArgs& a, int code) {
+  atomicCAS(a.err, 0, code);
+  if (a.err_host) *reinterpret_cast<volatile int*>(a.err_host) = code;
+}
 
 // Dynamic shared memory needed for a launch.
 size_t step_kernel_smem(const StepArgs& a);

@@ -182,7 +182,7 @@ __device__ __forceinline__ bool stream_wait(const StepArgs& a, uint64_t* bar, un
   while (!mbar_try_wait(bar, parity)) {
     if (*s_abort) return false;
     if (globaltimer_ns() - t0 > a.timeout_ns) {
-      atomicCAS(a.err, 0, DEV_ERR_COPY_TIMEOUT);
+      device_error(a, DEV_ERR_COPY_TIMEOUT);
       return false;
     }
   }
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   // kernel without its attributes) would read shared memory of CTAs that are
   // not there: every CTA returns instead.
   if (cluster_ctas() != (unsigned)cs) {
-    if (tid == 0) atomicCAS(a.err, 0, DEV_ERR_CONFIG);
+    if (tid == 0) device_error(a, DEV_ERR_CONFIG);
     return;
   }
   const CtaWork w = a.cta[blockIdx.x];
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
         const uint64_t t0 = globaltimer_ns();
         while (ld_acquire_gpu(a.bar) < bar_target) {
           if (ld_relaxed_gpu(a.err) != 0 || globaltimer_ns() - t0 > a.timeout_ns) {
-            atomicCAS(a.err, 0, DEV_ERR_BARRIER_TIMEOUT);
+            device_error(a, DEV_ERR_BARRIER_TIMEOUT);
             *(volatile int*)&s_abort = 1;
             ok = false;
             break;

@@ -1,0 +1,61 @@
+"""What one launch leaves for the next (the exchange words of V_dend, the trace slots in host memory): runs split into
+launches anywhere, states set between launches, errors between launches, traces longer than a slot."""
+import numpy as np
+import pytest
+
+from helpers import CONF, hetero_state
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ig(built):
+    import infoli_gb300
+
+    assert infoli_gb300.device_count() >= 1
+    return infoli_gb300
+
+
+@pytest.mark.parametrize("mode", ["stamped", "barrier", "stream"])
+@pytest.mark.parametrize("n", [1, 50, 1300])
+def test_a_new_state_between_launches_starts_afresh(ig, n, mode, monkeypatch):
+    conf = O.read_parameters(CONF)
+    monkeypatch.setenv("INFOLI_SYNC", mode)
+    monkeypatch.setenv("INFOLI_WAIT_TIMEOUT_MS", "300")
+    rp, col = ig.gen_uniform(n, 0.1 if n > 2 else 1.0, 2)
+    first, second = hetero_state(conf, n, 1), hetero_state(conf, n, 2)
+    with ig.Simulation(n, conf, rp, col, init_state=second) as sim:  # no stimulus before step 20,000
+        want, state = sim.run(24, 1, ig.TRACE_DEND)["dend"], sim.get_state()
+    with ig.Simulation(n, conf, rp, col, init_state=first) as sim:
+        for steps in (1, 2, 5):  # even and odd steps to begin the next launch with
+            sim.run(steps)
+            sim.set_state(second)
+            got = np.concatenate([sim.run(k, 1, ig.TRACE_DEND)["dend"] for k in (1, 1, 3, 19)])
+            assert np.array_equal(got, want)
+            assert np.array_equal(sim.get_state(), state)
+        if n > 1000 and mode != "stream":  # a launch that failed leaves words of steps that are run again
+            monkeypatch.setenv("INFOLI_STALL_CTA", "1")
+            with pytest.raises(ig.InfoliError):
+                sim.run(10)
+            monkeypatch.delenv("INFOLI_STALL_CTA")
+            sim.set_state(second)
+            sim.launch(5)
+            sim.launch(19)
+            sim.sync()
+            assert np.array_equal(sim.get_state(), state)
+
+
+@pytest.mark.parametrize("what", [2, 7])
+def test_traces_longer_than_a_slot(ig, what):
+    conf, n, steps = O.read_parameters(CONF), 61001, 300
+    rp, col, g = ig.gen_fixed_degree(n, 8, 4, (0.02, 0.06))
+    st0 = hetero_state(conf, n, 3)
+    with ig.Simulation(n, conf, rp, col, g=g, init_state=st0) as sim:
+        whole = sim.run(steps, 1, what)
+        assert sim.last_run_stats()[1] > 1
+    with ig.Simulation(n, conf, rp, col, g=g, init_state=st0) as sim:
+        parts = [sim.run(k, 1, what) for k in (1, 49, 250)]
+        assert sim.run(0, 1, what)["soma"].shape == (0, n)
+    for name, rows in whole.items():
+        assert rows.flags.c_contiguous and np.array_equal(rows, np.concatenate([p[name] for p in parts]))
