@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <memory>
 #include <numeric>
 
 namespace infoli {
@@ -88,6 +89,36 @@ std::vector<TileSpan> make_tiles(const std::vector<int>& u, int cap, int n_pad) 
   return t;
 }
 
+// Calls f(sender, conductance or 0) for receiver c's edges, senders ascending,
+// edges of one sender in the caller's order.
+template <class F>
+void for_sorted_row(const PlanInput& in, int c, F f) {
+  const int64_t e0 = in.row_ptr[c], e1 = in.row_ptr[c + 1];
+  if (std::is_sorted(in.col + e0, in.col + e1)) {
+    for (int64_t e = e0; e < e1; ++e) f(in.col[e], in.g ? in.g[e] : 0.0f);
+    return;
+  }
+  std::vector<std::pair<int, float>> snd;
+  snd.reserve((size_t)(e1 - e0));
+  for (int64_t e = e0; e < e1; ++e) snd.push_back({in.col[e], in.g ? in.g[e] : 0.0f});
+  std::stable_sort(snd.begin(), snd.end(),
+                   [](const std::pair<int, float>& x, const std::pair<int, float>& y) { return x.first < y.first; });
+  for (const auto& x : snd) f(x.first, x.second);
+}
+
+// The distinct senders of receivers [c0, c1), ascending.
+std::vector<int> unique_senders(const PlanInput& in, int c0, int c1) {
+  std::vector<uint64_t> seen(((size_t)in.n + 63) / 64, 0);
+  for (int64_t e = in.row_ptr[c0]; e < in.row_ptr[c1]; ++e) seen[(size_t)in.col[e] >> 6] |= 1ull << (in.col[e] & 63);
+  size_t count = 0;
+  for (uint64_t m : seen) count += (size_t)__builtin_popcountll(m);
+  std::vector<int> u;
+  u.reserve(count);
+  for (size_t k = 0; k < seen.size(); ++k)
+    for (uint64_t m = seen[k]; m; m &= m - 1) u.push_back((int)(k * 64 + (size_t)__builtin_ctzll(m)));
+  return u;
+}
+
 // Build the packed lane-chunk tables of a stamped, resident plan (see
 // infoli_plan.h): per receiver, its senders (ascending) become byte offsets
 // into the CTA's window (its sorted unique senders, win[b], one float each),
@@ -98,6 +129,11 @@ std::vector<TileSpan> make_tiles(const std::vector<int>& u, int cap, int n_pad) 
 // are rewritten to the lane-chunks (receiver-major, so a receiver's partial
 // sums stay contiguous and in sender order); the last group of a CTA is
 // filled with dummy chunks that write one spare slot.
+// What a simulation or a request waits for before its first step: 3,114 cells
+// and 2.2 million edges took 47 ms (four requests planned at once), 7 now,
+// with the entries not yet dealt held as bits by bank instead of searched, an
+// open bank taken before a longer path is tried, and the tile tables built
+// only for the plans that keep them.
 void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::vector<std::vector<int>>& win,
                  int dup_words, int cells_cap) {
   const bool edge_g = in.g != nullptr;
@@ -117,18 +153,27 @@ void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::v
     std::vector<uint16_t>& pe = loc[b].pe;
     std::vector<float>& pg = loc[b].pg;
     const std::vector<int>& u = win[b];
+    std::unique_ptr<uint16_t[]> place(new uint16_t[(size_t)in.n]);  // of the window's senders
+    for (size_t j = 0; j < u.size(); ++j) place[(size_t)u[j]] = (uint16_t)(L.tiles + sizeof(float) * j);
     struct LaneChunk {
       int recv, slot;
-      std::vector<std::pair<uint16_t, float>> e;
+      size_t begin;  // its entries: off[begin .. begin + count)
+      int count;
     };
     std::vector<LaneChunk> lc;
+    std::vector<uint16_t> off;
+    std::vector<float> val;
+    const size_t edges = (size_t)(in.row_ptr[w.cell_begin + w.n_cells] - in.row_ptr[w.cell_begin]);
+    off.reserve(edges);
+    if (edge_g) val.reserve(edges);
     int slot = 0, prev_begin = 0;
     for (int r = 0; r < w.n_cells; ++r) {
       const int c = w.cell_begin + r;
-      std::vector<std::pair<int, float>> snd;
-      for (int64_t e = in.row_ptr[c]; e < in.row_ptr[c + 1]; ++e) snd.push_back({in.col[e], edge_g ? in.g[e] : 0.0f});
-      std::stable_sort(snd.begin(), snd.end(),
-                       [](const std::pair<int, float>& x, const std::pair<int, float>& y) { return x.first < y.first; });
+      const size_t row = off.size();
+      for_sorted_row(in, c, [&](int s, float gv) {
+        off.push_back(place[(size_t)s]);
+        if (edge_g) val.push_back(gv);
+      });
       // each receiver's partial slots start on a 4-slot (16-byte) boundary; the
       // gaps are zeroed once per launch, so the update can read them 4 at a time.
       // Consecutive receivers start an odd number of 16-byte units apart (an
@@ -139,18 +184,8 @@ void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::v
       if (r > 0 && (((slot - prev_begin) >> 2) & 1) == 0) slot += 4;
       prev_begin = slot;
       P.cell_slots[c].begin = slot;
-      size_t j = 0;  // window position of the sender (senders ascending)
-      for (size_t k = 0; k < snd.size(); k += kLaneEdges) {
-        LaneChunk ch;
-        ch.recv = r;
-        ch.slot = slot++;
-        for (size_t q = k; q < std::min(snd.size(), k + kLaneEdges); ++q) {
-          const int s = snd[q].first;
-          while (u[j] < s) ++j;
-          ch.e.push_back({(uint16_t)(L.tiles + sizeof(float) * j), snd[q].second});
-        }
-        lc.push_back(std::move(ch));
-      }
+      for (size_t k = row; k < off.size(); k += kLaneEdges)
+        lc.push_back({r, slot++, k, (int)std::min<size_t>(kLaneEdges, off.size() - k)});
       P.cell_slots[c].count = slot - P.cell_slots[c].begin;
     }
     const int dummy_slot = (slot + 3) & ~3;  // past the last receiver's 4-slot block
@@ -159,16 +194,25 @@ void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::v
     const int ng = (int)(lc.size() + 31) / 32;
     w.n_groups = ng;
     for (int g = 0; g < ng; ++g) {
-      // the 32 chunks of this group (dummies past the end)
-      std::vector<std::vector<std::pair<uint16_t, float>>> rem(32);
-      std::vector<uint16_t> pad(32);
+      // the 32 chunks of this group (dummies past the end).  The entries of a
+      // lane's chunk not yet dealt as bits of a word: all of them, and those
+      // whose word lies in each bank
+      unsigned left[32] = {0}, has[32] = {0}, in_bank[32][32] = {{0}};
+      size_t begin[32] = {0};
+      uint16_t pad[32];
       for (int l = 0; l < 32; ++l) {
         const size_t ci = (size_t)g * 32 + l;
         int2_t d;
         if (ci < lc.size()) {
           d.x = lc[ci].slot;
           d.y = lc[ci].recv;
-          rem[l] = lc[ci].e;
+          begin[l] = lc[ci].begin;
+          for (int q = 0; q < lc[ci].count; ++q) {
+            const int b2 = (off[begin[l] + q] >> 2) & 31;
+            left[l] |= 1u << q;
+            in_bank[l][b2] |= 1u << q;
+            has[l] |= 1u << b2;
+          }
         } else {
           d.x = dummy_slot;
           d.y = 0;
@@ -176,100 +220,75 @@ void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::v
         pad[l] = (uint16_t)(L.vown + sizeof(float) * ((size_t)kScaledVArray * cells_cap + d.y));
         gdesc.push_back(d);
       }
+      const size_t base = pe.size();  // transposed quads: ((g * kQuads + k / 4) * 32 + l) * 4 + k % 4
+      pe.resize(base + kGroupEntries);
+      if (edge_g) pg.resize(base + kGroupEntries);
       // bank-distinct dealing, position by position: lanes whose chunk is
       // exhausted read their padding word (lanes of one receiver share it);
       // the others are matched to free banks by augmenting paths (Kuhn), so
       // each position has as many conflict-free lanes as the remaining
       // entries allow; unmatched lanes take any entry
-      std::vector<std::pair<uint16_t, float>> cell(32 * kLaneEdges);
       for (int k = 0; k < kLaneEdges; ++k) {
-        int bank_word[32];
-        for (int b2 = 0; b2 < 32; ++b2) bank_word[b2] = -1;
+        const size_t at = base + (size_t)(k / 4) * 128 + k % 4;
+        unsigned taken = 0;  // banks already claimed by padding words
         for (int l = 0; l < 32; ++l)
-          if (rem[l].empty()) {
-            cell[l * kLaneEdges + k] = {pad[l], 0.0f};
-            const int wd = pad[l] >> 2;
-            if (bank_word[wd & 31] < 0) bank_word[wd & 31] = wd;
+          if (!left[l]) {
+            pe[at + 4 * l] = pad[l];
+            taken |= 1u << ((pad[l] >> 2) & 31);
           }
         // an entry can be read from the first copy (bank b) or, when the
         // window is duplicated, from the second (bank b + 16)
-        const unsigned dup_mask = dup_words ? 0xffffffffu : 0u;
-        auto banks_of = [&](uint16_t off) {
-          const int b2 = (off >> 2) & 31;
-          return (1u << b2) | (dup_mask & (1u << ((b2 + 16) & 31)));
-        };
-        unsigned taken = 0;  // banks already claimed by padding words
-        for (int b2 = 0; b2 < 32; ++b2)
-          if (bank_word[b2] >= 0) taken |= 1u << b2;
         unsigned adj[32];
-        for (int l = 0; l < 32; ++l) {
-          adj[l] = 0;
-          for (const auto& e : rem[l]) adj[l] |= banks_of(e.first);
-          adj[l] &= ~taken;
-        }
+        for (int l = 0; l < 32; ++l) adj[l] = (has[l] | (dup_words ? has[l] << 16 | has[l] >> 16 : 0u)) & ~taken;
         int match_bank[32];  // bank -> lane
-        for (int b2 = 0; b2 < 32; ++b2) match_bank[b2] = -1;
+        unsigned open = ~0u;  // banks of no lane yet
         for (int l = 0; l < 32; ++l) {
           if (!adj[l]) continue;
           unsigned seen = 0;
-          // iterative augmenting-path search from lane l
+          // iterative augmenting-path search from lane l, an open bank first
           struct Frame {
-            int lane;
-            unsigned left;
+            int lane, bank;
           };
           Frame stack[33];
-          int prev_bank[33];
           int sp = 0;
-          stack[0] = {l, adj[l]};
-          bool done = false;
-          while (sp >= 0 && !done) {
+          stack[0].lane = l;
+          while (sp >= 0) {
             Frame& f = stack[sp];
-            const unsigned cand = f.left & ~seen;
+            if (const unsigned now = adj[f.lane] & open) {
+              f.bank = __builtin_ctz(now);
+              open &= ~(1u << f.bank);
+              for (int q = sp; q >= 0; --q) match_bank[stack[q].bank] = stack[q].lane;
+              break;
+            }
+            const unsigned cand = adj[f.lane] & ~seen;
             if (!cand) {
               --sp;
               continue;
             }
-            const int b2 = __builtin_ctz(cand);
-            f.left &= ~(1u << b2);
-            seen |= 1u << b2;
-            prev_bank[sp] = b2;
-            if (match_bank[b2] < 0) {
-              for (int q = sp; q >= 0; --q) match_bank[prev_bank[q]] = stack[q].lane;
-              done = true;
-            } else if (sp + 1 < 33) {
-              ++sp;
-              stack[sp] = {match_bank[b2], adj[match_bank[b2]]};
-            }
+            f.bank = __builtin_ctz(cand);
+            seen |= 1u << f.bank;
+            stack[++sp].lane = match_bank[f.bank];
           }
         }
         int lane_bank[32];
         for (int l = 0; l < 32; ++l) lane_bank[l] = -1;
         for (int b2 = 0; b2 < 32; ++b2)
-          if (match_bank[b2] >= 0) lane_bank[match_bank[b2]] = b2;
+          if (!(open >> b2 & 1u)) lane_bank[match_bank[b2]] = b2;
         for (int l = 0; l < 32; ++l) {
-          if (rem[l].empty()) continue;
-          size_t q = 0;
-          std::pair<uint16_t, float> pick = rem[l][0];
-          if (lane_bank[l] >= 0) {
-            while (!(banks_of(rem[l][q].first) & (1u << lane_bank[l]))) ++q;
-            pick = rem[l][q];
-            if (((pick.first >> 2) & 31) != lane_bank[l])  // the matched bank is the second copy's
-              pick.first = (uint16_t)(pick.first + sizeof(float) * (size_t)dup_words);
-          }
-          cell[l * kLaneEdges + k] = pick;
-          rem[l].erase(rem[l].begin() + q);
+          if (!left[l]) continue;
+          const int b2 = lane_bank[l];
+          const unsigned from = b2 < 0 ? left[l] : in_bank[l][b2] | (dup_words ? in_bank[l][b2 ^ 16] : 0u);
+          const int q = __builtin_ctz(from);
+          const uint16_t o = off[begin[l] + q];
+          const int own = (o >> 2) & 31;
+          // (the second copy's word where that is the matched bank)
+          pe[at + 4 * l] = b2 < 0 || own == b2 ? o : (uint16_t)(o + sizeof(float) * (size_t)dup_words);
+          if (edge_g) pg[at + 4 * l] = val[begin[l] + q];
+          left[l] &= ~(1u << q);
+          in_bank[l][own] &= ~(1u << q);
+          if (!in_bank[l][own]) has[l] &= ~(1u << own);
         }
       }
-      // transposed quads: ((g * kQuads + k / 4) * 32 + l) * 4 + k % 4
-      const size_t base = pe.size();
-      pe.resize(base + kGroupEntries);
-      if (edge_g) pg.resize(base + kGroupEntries);
-      for (int l = 0; l < 32; ++l)
-        for (int k = 0; k < kLaneEdges; ++k) {
-          const size_t at = base + ((size_t)(k / 4) * 32 + l) * 4 + (k % 4);
-          pe[at] = cell[l * kLaneEdges + k].first;
-          if (edge_g) pg[at] = cell[l * kLaneEdges + k].second;
-        }
     }
   }
   std::vector<int2_t> gdesc;
@@ -684,7 +703,6 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
   sh.gather = 4;
   sh.nbuf = 1;
   std::vector<int> starts;
-  int max_rows = 0;
   for (int cs = 1; cs <= kStreamMaxCluster; cs *= 2) {
     int most = in.grid_max;
     if (cs > 1) {
@@ -707,7 +725,6 @@ static bool make_stream_plan(const PlanInput& in, Plan* out, std::string* err) {
     sh.cells_cap = ((mr + cs - 1) / cs + 31) & ~31;
     if (stream_layout(sh).total > in.smem_budget) continue;
     starts.swap(st);
-    max_rows = mr;
     break;
   }
   if (starts.empty()) {
@@ -1001,6 +1018,112 @@ static bool stream_plan_wanted(const PlanInput& in) {
   return e >= (double)kStreamMinDegree * n;
 }
 
+// The tile and chunk tables of a barrier plan: CTAs of the cells between
+// `starts`, each with its tiles, rows cut by tile and then by chunk.
+static void tile_tables(const PlanInput& in, const std::vector<int>& starts,
+                        const std::vector<std::vector<TileSpan>>& tiles, int chunk, Plan* out) {
+  Plan& P = *out;
+  const int ctas = (int)starts.size() - 1;
+  const int64_t E = in.row_ptr[in.n];
+  // Each CTA's tables are built on their own (in parallel, indices local to
+  // the CTA), then concatenated in CTA order with their offsets applied.
+  struct Local {
+    std::vector<TileDesc> tiles;
+    std::vector<ChunkDesc> chunks;
+    std::vector<uint16_t> edges;
+    std::vector<float> edge_g;
+    int n_slots = 0;
+  };
+  std::vector<Local> loc(ctas);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int b = 0; b < ctas; ++b) {
+    Local& L = loc[b];
+    const std::vector<TileSpan>& tl = tiles[b];
+    // senders of the CTA's cells, each cell's sorted by id, end to end
+    std::vector<std::pair<int, float>> snd;
+    snd.reserve((size_t)(in.row_ptr[starts[b + 1]] - in.row_ptr[starts[b]]));
+    struct Pending {
+      int tile, recv, slot;
+      size_t begin, count;  // range in snd
+    };
+    std::vector<Pending> pend;
+    int slot = 0;
+    for (int c = starts[b]; c < starts[b + 1]; ++c) {
+      const int r = c - starts[b];
+      const size_t s0 = snd.size();
+      for (int64_t e = in.row_ptr[c]; e < in.row_ptr[c + 1]; ++e) snd.push_back({in.col[e], in.g ? in.g[e] : 0.0f});
+      std::stable_sort(snd.begin() + s0, snd.end(),
+                       [](const std::pair<int, float>& x, const std::pair<int, float>& y) { return x.first < y.first; });
+      P.cell_slots[c].begin = slot;
+      size_t k = s0;
+      for (int j = 0; j < (int)tl.size(); ++j) {
+        const size_t t0 = k;
+        while (k < snd.size() && snd[k].first < tl[j].hi) ++k;
+        for (size_t o = t0; o < k; o += chunk) pend.push_back({j, r, slot++, o, std::min(k - o, (size_t)chunk)});
+      }
+      P.cell_slots[c].count = slot - P.cell_slots[c].begin;
+    }
+    L.n_slots = slot;
+    // tile-major; inside a tile, larger chunks first (round-robin to warps)
+    std::stable_sort(pend.begin(), pend.end(), [](const Pending& x, const Pending& y) {
+      if (x.tile != y.tile) return x.tile < y.tile;
+      return x.count > y.count;
+    });
+    L.edges.reserve(snd.size());
+    if (in.g) L.edge_g.reserve(snd.size());
+    size_t pi = 0;
+    for (int j = 0; j < (int)tl.size(); ++j) {
+      TileDesc td{};
+      td.lo = tl[j].lo;
+      td.nfloats = tl[j].hi - tl[j].lo;
+      td.chunk_begin = (int)L.chunks.size();
+      while (pi < pend.size() && pend[pi].tile == j) {
+        const Pending& pc = pend[pi++];
+        ChunkDesc cd{};
+        cd.edge_begin = (int)L.edges.size();
+        cd.slot = pc.slot;
+        cd.recv = pc.recv;
+        cd.count = (int)pc.count;
+        for (size_t q = pc.begin; q < pc.begin + pc.count; ++q) {
+          L.edges.push_back((uint16_t)(snd[q].first - td.lo));
+          if (in.g) L.edge_g.push_back(snd[q].second);
+        }
+        L.chunks.push_back(cd);
+      }
+      td.chunk_end = (int)L.chunks.size();
+      L.tiles.push_back(td);
+    }
+  }
+  P.edges.reserve(E);
+  if (in.g) P.edge_g.reserve(E);
+  int slot_base = 0;
+  for (int b = 0; b < ctas; ++b) {
+    Local& L = loc[b];
+    CtaWork& w = P.cta[b];
+    w.tile_begin = (int)P.tiles.size();
+    w.n_tiles = (int)L.tiles.size();
+    w.slot_begin = slot_base;
+    w.n_slots = L.n_slots;
+    const int chunk0 = (int)P.chunks.size(), edge0 = (int)P.edges.size();
+    for (TileDesc td : L.tiles) {
+      td.chunk_begin += chunk0;
+      td.chunk_end += chunk0;
+      P.tiles.push_back(td);
+    }
+    for (ChunkDesc cd : L.chunks) {
+      cd.edge_begin += edge0;
+      P.chunks.push_back(cd);
+    }
+    P.edges.insert(P.edges.end(), L.edges.begin(), L.edges.end());
+    if (in.g) P.edge_g.insert(P.edge_g.end(), L.edge_g.begin(), L.edge_g.end());
+    slot_base += L.n_slots;
+    std::vector<TileDesc>().swap(L.tiles);
+    std::vector<ChunkDesc>().swap(L.chunks);
+    std::vector<uint16_t>().swap(L.edges);
+    std::vector<float>().swap(L.edge_g);
+  }
+}
+
 bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
   const int n = in.n;
   if (n <= 0 || !in.row_ptr || in.threads <= 0 || in.threads % 32 || in.grid_max <= 0) {
@@ -1086,11 +1209,7 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
 #pragma omp parallel for schedule(dynamic, 1) reduction(max : max_window)
   for (int b = 0; b < ctas; ++b) {
     std::vector<int>& u = uniq[b];
-    u.reserve((size_t)(in.row_ptr[starts[b + 1]] - in.row_ptr[starts[b]]));
-    for (int c = starts[b]; c < starts[b + 1]; ++c)
-      for (int64_t e = in.row_ptr[c]; e < in.row_ptr[c + 1]; ++e) u.push_back(in.col[e]);
-    std::sort(u.begin(), u.end());
-    u.erase(std::unique(u.begin(), u.end()), u.end());
+    u = unique_senders(in, starts[b], starts[b + 1]);
     if (!u.empty()) max_window = std::max(max_window, ((u.back() + 4) & ~3) - (u.front() & ~3));
   }
   if (!in.cta_starts && stream_plan_wanted(in)) {
@@ -1115,18 +1234,17 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
     int s = 0;
     for (int c = starts[b]; c < starts[b + 1]; ++c) {
       // edges of c split by tile, then by chunk size
-      int64_t e = in.row_ptr[c], e1 = in.row_ptr[c + 1];
-      std::vector<int> snd(in.col + e, in.col + e1);
-      std::sort(snd.begin(), snd.end());
-      size_t k = 0;
-      for (const TileSpan& t : tl) {
-        int cnt = 0;
-        while (k < snd.size() && snd[k] < t.hi) {
-          ++cnt;
-          ++k;
-        }
-        s += (cnt + chunk - 1) / chunk;
+      if (tl.size() == 1) {
+        s += (int)((in.row_ptr[c + 1] - in.row_ptr[c] + chunk - 1) / chunk);
+        continue;
       }
+      size_t j = 0;
+      int cnt = 0;
+      for_sorted_row(in, c, [&](int sender, float) {
+        for (; sender >= tl[j].hi; ++j, cnt = 0) s += (cnt + chunk - 1) / chunk;
+        ++cnt;
+      });
+      s += (cnt + chunk - 1) / chunk;
     }
     return s;
   };
@@ -1176,108 +1294,14 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
   P.max_slots = max_slots;
   P.smem_bytes = plan_smem_bytes(tile_cap, nbuf, threads, cells_cap, max_slots, in.kahan);
   P.cell_slots.assign(n, CellSlots{0, 0});
-  // Each CTA's tables are built on their own (in parallel, indices local to
-  // the CTA), then concatenated in CTA order with their offsets applied.
-  struct Local {
-    std::vector<TileDesc> tiles;
-    std::vector<ChunkDesc> chunks;
-    std::vector<uint16_t> edges;
-    std::vector<float> edge_g;
-    int n_slots = 0;
-  };
-  std::vector<Local> loc(ctas);
-#pragma omp parallel for schedule(dynamic, 1)
   for (int b = 0; b < ctas; ++b) {
-    Local& L = loc[b];
-    const std::vector<TileSpan>& tl = tiles[b];
-    // senders of the CTA's cells, each cell's sorted by id, end to end
-    std::vector<std::pair<int, float>> snd;
-    snd.reserve((size_t)(in.row_ptr[starts[b + 1]] - in.row_ptr[starts[b]]));
-    struct Pending {
-      int tile, recv, slot;
-      size_t begin, count;  // range in snd
-    };
-    std::vector<Pending> pend;
-    int slot = 0;
-    for (int c = starts[b]; c < starts[b + 1]; ++c) {
-      const int r = c - starts[b];
-      const size_t s0 = snd.size();
-      for (int64_t e = in.row_ptr[c]; e < in.row_ptr[c + 1]; ++e) snd.push_back({in.col[e], in.g ? in.g[e] : 0.0f});
-      std::stable_sort(snd.begin() + s0, snd.end(),
-                       [](const std::pair<int, float>& x, const std::pair<int, float>& y) { return x.first < y.first; });
-      P.cell_slots[c].begin = slot;
-      size_t k = s0;
-      for (int j = 0; j < (int)tl.size(); ++j) {
-        const size_t t0 = k;
-        while (k < snd.size() && snd[k].first < tl[j].hi) ++k;
-        for (size_t o = t0; o < k; o += chunk) pend.push_back({j, r, slot++, o, std::min(k - o, (size_t)chunk)});
-      }
-      P.cell_slots[c].count = slot - P.cell_slots[c].begin;
-    }
-    L.n_slots = slot;
-    // tile-major; inside a tile, larger chunks first (round-robin to warps)
-    std::stable_sort(pend.begin(), pend.end(), [](const Pending& x, const Pending& y) {
-      if (x.tile != y.tile) return x.tile < y.tile;
-      return x.count > y.count;
-    });
-    L.edges.reserve(snd.size());
-    if (in.g) L.edge_g.reserve(snd.size());
-    size_t pi = 0;
-    for (int j = 0; j < (int)tl.size(); ++j) {
-      TileDesc td{};
-      td.lo = tl[j].lo;
-      td.nfloats = tl[j].hi - tl[j].lo;
-      td.chunk_begin = (int)L.chunks.size();
-      while (pi < pend.size() && pend[pi].tile == j) {
-        const Pending& pc = pend[pi++];
-        ChunkDesc cd{};
-        cd.edge_begin = (int)L.edges.size();
-        cd.slot = pc.slot;
-        cd.recv = pc.recv;
-        cd.count = (int)pc.count;
-        for (size_t q = pc.begin; q < pc.begin + pc.count; ++q) {
-          L.edges.push_back((uint16_t)(snd[q].first - td.lo));
-          if (in.g) L.edge_g.push_back(snd[q].second);
-        }
-        L.chunks.push_back(cd);
-      }
-      td.chunk_end = (int)L.chunks.size();
-      L.tiles.push_back(td);
-    }
-  }
-  P.edges.reserve(E);
-  if (in.g) P.edge_g.reserve(E);
-  int slot_base = 0;
-  for (int b = 0; b < ctas; ++b) {
-    Local& L = loc[b];
     CtaWork w{};
     w.cell_begin = starts[b];
     w.n_cells = starts[b + 1] - starts[b];
-    w.tile_begin = (int)P.tiles.size();
-    w.n_tiles = (int)L.tiles.size();
-    w.slot_begin = slot_base;
-    w.n_slots = L.n_slots;
-    const int chunk0 = (int)P.chunks.size(), edge0 = (int)P.edges.size();
-    for (TileDesc td : L.tiles) {
-      td.chunk_begin += chunk0;
-      td.chunk_end += chunk0;
-      P.tiles.push_back(td);
-    }
-    for (ChunkDesc cd : L.chunks) {
-      cd.edge_begin += edge0;
-      P.chunks.push_back(cd);
-    }
-    P.edges.insert(P.edges.end(), L.edges.begin(), L.edges.end());
-    if (in.g) P.edge_g.insert(P.edge_g.end(), L.edge_g.begin(), L.edge_g.end());
-    slot_base += L.n_slots;
     P.cta.push_back(w);
-    std::vector<TileDesc>().swap(L.tiles);
-    std::vector<ChunkDesc>().swap(L.chunks);
-    std::vector<uint16_t>().swap(L.edges);
-    std::vector<float>().swap(L.edge_g);
   }
 
-  // ---- shared-memory shape; keep the static work resident when it fits
+  // ---- shared-memory shape
   SmemShape sh{};
   sh.tile_cap = tile_cap;
   sh.nbuf = nbuf;
@@ -1286,21 +1310,6 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
   sh.max_slots = max_slots;
   sh.kahan = in.kahan;
   sh.edge_g = in.g ? 1 : 0;
-  int mt = 0, mc = 0, me = 0;
-  for (const CtaWork& w : P.cta) {
-    if (w.n_tiles == 0) continue;
-    const int c0 = P.tiles[w.tile_begin].chunk_begin, c1 = P.tiles[w.tile_begin + w.n_tiles - 1].chunk_end;
-    const int e0 = c1 > c0 ? P.chunks[c0].edge_begin : 0;
-    const int e1 = c1 > c0 ? P.chunks[c1 - 1].edge_begin + P.chunks[c1 - 1].count : 0;
-    mt = std::max(mt, w.n_tiles);
-    mc = std::max(mc, c1 - c0);
-    me = std::max(me, e1 - e0);
-  }
-  SmemShape res = sh;
-  res.res_tiles = std::max(mt, 1);
-  res.res_chunks = std::max(mc, 1);
-  res.res_edges = std::max(me, 1);
-  if (!in.no_resident && smem_layout(res).total <= in.smem_budget) sh = res;
 
   // ---- stamped exchange when every CTA's window (its unique senders, one
   // word each) fits in shared memory at once
@@ -1345,9 +1354,6 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
       P.max_slots = packed.max_slots;
       // the windows replace the tiles: CTA b's window is gcol[tile_begin ..
       // tile_begin + n_tiles), its unique senders in ascending order
-      P.tiles.clear();
-      P.chunks.clear();
-      P.gcol.clear();
       for (int b = 0; b < ctas; ++b) {
         CtaWork& w = P.cta[b];
         w.tile_begin = (int)P.gcol.size();
@@ -1375,24 +1381,40 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
       return false;
     }
   }
+  if (!sh.stamped) {
+    // windows larger than shared memory: sender shares and entries streamed;
+    // dense rows with one conductance walk adjacency bits; short rows gather
+    // through staged tiles (each would be cut into a few edges per tile)
+    if (stream_plan_wanted(in)) {
+      Plan st;
+      if (make_stream_plan(in, &st, err)) {
+        *out = std::move(st);
+        return true;
+      }
+    }
+    if (in.sync_mode == kSyncAuto && !in.g && E * kBitsMinDensityInv >= (int64_t)n * (int64_t)n)
+      return make_bits_plan(in, out, err);
+    if (in.sync_mode == kSyncAuto && E <= (int64_t)kGatherMaxMeanDegree * n) return make_tgather_plan(in, out, err);
+    tile_tables(in, starts, tiles, chunk, out);
+    // the static work stays resident when it fits
+    int mt = 0, mc = 0, me = 0;
+    for (const CtaWork& w : P.cta) {
+      if (w.n_tiles == 0) continue;
+      const int c0 = P.tiles[w.tile_begin].chunk_begin, c1 = P.tiles[w.tile_begin + w.n_tiles - 1].chunk_end;
+      const int e0 = c1 > c0 ? P.chunks[c0].edge_begin : 0;
+      const int e1 = c1 > c0 ? P.chunks[c1 - 1].edge_begin + P.chunks[c1 - 1].count : 0;
+      mt = std::max(mt, w.n_tiles);
+      mc = std::max(mc, c1 - c0);
+      me = std::max(me, e1 - e0);
+    }
+    SmemShape res = sh;
+    res.res_tiles = std::max(mt, 1);
+    res.res_chunks = std::max(mc, 1);
+    res.res_edges = std::max(me, 1);
+    if (!in.no_resident && smem_layout(res).total <= in.smem_budget) sh = res;
+  }
   P.shape = sh;
   P.smem_bytes = smem_layout(sh).total;
-  // windows larger than shared memory and short rows: gather through L2
-  // instead of staging tiles (each row would be cut into a few edges per tile)
-  // windows larger than shared memory: dense rows with one conductance walk
-  // adjacency bits; short rows gather through staged tiles
-  if (!sh.stamped && stream_plan_wanted(in)) {
-    Plan st;
-    if (make_stream_plan(in, &st, err)) {
-      *out = std::move(st);
-      return true;
-    }
-  }
-  if (!sh.stamped && in.sync_mode == kSyncAuto && !in.g &&
-      E * kBitsMinDensityInv >= (int64_t)n * (int64_t)n)
-    return make_bits_plan(in, out, err);
-  if (!sh.stamped && in.sync_mode == kSyncAuto && E <= (int64_t)kGatherMaxMeanDegree * n)
-    return make_tgather_plan(in, out, err);
   return true;
 }
 
