@@ -96,7 +96,6 @@ __device__ __forceinline__ unsigned long long pack_stamp(float v, unsigned stamp
 // without; the issue of the loads, not their round trip, was the larger part
 // of the poll.
 constexpr int kPollBatch = 8;
-constexpr int kPollBatchSmall = 3;
 
 struct PollWindow {
   const int* cells;  // the window's sender ids (shared memory)
@@ -300,12 +299,12 @@ __device__ __forceinline__ bool poll_finish(const StepArgs& a, const unsigned lo
 
 // Phase A of stamped plans (packed lane-chunk layout, all in shared memory):
 // warp w takes groups w, w + nwarps, ... < ngroups; lane l of the warp owns
-// lane-chunk l of the group (up to kLaneEdges edges of one receiver) and
+// lane-chunk l of the group (up to 4 * QUADS edges of one receiver) and
 // reduces it alone -- no cross-lane reduction.  Each 8-byte load brings the
 // lane's next four byte offsets; padding entries address the receiver's own
 // V_dend and add exactly 0.  Two accumulators (even / odd entries) shorten
 // the dependent add chain; they are combined in a fixed order.
-template <bool KAHAN, bool EDGE_G>
+template <bool KAHAN, bool EDGE_G, int QUADS>
 __device__ __forceinline__ void couple_packed(const unsigned char* sm, const SmemLayout& L, int ngroups,
                                               const float* sVd, float* part, float* partc, int warp, int nwarps,
                                               int lane) {
@@ -326,8 +325,8 @@ __device__ __forceinline__ void couple_packed(const unsigned char* sm, const Sme
       const float2 nvc2 = make_float2(nvc, nvc);
       float2 nacc = make_float2(-0.0f, -0.0f);
 #pragma unroll
-      for (int kq = 0; kq < kQuads; ++kq) {
-        const int qi = (gi * kQuads + kq) * 32 + lane;
+      for (int kq = 0; kq < QUADS; ++kq) {
+        const int qi = (gi * QUADS + kq) * 32 + lane;
         const uint2 o = ent[qi];
         float4 g4 = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         if (EDGE_G) g4 = gv[qi];
@@ -372,8 +371,8 @@ __device__ __forceinline__ void couple_packed(const unsigned char* sm, const Sme
       float2 nacc = make_float2(-0.0f, -0.0f);
       float2 cmp = make_float2(0.0f, 0.0f);
 #pragma unroll
-      for (int kq = 0; kq < kQuads; ++kq) {
-        const int qi = (gi * kQuads + kq) * 32 + lane;
+      for (int kq = 0; kq < QUADS; ++kq) {
+        const int qi = (gi * QUADS + kq) * 32 + lane;
         const uint2 o = ent[qi];
         float4 g4 = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         if (EDGE_G) g4 = gv[qi];
@@ -488,7 +487,7 @@ __device__ __forceinline__ void couple_tile(const ChunkDesc* chunks, const uint1
 
 // BLOCK threads per CTA, one CTA per SM: 1024 threads get 64 registers each,
 // 512 threads 128 (fewer warps, no spills).
-template <int BLOCK, bool KAHAN, bool EDGE_G, bool LL, int NB>
+template <int BLOCK, bool KAHAN, bool EDGE_G, bool LL, int NB, int QUADS = kMaxLaneEdges / 4>
 __global__ void __launch_bounds__(BLOCK, 1) step_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_abort;
@@ -565,11 +564,12 @@ __global__ void __launch_bounds__(BLOCK, 1) step_kernel(const __grid_constant__ 
     for (int i = tid; i < w.n_tiles; i += blockDim.x) s_w[i] = a.gcol[w.tile_begin + i];
     const int nd = w.n_groups * 32;
     for (int i = tid; i < nd; i += blockDim.x) s_d[i] = a.gdesc[(size_t)w.group_begin * 32 + i];
-    const int nq = w.n_groups * (kGroupEntries / 4);  // 8-byte quads
-    const uint2* ge = reinterpret_cast<const uint2*>(a.edges) + (size_t)w.group_begin * (kGroupEntries / 4);
+    constexpr int gq = QUADS * 32;  // 8-byte quads of a group
+    const int nq = w.n_groups * gq;
+    const uint2* ge = reinterpret_cast<const uint2*>(a.edges) + (size_t)w.group_begin * gq;
     for (int i = tid; i < nq; i += blockDim.x) s_e[i] = ge[i];
     if (EDGE_G) {
-      const float4* gg = reinterpret_cast<const float4*>(a.edge_g) + (size_t)w.group_begin * (kGroupEntries / 4);
+      const float4* gg = reinterpret_cast<const float4*>(a.edge_g) + (size_t)w.group_begin * gq;
       for (int i = tid; i < nq; i += blockDim.x) s_g[i] = gg[i];
     }
     pw.cells = s_w;
@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(BLOCK, 1) step_kernel(const __grid_constant__ 
       __syncthreads();
       if (s_abort) break;
       if (prof) t_ready = clock64();
-      couple_packed<KAHAN, EDGE_G>(smem_raw, L, w.n_groups, sVq, part, partc, warp, nwarps, lane);
+      couple_packed<KAHAN, EDGE_G, QUADS>(smem_raw, L, w.n_groups, sVq, part, partc, warp, nwarps, lane);
       __syncthreads();
     } else if (w.n_tiles > 0) {
       for (int j = 0; j < w.n_tiles; ++j) {
@@ -1549,13 +1549,23 @@ cudaError_t launch_gather_block(const StepArgs& a, int grid, cudaStream_t stream
   return g ? launch_gather<BLOCK, false, true>(a, grid, stream) : launch_gather<BLOCK, false, false>(a, grid, stream);
 }
 
-template <int BLOCK, bool K, bool G, bool LL, int NB = kPollBatch>
+template <int BLOCK, bool K, bool G, bool LL, int NB = kPollBatch, int QUADS = kMaxLaneEdges / 4>
 cudaError_t launch_variant(const StepArgs& a, int grid, size_t smem, cudaStream_t stream) {
-  auto fn = step_kernel<BLOCK, K, G, LL, NB>;
+  auto fn = step_kernel<BLOCK, K, G, LL, NB, QUADS>;
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<StepArgs*>(&a)};
   return cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(BLOCK), args, smem, stream);
+}
+
+template <int BLOCK, int QUADS>
+cudaError_t launch_small(const StepArgs& a, int grid, size_t smem, cudaStream_t stream) {
+  constexpr int S = kPollBatchSmall;
+  if (a.shape.kahan)
+    return a.edge_g ? launch_variant<BLOCK, true, true, true, S, QUADS>(a, grid, smem, stream)
+                    : launch_variant<BLOCK, true, false, true, S, QUADS>(a, grid, smem, stream);
+  return a.edge_g ? launch_variant<BLOCK, false, true, true, S, QUADS>(a, grid, smem, stream)
+                  : launch_variant<BLOCK, false, false, true, S, QUADS>(a, grid, smem, stream);
 }
 
 template <int BLOCK>
@@ -1564,13 +1574,13 @@ cudaError_t launch_block(const StepArgs& a, int grid, size_t smem, cudaStream_t 
   if (a.shape.stamped) {
     // the small poll batch when every thread's share of the largest window
     // fits in it (one round of loads)
-    if (a.shape.poll_words <= kPollBatchSmall * BLOCK) {
-      constexpr int S = kPollBatchSmall;
-      if (a.shape.kahan) return g ? launch_variant<BLOCK, true, true, true, S>(a, grid, smem, stream)
-                                  : launch_variant<BLOCK, true, false, true, S>(a, grid, smem, stream);
-      return g ? launch_variant<BLOCK, false, true, true, S>(a, grid, smem, stream)
-               : launch_variant<BLOCK, false, false, true, S>(a, grid, smem, stream);
+    const bool small = a.shape.poll_words <= kPollBatchSmall * BLOCK;
+    if (a.shape.lane_edges != kMaxLaneEdges) {  // kernels of their own: the three loops in one cost 0.1 us per step
+      if (BLOCK != 512 || !small) return cudaErrorInvalidValue;
+      return a.shape.lane_edges == 8 ? launch_small<512, 2>(a, grid, smem, stream)
+                                     : launch_small<512, 4>(a, grid, smem, stream);
     }
+    if (small) return launch_small<BLOCK, kMaxLaneEdges / 4>(a, grid, smem, stream);
     if (a.shape.kahan) return g ? launch_variant<BLOCK, true, true, true>(a, grid, smem, stream)
                                 : launch_variant<BLOCK, true, false, true>(a, grid, smem, stream);
     return g ? launch_variant<BLOCK, false, true, true>(a, grid, smem, stream)

@@ -39,14 +39,17 @@ namespace infoli {
 
 enum { kChunkEdges = 128, kMaxChunkEdges = 8192 };
 
-// Packed layout of stamped plans.  A lane-chunk is up to kLaneEdges edges of
-// one receiver reduced by ONE lane; 32 lane-chunks form a group handled by
-// one warp.  Entries are stored transposed in 4-entry quads so lane l reads
-// its next four entries with one 8-byte load:
-//   entry k of lane l in group g at ((g * kQuads + k / 4) * 32 + l) * 4 + k % 4
+// Packed layout of stamped plans.  A lane-chunk is up to `lane_edges` (8, 16
+// or 32, one number per plan) edges of one receiver reduced by ONE lane; 32
+// lane-chunks form a group handled by one warp.  Entries are stored transposed
+// in 4-entry quads so lane l reads its next four entries with one 8-byte load:
+//   entry k of lane l in group g at ((g * lane_edges / 4 + k / 4) * 32 + l) * 4 + k % 4
 // Each entry is the byte offset, from the start of dynamic shared memory, of
 // the sender's V_dend; padding entries address the receiver's own V_dend.
-enum { kLaneEdges = 32, kQuads = kLaneEdges / 4, kGroupEntries = 32 * kLaneEdges };
+enum { kMaxLaneEdges = 32 };
+// Stamped plans: words that a thread polls in one round of loads where the
+// largest window allows it (StepArgs, SmemShape::poll_words).
+enum { kPollBatchSmall = 3 };
 
 typedef struct {
   int cell_begin;   // first owned cell (index into the V_dend / state arrays)
@@ -123,6 +126,7 @@ typedef struct {
                    // each staging its share of V_dend whole (tile_cap floats) and
                    // streaming its lane-chunks' entries from global memory
   int slices;      // bitmask plan: threads per receiver (column slices)
+  int lane_edges;  // stamped: entries per lane-chunk (8, 16 or 32)
   int poll_words;  // stamped: the most words one CTA polls per step (window
                    // senders + progress probes); picks the poll batch size
   int cluster;     // stream plan: CTAs per cluster (sender shares)

@@ -119,10 +119,61 @@ std::vector<int> unique_senders(const PlanInput& in, int c0, int c1) {
   return u;
 }
 
+// First partial slot of a CTA's receiver r, from the end of the slots before
+// it.  Each receiver's partial slots start on a 4-slot (16-byte) boundary; the
+// gaps are zeroed once per launch, so the update can read them 4 at a time.
+// Consecutive receivers start an odd number of 16-byte units apart (an unread
+// unit is added after an even-sized block), so the 8 lanes of each phase of a
+// 16-byte shared-memory load (one receiver per lane) fall in 8 different bank
+// groups instead of 2.
+int next_receiver_slot(int slot, int prev_begin, int r) {
+  slot = (slot + 3) & ~3;
+  return r > 0 && (((slot - prev_begin) >> 2) & 1) == 0 ? slot + 4 : slot;
+}
+
+// What the CTA with the most of them needs for lane-chunks of `lane_edges`.
+struct PackedSize {
+  int slots = 1, groups = 1;
+};
+PackedSize packed_size(const PlanInput& in, const std::vector<int>& starts, int lane_edges) {
+  PackedSize m;
+  for (size_t b = 0; b + 1 < starts.size(); ++b) {
+    int slot = 0, begin = 0, chunks = 0;
+    for (int c = starts[b]; c < starts[b + 1]; ++c) {
+      begin = next_receiver_slot(slot, begin, c - starts[b]);
+      const int count = (int)((in.row_ptr[c + 1] - in.row_ptr[c] + lane_edges - 1) / lane_edges);
+      slot = begin + count;
+      chunks += count;
+    }
+    m.slots = std::max(m.slots, ((slot + 3) & ~3) + 1);  // and the dummies' slot
+    m.groups = std::max(m.groups, (chunks + 31) / 32);
+  }
+  return m;
+}
+
+// Entries per lane-chunk.  A lane takes its entries one after another, and in
+// a small network most warps have no group, so shorter chunks over more warps
+// are faster where rows are short: us per step, 32 -> 8: 44 cells x 6 senders
+// 1.52 -> 1.24, 271 x 7 1.47 -> 1.38, 4,379 x 15 1.94 -> 1.85, 10,684 x 9
+// 2.16 -> 2.09; 32 -> 16: 201 x 53 1.51 -> 1.41, 92x21 grid (reach 5.7) 1.51
+// -> 1.41.  The receiver's owner adds a partial sum per chunk, four to a load,
+// which costs more than it saves with longer rows (17x46 grid of reach 16,
+// chunks of 16: 1.71 -> 1.92; 1,000 x 100, chunks of 8: 1.59 -> 1.74) or with
+// more groups (72x74 grid of reach 6: 1.93 -> 1.97 with 8 of them).
+int lane_edges_for(const PlanInput& in, const std::vector<int>& starts, int window) {
+  const int warps = in.threads / 32;
+  // (kernels of one round of polls; a CTA has at most one probe per other CTA)
+  if (in.threads != 512 || window + (int)starts.size() > kPollBatchSmall * in.threads) return kMaxLaneEdges;
+  int64_t longest = 0;
+  for (int c = 0; c < in.n; ++c) longest = std::max(longest, in.row_ptr[c + 1] - in.row_ptr[c]);
+  if (longest <= 32 && packed_size(in, starts, 8).groups <= warps / 2) return 8;
+  return longest <= 96 && packed_size(in, starts, 16).groups <= warps * 3 / 8 ? 16 : kMaxLaneEdges;
+}
+
 // Build the packed lane-chunk tables of a stamped, resident plan (see
 // infoli_plan.h): per receiver, its senders (ascending) become byte offsets
 // into the CTA's window (its sorted unique senders, win[b], one float each),
-// cut into lane-chunks of kLaneEdges;
+// cut into lane-chunks of lane_edges;
 // the chunks of a CTA, receiver-major, are dealt 32 per group.  Inside a
 // group, entries are permuted per chunk so that the 32 lanes reading
 // position k hit distinct shared-memory banks where possible.  Receiver slots
@@ -135,7 +186,7 @@ std::vector<int> unique_senders(const PlanInput& in, int c0, int c1) {
 // open bank taken before a longer path is tried, and the tile tables built
 // only for the plans that keep them.
 void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::vector<std::vector<int>>& win,
-                 int dup_words, int cells_cap) {
+                 int dup_words, int cells_cap, int lane_edges) {
   const bool edge_g = in.g != nullptr;
   // CTAs are packed in parallel into local tables, then concatenated
   struct Local {
@@ -174,18 +225,10 @@ void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::v
         off.push_back(place[(size_t)s]);
         if (edge_g) val.push_back(gv);
       });
-      // each receiver's partial slots start on a 4-slot (16-byte) boundary; the
-      // gaps are zeroed once per launch, so the update can read them 4 at a time.
-      // Consecutive receivers start an odd number of 16-byte units apart (an
-      // unread unit is added after an even-sized block), so the 8 lanes of each
-      // phase of a 16-byte shared-memory load (one receiver per lane) fall in
-      // 8 different bank groups instead of 2
-      slot = (slot + 3) & ~3;
-      if (r > 0 && (((slot - prev_begin) >> 2) & 1) == 0) slot += 4;
-      prev_begin = slot;
+      slot = prev_begin = next_receiver_slot(slot, prev_begin, r);
       P.cell_slots[c].begin = slot;
-      for (size_t k = row; k < off.size(); k += kLaneEdges)
-        lc.push_back({r, slot++, k, (int)std::min<size_t>(kLaneEdges, off.size() - k)});
+      for (size_t k = row; k < off.size(); k += lane_edges)
+        lc.push_back({r, slot++, k, (int)std::min<size_t>(lane_edges, off.size() - k)});
       P.cell_slots[c].count = slot - P.cell_slots[c].begin;
     }
     const int dummy_slot = (slot + 3) & ~3;  // past the last receiver's 4-slot block
@@ -220,15 +263,15 @@ void pack_groups(Plan& P, const SmemLayout& L, const PlanInput& in, const std::v
         pad[l] = (uint16_t)(L.vown + sizeof(float) * ((size_t)kScaledVArray * cells_cap + d.y));
         gdesc.push_back(d);
       }
-      const size_t base = pe.size();  // transposed quads: ((g * kQuads + k / 4) * 32 + l) * 4 + k % 4
-      pe.resize(base + kGroupEntries);
-      if (edge_g) pg.resize(base + kGroupEntries);
+      const size_t base = pe.size();
+      pe.resize(base + 32 * lane_edges);
+      if (edge_g) pg.resize(base + 32 * lane_edges);
       // bank-distinct dealing, position by position: lanes whose chunk is
       // exhausted read their padding word (lanes of one receiver share it);
       // the others are matched to free banks by augmenting paths (Kuhn), so
       // each position has as many conflict-free lanes as the remaining
       // entries allow; unmatched lanes take any entry
-      for (int k = 0; k < kLaneEdges; ++k) {
+      for (int k = 0; k < lane_edges; ++k) {
         const size_t at = base + (size_t)(k / 4) * 128 + k % 4;
         unsigned taken = 0;  // banks already claimed by padding words
         for (int l = 0; l < 32; ++l)
@@ -1322,36 +1365,29 @@ bool make_plan_base(const PlanInput& in, Plan* out, std::string* err) {
     // Preferred: two copies of the window, the second 16 banks away, so every
     // gather can pick the copy whose bank is free; else a single copy.
     SmemShape st = sh;
-    Plan packed;
     bool fits = false;
-    for (int dup = 1; dup >= 0 && !fits; --dup) {
-      st = sh;
-      st.nbuf = 1;
-      st.stamped = 1;
-      const int w4 = (sum_max + 3) & ~3;
-      st.dup_words = dup ? ((w4 + 31) & ~31) + 16 : 0;
-      st.tile_cap = dup ? st.dup_words + w4 : w4;
-      const SmemLayout SL0 = smem_layout(st);  // tile and cell-array offsets do not depend on the rest
-      const bool offsets_fit = SL0.vown + sizeof(float) * (size_t)(kScaledVArray + 1) * cells_cap <= 65536;
-      if (in.no_resident || !offsets_fit) continue;
-      packed = P;
-      pack_groups(packed, SL0, in, uniq, st.dup_words, cells_cap);
-      int mg = 1;
-      for (const CtaWork& w : packed.cta) mg = std::max(mg, w.n_groups);
-      st.max_slots = packed.max_slots;
-      st.res_tiles = (sum_max + 3) / 4;  // the window's cell ids, four per 16-byte descriptor slot
-      st.res_chunks = mg * 32;
-      st.res_edges = mg * kGroupEntries;
-      fits = smem_layout(st).total <= in.smem_budget;
-    }
+    const int lane_edges = lane_edges_for(in, starts, sum_max);
+    for (int dup = 1; dup >= 0 && !fits; --dup)
+      for (int le = lane_edges; le <= kMaxLaneEdges && !fits; le *= 2) {
+        st = sh;
+        st.nbuf = 1;
+        st.stamped = 1;
+        st.lane_edges = le;
+        const int w4 = (sum_max + 3) & ~3;
+        st.dup_words = dup ? ((w4 + 31) & ~31) + 16 : 0;
+        st.tile_cap = dup ? st.dup_words + w4 : w4;
+        const PackedSize most = packed_size(in, starts, le);
+        st.max_slots = most.slots;
+        st.res_tiles = (sum_max + 3) / 4;  // the window's cell ids, four per 16-byte descriptor slot
+        st.res_chunks = most.groups * 32;
+        st.res_edges = most.groups * 32 * le;
+        const SmemLayout SL = smem_layout(st);
+        const bool offsets_fit = SL.vown + sizeof(float) * (size_t)(kScaledVArray + 1) * cells_cap <= 65536;
+        fits = !in.no_resident && offsets_fit && SL.total <= in.smem_budget;
+      }
     if (fits) {
       sh = st;
-      P.cta.swap(packed.cta);
-      P.cell_slots.swap(packed.cell_slots);
-      P.gdesc.swap(packed.gdesc);
-      P.edges.swap(packed.edges);
-      P.edge_g.swap(packed.edge_g);
-      P.max_slots = packed.max_slots;
+      pack_groups(P, smem_layout(st), in, uniq, st.dup_words, cells_cap, st.lane_edges);
       // the windows replace the tiles: CTA b's window is gcol[tile_begin ..
       // tile_begin + n_tiles), its unique senders in ascending order
       for (int b = 0; b < ctas; ++b) {
@@ -1884,15 +1920,16 @@ extern "C" int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t*
         if (P.probes[w.probe_begin + q] < 0 || P.probes[w.probe_begin + q] >= n) return -5;
       probes += w.n_probes;
       groups += w.n_groups;
+      const int le = P.shape.lane_edges;
       // shared-memory wavefronts of the V_dend gathers: per (group, entry
       // position) the largest number of distinct words any bank serves
       for (int gi = 0; gi < w.n_groups; ++gi)
-        for (int k = 0; k < kLaneEdges; ++k) {
+        for (int k = 0; k < le; ++k) {
           unsigned words[32][32];
           int cnt[32] = {0};
           int worst = 1;
           for (int l = 0; l < 32; ++l) {
-            const size_t at = (((size_t)w.group_begin + gi) * kQuads + k / 4) * 32 * 4 + (size_t)l * 4 + k % 4;
+            const size_t at = (((size_t)w.group_begin + gi) * (le / 4) + k / 4) * 128 + (size_t)l * 4 + k % 4;
             const unsigned word = P.edges[at] >> 2, bank = word & 31;
             bool seen = false;
             for (int q = 0; q < cnt[bank]; ++q) seen |= words[bank][q] == word;
@@ -1908,8 +1945,8 @@ extern "C" int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t*
           if (d.x < 0 || d.x >= P.shape.max_slots || d.y < 0 || d.y >= std::max(w.n_cells, 1)) return -6;
           const float vc = sVd[d.y];
           float acc0 = 0.0f, acc1 = 0.0f;
-          for (int k = 0; k < kLaneEdges; ++k) {
-            const size_t at = (((size_t)w.group_begin + gi) * kQuads + k / 4) * 32 * 4 + (size_t)l * 4 + k % 4;
+          for (int k = 0; k < le; ++k) {
+            const size_t at = (((size_t)w.group_begin + gi) * (le / 4) + k / 4) * 128 + (size_t)l * 4 + k % 4;
             const unsigned off = P.edges[at];
             if (off % 4 || off + 4 > L.vown + sizeof(float) * (size_t)(kScaledVArray + 1) * P.shape.cells_cap) return -7;
             const float V = vc - *reinterpret_cast<const float*>(sm.data() + off);
