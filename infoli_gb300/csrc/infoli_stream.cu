@@ -155,7 +155,8 @@ __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& 
 // an error-free sum per addition whose errors are applied once.  Valid in the
 // lanes with sub == 0.
 template <bool KAHAN>
-__device__ __forceinline__ float sum_slots(int2 sl, const float* part, int sub, int width) {
+__device__ __forceinline__ float sum_slots(uint32_t slots, const float* part, int sub, int width) {
+  const int first = slots & 0xffffu, count = slots >> 16;
   float s = 0.0f, e = 0.0f;
   auto add = [&](float x) {
     const float t = s + x;
@@ -166,7 +167,7 @@ __device__ __forceinline__ float sum_slots(int2 sl, const float* part, int sub, 
     s = t;
   };
 #pragma unroll 4
-  for (int q = sub; q < sl.y; q += width) add(part[sl.x + q]);
+  for (int q = sub; q < count; q += width) add(part[first + q]);
   for (int o = 1; o < width; o <<= 1) {
     const float s2 = __shfl_down_sync(0xffffffffu, s, o);
     const float e2 = KAHAN ? __shfl_down_sync(0xffffffffu, e, o) : 0.0f;
@@ -200,6 +201,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   float* part = reinterpret_cast<float*>(smem_raw + L.part);
   uint64_t* mbar = reinterpret_cast<uint64_t*>(smem_raw + L.mbar);
   float* sums = reinterpret_cast<float*>(smem_raw + L.sums);
+  uint32_t* s_slots = reinterpret_cast<uint32_t*>(smem_raw + L.slots);
+  float* s_app = reinterpret_cast<float*>(smem_raw + L.app);
   const int cs = a.shape.cluster, share = a.shape.tile_cap, cap = a.shape.cells_cap;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   // A launch whose clusters are not the plan's (a tool that relaunches the
@@ -233,6 +236,11 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     fence_mbar_init();
     s_abort = 0;
     for (int k = 0; k < kStreamMaxCluster; ++k) s_peer[k] = 0.0f;
+  }
+  const int row0 = cs == 1 ? w.cell_begin : w.tile_begin, nrows = cs == 1 ? w.n_cells : w.n_tiles;
+  for (int q = tid; q < nrows; q += kStreamThreads) {
+    const int2 s = __ldg(a.cell_slots + (size_t)(row0 + q) * cs + w.pad1);
+    s_slots[q] = (uint32_t)s.x | (uint32_t)s.y << 16;
   }
   Volts v{};
   if (owner) {
@@ -293,6 +301,16 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
       g.xs = st[F_XS * np];
       g.ha = st[F_HA * np];
       g.xa = st[F_XA * np];
+      float iapp;
+      if (a.stim_kind == STIM_PULSE) {
+        iapp = (step >= a.stim_start && step < a.stim_end) ? a.stim_amp : 0.0f;
+      } else if (a.stim_kind == STIM_CELL) {
+        const int onset = __ldg(a.cell_onset + cell);
+        iapp = (step >= onset && step < onset + a.stim_dur) ? __ldg(a.cell_amp + cell) : 0.0f;
+      } else {
+        iapp = a.stim_table[(size_t)st_i * np + cell];
+      }
+      s_app[tid] = iapp;
       Currents cur;
       run_units(a.P, v, g, cur);
       st[F_Q * np] = g.q;
@@ -348,26 +366,15 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
       if (!stream_wait(a, mbar, (unsigned)st_i & 1u, &s_abort)) s_abort = 1;
       mark(1);
     });
-    // what the update reads from global memory, in flight while the other warps finish
-    const int2 none = make_int2(0, 0);
     const int per = cs > 1 ? (w.n_tiles + cs - 1) / cs : 0;  // rows of a CTA of the cluster
-    int2 slots = none;
     const int sr = tid >> wlog;  // the receiver that this thread adds slots of
-    if (sr < (cs == 1 ? w.n_cells : w.n_tiles))
-      slots = __ldg(a.cell_slots + (size_t)((cs == 1 ? w.cell_begin : w.tile_begin) + sr) * cs + w.pad1);
-    float my_amp = 0.0f;
-    int my_onset = 0;
-    if (owner && a.stim_kind == STIM_CELL) {
-      my_amp = __ldg(a.cell_amp + cell);
-      my_onset = __ldg(a.cell_onset + cell);
-    }
+    const uint32_t slots = sr < nrows ? s_slots[sr] : 0u;
     __syncthreads();
     if (cs > 1) {
       // every row's sum over this share goes to its owner's CTA (a store: a
       // remote load would stand in the update's way)
       for (int q = tid; q < w.n_tiles; q += kStreamThreads) {
-        if (q >= kStreamThreads) slots = __ldg(a.cell_slots + (size_t)(w.tile_begin + q) * cs + w.pad1);
-        const float s = sum_slots<KAHAN>(slots, part, 0, 1);
+        const float s = sum_slots<KAHAN>(s_slots[q], part, 0, 1);
         const int k = (q >= per) + (q >= 2 * per) + (q >= 3 * per);
         st_peer(peer_addr(smem_u32(sums + w.pad1 * cap + (q - k * per)), (unsigned)k), s);
       }
@@ -391,14 +398,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     if (owner) {
       ic *= kInvVScale;
       if (!EDGE_G) ic *= a.g_uniform;
-      float iapp;
-      if (a.stim_kind == STIM_PULSE)
-        iapp = (step >= a.stim_start && step < a.stim_end) ? a.stim_amp : 0.0f;
-      else if (a.stim_kind == STIM_CELL)
-        iapp = (step >= my_onset && step < my_onset + a.stim_dur) ? my_amp : 0.0f;
-      else
-        iapp = a.stim_table[(size_t)st_i * np + cell];
-      v.Vd = voltage_second(a.P, vk, v.Vd, vh, ic, iapp);
+      v.Vd = voltage_second(a.P, vk, v.Vd, vh, ic, s_app[tid]);
       v.Vs = vh.Vs;
       v.Va = vh.Va;
       a.vds[(step + 1) & 1][cell] = v.Vd * kVScale;
