@@ -1508,7 +1508,7 @@ template <int BLOCK, bool K>
 cudaError_t launch_bits(const StepArgs& a, int grid, cudaStream_t stream) {
   const size_t smem = tgather_smem_bytes(a.shape);
   auto fn = bits_kernel<BLOCK, K>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory((const void*)fn);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<StepArgs*>(&a)};
   return cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(BLOCK), args, smem, stream);
@@ -1518,7 +1518,7 @@ template <int BLOCK, bool K, bool G>
 cudaError_t launch_tgather(const StepArgs& a, int grid, cudaStream_t stream) {
   const size_t smem = tgather_smem_bytes(a.shape);
   auto fn = tgather_kernel<BLOCK, K, G>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory((const void*)fn);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<StepArgs*>(&a)};
   return cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(BLOCK), args, smem, stream);
@@ -1528,7 +1528,7 @@ template <int BLOCK, bool K, bool G>
 cudaError_t launch_gather(const StepArgs& a, int grid, cudaStream_t stream) {
   const size_t smem = gather_smem_bytes(BLOCK);
   auto fn = gather_kernel<BLOCK, K, G>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory((const void*)fn);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<StepArgs*>(&a)};
   return cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(BLOCK), args, smem, stream);
@@ -1552,7 +1552,7 @@ cudaError_t launch_gather_block(const StepArgs& a, int grid, cudaStream_t stream
 template <int BLOCK, bool K, bool G, bool LL, int NB = kPollBatch, int QUADS = kMaxLaneEdges / 4>
 cudaError_t launch_variant(const StepArgs& a, int grid, size_t smem, cudaStream_t stream) {
   auto fn = step_kernel<BLOCK, K, G, LL, NB, QUADS>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory((const void*)fn);
   if (e != cudaSuccess) return e;
   void* args[] = {const_cast<StepArgs*>(&a)};
   return cudaLaunchCooperativeKernel((const void*)fn, dim3(grid), dim3(BLOCK), args, smem, stream);
@@ -1617,11 +1617,11 @@ int max_coresident_ctas(int threads, size_t smem, cudaError_t* err) {
   if (e == cudaSuccess) {
     if (threads == 1024) {
       auto fn = step_kernel<1024, false, false, false, kPollBatch>;
-      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = allow_shared_memory((const void*)fn);
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     } else if (threads == 512) {
       auto fn = step_kernel<512, false, false, false, kPollBatch>;
-      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      e = allow_shared_memory((const void*)fn);
       if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem);
     } else {
       e = cudaErrorInvalidValue;

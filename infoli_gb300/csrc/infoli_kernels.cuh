@@ -97,6 +97,15 @@ __device__ __forceinline__ void device_error(const StepArgs& a, int code) {
   if (a.err_host) *reinterpret_cast<volatile int*>(a.err_host) = code;
 }
 
+// Lets launches of a step kernel ask for as much dynamic shared memory as any
+// plan may (227 KB less 1 KB for the kernels' static part, the planner's
+// budget).  One value for every call: the attribute belongs to the function, and
+// a smaller one set by another thread between this call and a launch or an
+// occupancy query would fail it.
+inline cudaError_t allow_shared_memory(const void* fn) {
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448 - 1024);
+}
+
 // Dynamic shared memory needed for a launch.
 size_t step_kernel_smem(const StepArgs& a);
 

@@ -471,7 +471,7 @@ void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, i
 cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t stream) {
   const size_t smem = stream_layout(a.shape).total;
   const void* fn = stream_fn(a.shape.kahan != 0, a.edge_g != nullptr, a.shape.byte_off != 0, a.shape.block);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory((const void*)fn);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
@@ -482,7 +482,7 @@ cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t strea
 
 int max_stream_ctas(int cluster, size_t smem) {
   const void* fn = stream_fn(true, true, false, 8);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (allow_shared_memory((const void*)fn) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
   stream_config(cfg, at, cluster, cluster, smem, nullptr);

@@ -1,5 +1,7 @@
 """What one launch leaves for the next (the exchange words of V_dend, the trace slots in host memory): runs split into
 launches anywhere, states set between launches, errors between launches, traces longer than a slot."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -59,3 +61,25 @@ def test_traces_longer_than_a_slot(ig, what):
         assert sim.run(0, 1, what)["soma"].shape == (0, n)
     for name, rows in whole.items():
         assert rows.flags.c_contiguous and np.array_equal(rows, np.concatenate([p[name] for p in parts]))
+
+
+def test_threads_create_and_run_simulations_of_different_sizes(ig):
+    """A kernel's limit of shared memory is one for all threads: plans of very different sizes, side by side."""
+    conf, failed = O.read_parameters(CONF), []
+    nets = [(n, *ig.gen_uniform(n, p, 2)) for n, p in ((60, 0.2), (300, 0.1), (1500, 0.3), (2500, 0.25))]
+
+    def work(k):
+        try:
+            for i in range(40):
+                n, rp, col = nets[(k + i) % len(nets)]
+                with ig.Simulation(n, conf, rp, col, init_state=hetero_state(conf, n, 3)) as sim:
+                    sim.run(2)
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed[0]
