@@ -58,7 +58,7 @@ STEPS_PER_ITER = 1000
 TRACE_EVERY = 100
 CPU_SAMPLE_STEPS = 2000  # timesteps of the oracle port, reported beside the reference build
 N_SM_FALLBACK = 152
-SFU_EX2_PER_CLK_SM = 16  # MUFU.EX2 results per clock per SM
+SFU_EX2_PER_CLK_SM = 32  # exp2 results per clock per SM (measured: 62 per ns and SM)
 
 CONF_PATH = os.path.join(ROOT, "infoli_gb300", "host", "default.conf")
 REF_DIR = os.path.join(ROOT, "oracle", "_ref")
@@ -925,7 +925,8 @@ def run_gpu_batched(args, world, rank, local, warmup=None):
             "speedup_batched_vs_plain": value / plain_rate},
         "e2e": {"value": e2e_value, "unit": "sims/s", "h2d_bytes_per_step": int(st.nbytes),
                 "d2h_bytes_per_step": int(st.nbytes)},
-        # per bench step: one launch per cluster-size group + the step-index advance
+        # per bench step, at least: one launch per cluster-size group (entry lists also
+        # split a size by length) + the step-index advance
         "gpu_launches": steps * (len({(int(n) + info["block"] - 1) // info["block"]
                                       for n in meta["sizes"]}) + 1),
         "wall_s": wall,

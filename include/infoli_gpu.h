@@ -324,6 +324,9 @@ typedef struct {
    *                   shape allows stay resident (two 512-thread CTAs per
    *                   SM; the same as INFOLI_RES_FIT for 1,024 threads);
    *   INFOLI_RES_NONE none.
+   * Batches run on entry lists made from the bitmasks unless those would take
+   * over half of the free device memory; lists are always streamed, and
+   * residency then changes nothing.
    * infoli_batch_autotune picks it together with block. */
   int residency;
 } infoli_batch_desc;
@@ -521,13 +524,14 @@ int infoli_run_noalloc(const float* params, int n_cells, const int64_t* d_row_pt
 /* Host-side check of the work planner (no GPU needed; no counterpart in the
  * reference): plans an n-cell network for a device with grid_max co-resident
  * CTAs of `threads` threads and smem_budget bytes of shared memory per CTA
- * (sync_mode 0 auto, 1 grid barrier, 2 stamped words; grid 0 = automatic),
+ * (sync_mode 0 auto, 1 grid barrier, 2 stamped words, 3 gather, 4 tiled
+ * gather, 5 bitmask, 6 stream; grid 0 = automatic),
  * then computes the gap-junction currents of the voltages vdend[n] by walking
  * the plan's tables with the step kernel's addressing, every shared-memory
  * offset bounds-checked.  info[10] = {CTAs, stamped, tiles (stamped plans: 1
  * when the planner relabelled the cells), chunks or groups, partial slots,
  * shared bytes, progress probes, resident, shared-memory wavefronts of the
- * stamped V_dend gathers, gather instructions}.  vdend and ic_out are in the
+ * stamped (or stream) plan's V_dend gathers, gather instructions}.  vdend and ic_out are in the
  * caller's cell order either way.  Returns 0 or a negative code naming the
  * violated invariant. */
 int infoli_plan_emulate(int n, const int64_t* row_ptr, const int32_t* col, const float* g, float g_uniform,
