@@ -727,7 +727,8 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
   CK(cudaEventElapsedTime(&ms, s->ev_t0, s->ev_t1));
   s->last_ms = ms;
   s->last_launches = launches;
-  int rc = s->h_err ? report_device_error(s, *s->h_err) : check_device_error(s);
+  // (after an unchecked asynchronous launch the device's word may be older than this run)
+  int rc = s->h_err && !s->async_pending ? report_device_error(s, *s->h_err) : check_device_error(s);
   if (rc) return rc;
   s->step += n_steps;
   return INFOLI_OK;

@@ -48,6 +48,23 @@ def test_a_new_state_between_launches_starts_afresh(ig, n, mode, monkeypatch):
             assert np.array_equal(sim.get_state(), state)
 
 
+@pytest.mark.parametrize("mode", ["stamped", "barrier", "stream"])
+def test_a_run_after_an_unchecked_launch_that_failed_reports_it(ig, mode, monkeypatch):
+    conf, n = O.read_parameters(CONF), 1300
+    monkeypatch.setenv("INFOLI_SYNC", mode)
+    monkeypatch.setenv("INFOLI_WAIT_TIMEOUT_MS", "300")
+    rp, col = ig.gen_uniform(n, 0.1, 2)
+    st0 = hetero_state(conf, n, 1)
+    with ig.Simulation(n, conf, rp, col, init_state=st0) as sim, ig.Simulation(n, conf, rp, col, init_state=st0) as ref:
+        monkeypatch.setenv("INFOLI_STALL_CTA", "1")
+        sim.launch(5)
+        monkeypatch.delenv("INFOLI_STALL_CTA")
+        with pytest.raises(ig.InfoliError):
+            sim.run(1)
+        sim.set_state(st0)
+        assert np.array_equal(sim.run(20, 1, ig.TRACE_DEND)["dend"], ref.run(20, 1, ig.TRACE_DEND)["dend"])
+
+
 @pytest.mark.parametrize("what", [2, 7])
 def test_traces_longer_than_a_slot(ig, what):
     conf, n, steps = O.read_parameters(CONF), 61001, 300
