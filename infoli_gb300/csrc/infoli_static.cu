@@ -115,7 +115,7 @@ __device__ __forceinline__ float noalloc_row(const NoAllocArgs& a, const float* 
 
 // What bounds a step: the grid barrier and the L2 round trips to the senders'
 // V_dend, so a CTA has few cells and every lane eight loads in flight.
-// 5,003 cells x 60 senders, per-edge g, 200 steps: 1,264 us per call
+// 5,003 cells x 60 senders, per-edge g, 200 steps: 1,030 us per call
 // against 5,180 with one thread per cell on 10 CTAs (the edges of a row one
 // after another, the gate units after them).
 __global__ void __launch_bounds__(kNoAllocBlock, 2) noalloc_step_kernel(const __grid_constant__ NoAllocArgs a,
