@@ -193,7 +193,12 @@ __device__ __forceinline__ bool stream_wait(const StepArgs& a, uint64_t* bar, un
 template <bool KAHAN, bool EDGE_G, bool BYTE, int N>
 __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int s_abort;
+  __shared__ int s_abort;  // a wait of this step gave up: set before the step's first CTA barrier
+  // The launch ends: set between that barrier and the step's last one, where
+  // every warp reads it.  (s_abort itself may be set again by the producer of
+  // the next step, and a slow warp that read it then would leave a step before
+  // the others, which wait for it without a limit.)
+  __shared__ int s_stop;
   __shared__ float s_peer[kStreamMaxCluster];  // set by a CTA of the cluster that gave up
   __shared__ unsigned long long s_prof[4];  // cycles: gate units, wait for the share, coupling, rest
   const StreamLayout L = stream_layout(a.shape);
@@ -234,7 +239,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   if (tid == 0) {
     mbar_init(mbar, 1);
     fence_mbar_init();
-    s_abort = 0;
+    s_abort = s_stop = 0;
     for (int k = 0; k < kStreamMaxCluster; ++k) s_peer[k] = 0.0f;
   }
   const int row0 = cs == 1 ? w.cell_begin : w.tile_begin, nrows = cs == 1 ? w.n_cells : w.n_tiles;
@@ -413,10 +418,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     if (trace_now) ++row;
     // a CTA that gave up takes its cluster with it (no CTA may leave while
     // another writes to its shared memory)
-    if (cs > 1 && tid < cs && s_peer[tid] != 0.0f) s_abort = 1;
+    if (tid < cs && (cs > 1 ? s_peer[tid] != 0.0f : s_abort != 0)) s_stop = 1;
     __syncthreads();
     mark(3);
-    if (s_abort) break;
+    if (s_stop) break;
   }
   if (prof) {
     unsigned long long* pr = a.prof + (size_t)blockIdx.x * kProfSlots;
