@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   // the next step, and a slow warp that read it then would leave a step before
   // the others, which wait for it without a limit.)
   __shared__ int s_stop;
+  __shared__ int s_copied;  // steps of the launch whose copies have been issued
   __shared__ float s_peer[kStreamMaxCluster];  // set by a CTA of the cluster that gave up
   __shared__ unsigned long long s_prof[4];  // cycles: gate units, wait for the share, coupling, rest
   const StreamLayout L = stream_layout(a.shape);
@@ -239,7 +240,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   if (tid == 0) {
     mbar_init(mbar, 1);
     fence_mbar_init();
-    s_abort = s_stop = 0;
+    s_abort = s_stop = s_copied = 0;
     for (int k = 0; k < kStreamMaxCluster; ++k) s_peer[k] = 0.0f;
   }
   const int row0 = cs == 1 ? w.cell_begin : w.tile_begin, nrows = cs == 1 ? w.n_cells : w.n_tiles;
@@ -362,6 +363,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
           bulk_g2s(smem_raw + o, reinterpret_cast<const unsigned char*>(src + lo) + o,
                    (unsigned)min(kCopyBytes, nshare * 4 - o), mbar);
         if (nrow) bulk_g2s(smem_raw + L.rows, src + row_lo, (unsigned)nrow * 4u, mbar);
+        s_copied = st_i + 1;
       }
     }
     __syncwarp();
@@ -433,6 +435,14 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     atomicAdd(pr + PROF_SPAN_NS, (unsigned long long)(globaltimer_ns() - ns_begin));
     atomicAdd(pr + PROF_SPAN_CYCLES, (unsigned long long)(clock64() - cy_begin));
   }
+  // The other warps' waits may run out just as the grid barrier completes: the
+  // copies issued then still land in this CTA's shared memory before it leaves.
+  if (producer && s_copied > 0) {
+    const uint64_t t0 = globaltimer_ns();
+    while (!mbar_try_wait(mbar, (unsigned)(s_copied - 1) & 1u) && globaltimer_ns() - t0 <= a.timeout_ns) {
+    }
+  }
+  __syncwarp();
   if (cs > 1) cluster_sync_all();
 
   if (owner) {
