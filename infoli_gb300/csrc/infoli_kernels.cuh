@@ -91,10 +91,10 @@ enum {
   PROF_SPAN_CYCLES, kProfSlots = 8
 };
 
-// Records the launch's first error.
+// Records the launch's first error, in both words: waits that end because of
+// another CTA's error call this too, with codes of their own.
 __device__ __forceinline__ void device_error(const StepArgs& a, int code) {
-  atomicCAS(a.err, 0, code);
-  if (a.err_host) *reinterpret_cast<volatile int*>(a.err_host) = code;
+  if (atomicCAS(a.err, 0, code) == 0 && a.err_host) *reinterpret_cast<volatile int*>(a.err_host) = code;
 }
 
 // Lets launches of a step kernel ask for as much dynamic shared memory as any
