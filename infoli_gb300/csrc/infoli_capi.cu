@@ -678,7 +678,7 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
   std::vector<Pending> pend;
   int launches = 0;
   CK(cudaEventRecord(s->ev_t0, s->stream));
-  int done = 0, li = 0;
+  int done = 0, traced = 0;
   auto drain = [&](const Pending& p) -> int {
     CK(cudaEventSynchronize(s->ev_kernel[p.slot]));
     // rows are the multiples of trace_every in the launch's step range
@@ -693,14 +693,14 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
   };
   while (done < n_steps) {
     const int len = std::min(launch_steps, n_steps - done);
-    const int slot = li & 1;
+    const int slot = traced & 1;  // launches without a row take none
     a.step0 = s->step + done;
     a.n_steps = len;
     a.stim_table = table_at(s, a.step0);
     a.trace = nq ? s->h_trace[slot] : nullptr;
     const int rows = count_rows(a.step0, len, trace_every);
     // the slot's previous contents must have been consumed
-    if (pend.size() >= 2) {
+    if (rows > 0 && pend.size() >= 2) {
       int rc = drain(pend.front());
       if (rc) return rc;
       pend.erase(pend.begin());
@@ -712,9 +712,9 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
     if (rows > 0) {
       CK(cudaEventRecord(s->ev_kernel[slot], s->stream));
       pend.push_back({slot, a.step0, rows});
+      ++traced;
     }
     done += len;
-    ++li;
   }
   CK(cudaEventRecord(s->ev_t1, s->stream));
   for (const Pending& p : pend) {

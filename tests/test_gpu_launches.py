@@ -100,3 +100,21 @@ def test_threads_create_and_run_simulations_of_different_sizes(ig):
     for t in threads:
         t.join()
     assert not failed, failed[0]
+
+
+@pytest.mark.parametrize("every", [8192, 10000, 16384, 20000])
+def test_trace_intervals_longer_than_a_launch(ig, every):
+    """Launches without a trace row between those with one (a launch has at most 8,192 steps): each row is that of its step."""
+    conf, n, steps = O.read_parameters(CONF), 30, 60000
+    rp, col = ig.gen_uniform(n, 0.2, 2)
+    st0 = hetero_state(conf, n, 3)
+    with ig.Simulation(n, conf, rp, col, init_state=st0) as sim:
+        got, state = sim.run(steps, every, ig.TRACE_SOMA)["soma"], sim.get_state()
+    want = []
+    with ig.Simulation(n, conf, rp, col, init_state=st0) as sim:
+        for t in range(0, steps, every):
+            sim.run(t - sim.step)
+            want.append(sim.run(1, 1, ig.TRACE_SOMA)["soma"][0])
+        sim.run(steps - sim.step)
+        assert np.array_equal(state, sim.get_state())
+    assert np.array_equal(got, np.array(want))
