@@ -556,9 +556,10 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
                            pl.chunks.size() * sizeof(ChunkDesc) + pl.cell_slots.size() * sizeof(CellSlots) +
                            pl.edges.size() * sizeof(uint16_t) + pl.edge_g.size() * sizeof(float) +
                            pl.probes.size() * sizeof(int) + pl.gdesc.size() * sizeof(int2_t) +
-                           pl.gcol.size() * sizeof(int32_t)) +
+                           pl.gcol.size() * sizeof(int32_t) + pl.perm.size() * sizeof(int32_t)) +
                  (int64_t)np * (2 * sizeof(float) + F_COUNT * sizeof(float) + sizeof(double)) + 256 +
-                 (pl.shape.stamped ? (int64_t)np * 2 * sizeof(unsigned long long) : 0);
+                 (pl.shape.stamped ? (int64_t)np * 2 * sizeof(unsigned long long) : 0) +
+                 (pl.shape.gather >= 3 ? (int64_t)np * 2 * sizeof(float) : 0);
   *out = s;
   return INFOLI_OK;
 }
