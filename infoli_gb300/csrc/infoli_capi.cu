@@ -91,6 +91,43 @@ cudaError_t pool_alloc(T** dst, size_t bytes, int device, cudaStream_t st) {
   return cudaMallocFromPoolAsync((void**)dst, bytes, pool, st);
 }
 
+// Error words of the handles, in pinned memory that every device's kernels may
+// write.  One page per process, made with the first handle: pinned memory of a
+// handle's own would be freed with it, and cudaFreeHost waits for every kernel
+// on the device.  A handle beyond the page's words gets none (null) and reads
+// its device word instead.
+struct ErrorWords {
+  enum { kWords = 1024 };
+  std::mutex mu;
+  int* page = nullptr;
+  std::vector<int> free_words;
+
+  int* take() {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!page) {
+      if (cudaHostAlloc((void**)&page, kWords * sizeof(int), cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        page = nullptr;
+        return nullptr;
+      }
+      for (int i = kWords - 1; i >= 0; --i) free_words.push_back(i);
+    }
+    if (free_words.empty()) return nullptr;
+    const int i = free_words.back();
+    free_words.pop_back();
+    return page + i;
+  }
+  void give(int* w) {  // no kernel of the handle runs any more
+    if (!w) return;
+    std::lock_guard<std::mutex> lk(mu);
+    free_words.push_back((int)(w - page));
+  }
+};
+ErrorWords& error_words() {
+  static ErrorWords* w = new ErrorWords();  // outlives handles that are destroyed at exit
+  return *w;
+}
+
 template <class T>
 int dev_upload(T** dst, const T* src, size_t count, int device, cudaStream_t st) {
   *dst = nullptr;
@@ -145,7 +182,7 @@ struct infoli_sim {
   // trace ring
   float* h_trace[2] = {nullptr, nullptr};
   size_t trace_floats[2] = {0, 0};  // room in each slot
-  int* h_err = nullptr;             // pinned: where a run's kernels report an error, or null
+  int* h_err = nullptr;             // where a run's kernels report an error (ErrorWords), or null
   bool stamps_valid = false;  // the stamped words are those of the current state and step
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_kernel[2] = {nullptr, nullptr};
@@ -172,7 +209,8 @@ void release(infoli_sim* s) {
       if (p) cudaFreeAsync(p, s->stream);
     cudaStreamSynchronize(s->stream);
   }
-  for (void* h : {(void*)s->h_trace[0], (void*)s->h_trace[1], (void*)s->h_err})
+  error_words().give(s->h_err);
+  for (float* h : s->h_trace)
     if (h) cudaFreeHost(h);
   for (cudaEvent_t e : {s->ev_kernel[0], s->ev_kernel[1], s->ev_t0, s->ev_t1})
     if (e) cudaEventDestroy(e);
@@ -428,6 +466,7 @@ int infoli_sim_create(const infoli_sim_desc* d, infoli_sim** out) {
   if (cudaSetDevice(s->device) != cudaSuccess) return fail(infoli__fail(INFOLI_ERR_CUDA, "cudaSetDevice failed"));
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess)
     return fail(infoli__fail(INFOLI_ERR_CUDA, "stream creation failed"));
+  s->h_err = error_words().take();
 
   // ---- plan
   int nsm = 0, smem_optin = 0;
@@ -659,10 +698,6 @@ int infoli_sim_run(infoli_sim* s, int n_steps, int trace_every, int trace_what, 
     const size_t want = std::min(need, (size_t)rows_needed * row_floats);
     for (int i = 0; i < (n_steps > launch_steps ? 2 : 1); ++i)
       if (int rc = trace_slot(s, i, want)) return rc;
-  }
-  if (!s->h_err && cudaMallocHost((void**)&s->h_err, sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    s->h_err = nullptr;
   }
   if (s->h_err) *s->h_err = DEV_OK;
 

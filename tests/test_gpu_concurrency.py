@@ -1,0 +1,67 @@
+"""What one handle's calls may wait for: its own work, not the launches of others that leave SMs free."""
+import numpy as np
+import pytest
+
+from helpers import CONF, hetero_state
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ig(built):
+    import infoli_gb300
+
+    assert infoli_gb300.device_count() >= 1
+    return infoli_gb300
+
+
+@pytest.fixture
+def busy(ig):
+    """A simulation of a few CTAs with about two seconds of steps enqueued."""
+    conf, n = O.read_parameters(CONF), 50
+    rp, col = ig.gen_uniform(n, 0.3, 2)
+    with ig.Simulation(n, conf, rp, col, init_state=hetero_state(conf, n, 3)) as sim:
+        sim.run(10)
+        with _small(ig) as other:  # a kernel's first use loads it, which waits for the device
+            other.run(20)
+            other.get_state()
+        sim.launch(1_500_000)
+        yield sim
+        sim.sync()
+
+
+def _small(ig, n=50):
+    conf = O.read_parameters(CONF)
+    rp, col = ig.gen_uniform(n, 0.3, 4) if n > 2 else ig.gen_uniform(n, 1.0, 4)
+    return ig.Simulation(n, conf, rp, col, init_state=hetero_state(conf, n, 5))
+
+
+def test_create_run_and_destroy_beside_a_running_simulation(ig, busy):
+    sim = _small(ig)
+    sim.run(20)
+    sim.get_state()
+    sim.close()
+    assert not busy.query()
+
+
+def test_more_handles_than_error_words(ig, monkeypatch):
+    sims = [_small(ig, 2) for _ in range(1030)]
+    want = None
+    for sim in sims:
+        sim.run(3)
+        got = sim.get_state()
+        assert want is None or np.array_equal(got, want)
+        want = got
+    monkeypatch.setenv("INFOLI_STALL_CTA", "1")
+    monkeypatch.setenv("INFOLI_WAIT_TIMEOUT_MS", "100")
+    with _small(ig, 500) as last:  # without a word of its own: errors come from the device's
+        with pytest.raises(ig.InfoliError) as e:
+            last.run(5)
+        assert e.value.code == ig.capi.ERR_TIMEOUT
+    for sim in sims:
+        sim.close()
+    with _small(ig, 500) as again:
+        with pytest.raises(ig.InfoliError) as e:
+            again.run(5)
+        assert e.value.code == ig.capi.ERR_TIMEOUT
