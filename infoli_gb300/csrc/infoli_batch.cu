@@ -630,10 +630,13 @@ uint32_t reverse_bits(uint32_t x) {
 void batch_release(infoli_batch* b) {
   if (!b) return;
   cudaSetDevice(b->device);
-  if (b->stream) cudaStreamSynchronize(b->stream);
+  if (b->stream) {
+    if (b->d_bits) cudaFreeAsync(b->d_bits, b->stream);
+    cudaStreamSynchronize(b->stream);
+  }
   if (b->graph_exec) cudaGraphExecDestroy(b->graph_exec);
   if (b->graph) cudaGraphDestroy(b->graph);
-  for (void* p : {(void*)b->d_cta, (void*)b->d_bits, (void*)b->d_st, (void*)b->d_ca, (void*)b->d_step,
+  for (void* p : {(void*)b->d_cta, (void*)b->d_st, (void*)b->d_ca, (void*)b->d_step,
                   (void*)b->d_cta_ns, (void*)b->d_ent, (void*)b->d_grp})
     if (p) cudaFree(p);
   for (BatchGroup& g : b->groups) {
@@ -944,8 +947,14 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
       std::fill(st.begin() + (size_t)k * b->total, st.begin() + (size_t)(k + 1) * b->total, d->init_values[k]);
   }
   std::vector<double> ca(st.begin() + 4 * b->total, st.begin() + 5 * b->total);
+  // Everything goes over the batch's own stream, and the bitmasks of the lists,
+  // needed only for their packing, come from the library's pool: a wait for the
+  // device or a cudaFree would wait for other handles' launches too.
+  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
+    return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: stream creation failed"));
   if (cudaMalloc((void**)&b->d_cta, sizeof(BatchCta) * b->cta.size()) != cudaSuccess ||
-      cudaMalloc((void**)&b->d_bits, sizeof(uint32_t) * std::max<size_t>(1, up_words)) != cudaSuccess ||
+      cudaMallocFromPoolAsync((void**)&b->d_bits, sizeof(uint32_t) * std::max<size_t>(1, up_words),
+                              infoli__device_pool(b->device), b->stream) != cudaSuccess ||
       (b->lists && (cudaMalloc((void**)&b->d_ent, (size_t)std::max(1LL, rows_total) * 512) != cudaSuccess ||
                     cudaMalloc((void**)&b->d_grp, sizeof(int2) * grp.size()) != cudaSuccess)) ||
       cudaMalloc((void**)&b->d_st, sizeof(float) * st.size()) != cudaSuccess ||
@@ -967,33 +976,36 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
   // the CTAs on the device at a time read their lists from L2 where they fit
   const double in_flight = (double)rows_total * 512.0 * std::min(1.0, (double)kBatchSms / (double)b->cta.size());
   for (BatchGroup& g : b->groups) g.l2_keep = (float)std::min(1.0, kBatchL2Bytes / std::max(1.0, in_flight));
-  if (cudaMemcpy(b->d_cta, b->cta.data(), sizeof(BatchCta) * b->cta.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b->d_bits, up_bits, sizeof(uint32_t) * up_words, cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b->d_st, st.data(), sizeof(float) * st.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(b->d_ca, ca.data(), sizeof(double) * ca.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemset(b->d_step, 0, sizeof(int)) != cudaSuccess ||
-      cudaMemset(b->d_cta_ns, 0, sizeof(unsigned long long) * 2 * b->cta.size()) != cudaSuccess)
-    return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: upload failed"));
+  auto upload = [&](void* dst, const void* src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, b->stream);
+  };
+  cudaError_t e = upload(b->d_cta, b->cta.data(), sizeof(BatchCta) * b->cta.size());
+  if (e == cudaSuccess) e = upload(b->d_bits, up_bits, sizeof(uint32_t) * up_words);
+  if (e == cudaSuccess) e = upload(b->d_st, st.data(), sizeof(float) * st.size());
+  if (e == cudaSuccess) e = upload(b->d_ca, ca.data(), sizeof(double) * ca.size());
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_step, 0, sizeof(int), b->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b->d_cta_ns, 0, sizeof(unsigned long long) * 2 * b->cta.size(), b->stream);
   if (b->lists) {
-    cudaError_t e = cudaMemcpy(b->d_grp, grp.data(), sizeof(int2) * grp.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(b->d_grp, grp.data(), sizeof(int2) * grp.size());
     // lanes without a receiver read entry 0
-    if (e == cudaSuccess) e = cudaMemset(b->d_ent, 0, (size_t)std::max(1LL, rows_total) * 512);
+    if (e == cudaSuccess) e = cudaMemsetAsync(b->d_ent, 0, (size_t)std::max(1LL, rows_total) * 512, b->stream);
     for (int i = 0; i < d->n_nets && e == cudaSuccess; ++i) {
       const int n = d->n_cells[i], cs = ctas_of(i, lanes[i]), per = (n + cs - 1) / cs, rows = 32 / lanes[i];
-      batch_pack_kernel<<<(n + kPackWarps - 1) / kPackWarps, kPackWarps * 32>>>(
+      batch_pack_kernel<<<(n + kPackWarps - 1) / kPackWarps, kPackWarps * 32, 0, b->stream>>>(
           b->d_bits + in_base[i], n, per, (per + rows - 1) / rows, lanes[i] - 1, b->d_grp + group_base[i], b->d_ent);
       e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e != cudaSuccess)
-      return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: entry lists: %s", cudaGetErrorString(e)));
-    cudaFree(b->d_bits);
-    b->d_bits = nullptr;
+    if (e == cudaSuccess) {
+      e = cudaFreeAsync(b->d_bits, b->stream);
+      b->d_bits = nullptr;
+    }
   }
-  if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
+  if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
+  if (e != cudaSuccess)
+    return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: upload failed: %s", cudaGetErrorString(e)));
+  if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess)
-    return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: stream/event creation failed"));
+    return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: event creation failed"));
   for (BatchGroup& g : b->groups)
     if (cudaStreamCreateWithPriority(&g.stream, cudaStreamNonBlocking, g.priority) != cudaSuccess ||
         cudaEventCreateWithFlags(&g.done, cudaEventDisableTiming) != cudaSuccess)

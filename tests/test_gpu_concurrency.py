@@ -65,3 +65,24 @@ def test_more_handles_than_error_words(ig, monkeypatch):
         with pytest.raises(ig.InfoliError) as e:
             again.run(5)
         assert e.value.code == ig.capi.ERR_TIMEOUT
+
+
+def _batch(ig):
+    conf = O.read_parameters(CONF)
+    nets = [(n, ig.gen_bitmask(n, 0.2, n), 0.03) for n in (300, 1500)]
+    return ig.Batch(conf, nets, init_state=hetero_state(conf, 1800, 3))
+
+
+def test_batch_create_beside_a_running_simulation(ig):
+    conf, n = O.read_parameters(CONF), 50
+    rp, col = ig.gen_uniform(n, 0.3, 2)
+    with _batch(ig) as first, ig.Simulation(n, conf, rp, col, init_state=hetero_state(conf, n, 3)) as busy:
+        first.run(30)
+        busy.run(10)
+        busy.launch(1_500_000)
+        second = _batch(ig)
+        assert not busy.query()
+        busy.sync()
+        second.run(30)
+        assert np.array_equal(second.get_state(), first.get_state())
+        second.close()
