@@ -325,8 +325,9 @@ typedef struct {
    *                   SM; the same as INFOLI_RES_FIT for 1,024 threads);
    *   INFOLI_RES_NONE none.
    * Batches run on entry lists made from the bitmasks unless those would take
-   * over half of the free device memory; lists are always streamed, and
-   * residency then changes nothing.
+   * over half of the free device memory (INFOLI_BATCH_ROWS=bits in the
+   * environment: bitmask rows whatever their size); lists are always streamed,
+   * and residency then changes nothing.
    * infoli_batch_autotune picks it together with block. */
   int residency;
 } infoli_batch_desc;

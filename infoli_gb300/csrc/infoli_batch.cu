@@ -824,10 +824,13 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
     groups_total += (long long)groups[i].size();
   }
   // Entry lists (16 bits per edge, 512 bytes per pair row) unless they would
-  // take more than half of the free memory: then the rows as bits.
+  // take more than half of the free memory, or the caller's environment asks
+  // for the rows as bits.
   size_t mem_free = 0, mem_total = 0;
   cudaMemGetInfo(&mem_free, &mem_total);
-  b->lists = (double)rows_total * 512.0 <= 0.5 * (double)mem_free && rows_total <= INT32_MAX;
+  const char* rows_env = getenv("INFOLI_BATCH_ROWS");
+  b->lists = (double)rows_total * 512.0 <= 0.5 * (double)mem_free && rows_total <= INT32_MAX &&
+             !(rows_env && !std::strcmp(rows_env, "bits"));
   if (!b->lists) std::fill(lanes.begin(), lanes.end(), 1);
   int smem_optin = 0, smem_sm = 0, prio_lo = 0, prio_hi = 0;
   cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
