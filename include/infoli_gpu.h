@@ -368,8 +368,9 @@ int infoli_batch_destroy(infoli_batch* b);
  * It returns the pick in out->block and out->residency -- the first
  * candidate unless a later one is more than 2% faster than the pick so far
  * (trial noise is a few percent; the first candidate is the default layout)
- * -- and the device time per step of every candidate; pass both to
- * infoli_batch_create.  The trial steps start at step 0, so they see no
+ * -- and the device time per step of every candidate (candidates that differ in
+ * residency alone are one layout, timed once, where the batch runs on entry
+ * lists); pass both to infoli_batch_create.  The trial steps start at step 0, so they see no
  * stimulus pulse.  desc itself is not modified. */
 enum { INFOLI_TUNE_CANDIDATES = 5 };
 typedef struct {

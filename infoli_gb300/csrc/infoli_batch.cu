@@ -1147,7 +1147,8 @@ extern "C" int infoli_batch_destroy(infoli_batch* b) {
 // The launch layout -- cells per CTA (and with it the cluster sizes and how
 // many networks share an SM) together with which networks keep their bitmask
 // rows in shared memory (which in turn decides whether two 512-thread CTAs
-// fit on an SM) -- is picked by timing every candidate on a trial batch.
+// fit on an SM; entry lists have none, so with them one candidate per CTA size
+// is timed) -- is picked by timing every candidate on a trial batch.
 // The trial batch is a stratified sample of the networks: sorted by size,
 // m evenly spaced picks, m the smallest count whose cells reach the target
 // (every SM's 1,024 threads twice over; m at most 4,096 unless the caller
@@ -1254,8 +1255,15 @@ extern "C" int infoli_batch_autotune(const infoli_batch_desc* d, int max_sample,
   const int cand_block[INFOLI_TUNE_CANDIDATES] = {1024, 1024, 512, 512, 512};
   const int cand_res[INFOLI_TUNE_CANDIDATES] = {INFOLI_RES_FIT, INFOLI_RES_NONE, INFOLI_RES_FIT, INFOLI_RES_OCC,
                                                 INFOLI_RES_NONE};
-  int best = 0;
+  int best = 0, by_lists = -1;  // by_lists: the last candidate timed on entry lists
   for (int s = 0; s < INFOLI_TUNE_CANDIDATES; ++s) {
+    out->cand_block[s] = cand_block[s];
+    out->cand_residency[s] = cand_res[s];
+    // entry lists have no residency: the same layout again, and its time
+    if (by_lists >= 0 && cand_block[by_lists] == cand_block[s]) {
+      out->cand_ms_per_step[s] = out->cand_ms_per_step[by_lists];
+      continue;
+    }
     t.block = cand_block[s];
     t.residency = cand_res[s];
     infoli_batch* b = nullptr;
@@ -1269,9 +1277,8 @@ extern "C" int infoli_batch_autotune(const infoli_batch_desc* d, int max_sample,
       rc = infoli_batch_run(b, trial_steps);
       if (k == 0 || b->last_ms < ms) ms = b->last_ms;
     }
-    out->cand_block[s] = cand_block[s];
-    out->cand_residency[s] = cand_res[s];
     out->cand_ms_per_step[s] = ms / (float)trial_steps;
+    if (b->lists) by_lists = s;
     batch_release(b);  // keeps the error message of a failed run
     if (rc != INFOLI_OK) return rc;
     // a later candidate replaces the pick only when it is clearly faster:

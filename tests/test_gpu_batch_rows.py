@@ -50,3 +50,20 @@ def test_bitmask_rows_match_the_oracle_in_every_layout(ig, kahan, monkeypatch):
         mine = first[:, offsets[i]:offsets[i + 1]]
         assert np.max(np.abs(mine[O.S["V_soma"]] - s[O.S["V_soma"]])) <= TOL_VSOMA_MV
         assert np.max(np.abs(mine[O.S["V_dend"]] - s[O.S["V_dend"]])) <= TOL_VSOMA_MV
+
+
+@pytest.mark.parametrize("rows", ["lists", "bits"])
+def test_autotune_times_each_layout_once(ig, rows, monkeypatch):
+    """Entry lists have no residency: candidates that differ in it alone are one layout with one time."""
+    if rows == "bits":
+        monkeypatch.setenv("INFOLI_BATCH_ROWS", "bits")
+    conf = O.read_parameters(CONF)
+    nets = [(n, ig.gen_bitmask(n, p, 5 + n), 0.03) for n, p in zip(SIZES, DENS)]
+    with ig.Batch(conf, nets, init_values=O.default_state(1, conf)[:, 0], shape="auto", tune_steps=20) as bt:
+        ms = bt.tune["ms_per_step"]
+        assert all(v > 0 for v in ms.values())
+        assert ms[f"{bt.tune['block']}/{bt.tune['residency']}"] * 0.98 <= min(ms.values())
+        if rows == "lists":
+            assert ms["1024/none"] == ms["1024/fit"] and ms["512/none"] == ms["512/occupancy"] == ms["512/fit"]
+            assert bt.tune["residency"] == "fit"
+        bt.run(10)
