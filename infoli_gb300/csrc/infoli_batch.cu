@@ -616,8 +616,6 @@ namespace {
 // Of the entry lists that the CTAs on the device read, what L2 (129 MB) is
 // asked to keep from step to step (more was slower for one network's lists).
 constexpr double kBatchL2Bytes = 70e6;
-constexpr int kBatchSms = 152;
-constexpr int kListMaxCtas = 16;  // CTAs per network, entry lists
 
 uint32_t reverse_bits(uint32_t x) {
   x = ((x >> 1) & 0x55555555u) | ((x & 0x55555555u) << 1);
@@ -698,7 +696,10 @@ int max_clusters(int block, int cluster, size_t smem, int lanes) {
   fill_config(cfg, at, cluster, block, cluster, smem, 0, nullptr);
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kernel_ptr(block, false, lanes), &cfg) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel_ptr(block, false, lanes), &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
   return n;
 }
 
@@ -786,16 +787,25 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
     weight[i] = (double)ones / n + 64.0;
     edges[i] = ones;
   }
-  // Two lanes per receiver where they cost no further CTA, and for networks
-  // whose CTAs would still run when all others are done (more than 3/4 of an
-  // SM's share of the whole batch each).
+  int smem_optin = 0, smem_sm = 0, sms = 0, prio_lo = 0, prio_hi = 0;
+  cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+  cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
+  const size_t budget = (size_t)smem_optin - 1024;
+  if (set_attrs(b->block, budget, std::max(max_cs, (int)kListMaxCtas)) != cudaSuccess)
+    return fail(infoli__fail(INFOLI_ERR_CUDA, "batch_create: kernel attributes could not be set"));
+  // Two lanes per receiver where the rule wants them and the device runs the
+  // clusters they make (asked for the largest network's shared memory).
   double all_edges = 0.0;
   for (long long e : edges) all_edges += (double)e;
-  auto ctas_of = [&](int i, int ln) { return (d->n_cells[i] * ln + b->block - 1) / b->block; };
+  auto ctas_of = [&](int i, int ln) { return list_ctas(d->n_cells[i], ln, b->block); };
+  bool runs[kListMaxCtas + 1] = {};
+  const int n_most = *std::max_element(d->n_cells, d->n_cells + d->n_nets);
+  for (int cs = 1; cs <= kListMaxCtas; ++cs)
+    runs[cs] = max_clusters(b->block, cs, list_smem(b->block, ((n_most + 31) / 32) * 32 + 32), 2) > 0;
   for (int i = 0; i < d->n_nets; ++i)
-    if (ctas_of(i, 2) == ctas_of(i, 1) ||
-        (ctas_of(i, 2) <= kListMaxCtas && (double)edges[i] / ctas_of(i, 1) > 0.75 * all_edges / kBatchSms))
-      lanes[i] = 2;
+    lanes[i] = list_lanes(d->n_cells[i], (double)edges[i], all_edges, b->block, sms, runs);
 #pragma omp parallel for schedule(dynamic, 1)
   for (int i = 0; i < d->n_nets; ++i) {
     const int n = d->n_cells[i], cs = ctas_of(i, lanes[i]), per = (n + cs - 1) / cs;
@@ -823,20 +833,13 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
     rows_total += pair_rows[i];
     groups_total += (long long)groups[i].size();
   }
-  // Entry lists (16 bits per edge, 512 bytes per pair row) unless they would
-  // take more than half of the free memory, or the caller's environment asks
-  // for the rows as bits.
+  // Entry lists unless memory is short or the caller's environment asks for
+  // the rows as bits.
   size_t mem_free = 0, mem_total = 0;
   cudaMemGetInfo(&mem_free, &mem_total);
   const char* rows_env = getenv("INFOLI_BATCH_ROWS");
-  b->lists = (double)rows_total * 512.0 <= 0.5 * (double)mem_free && rows_total <= INT32_MAX &&
-             !(rows_env && !std::strcmp(rows_env, "bits"));
+  b->lists = lists_fit(rows_total, in_total, (double)mem_free) && !(rows_env && !std::strcmp(rows_env, "bits"));
   if (!b->lists) std::fill(lanes.begin(), lanes.end(), 1);
-  int smem_optin = 0, smem_sm = 0, prio_lo = 0, prio_hi = 0;
-  cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
-  cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->device);
-  cudaDeviceGetStreamPriorityRange(&prio_lo, &prio_hi);
-  const size_t budget = (size_t)smem_optin - 1024;
   // shared memory a group may spend on resident rows: all of a CTA's budget
   // (FIT), what keeps 2048 / block CTAs on an SM (OCC; the runtime reserves
   // 1 KB per CTA), or nothing (NONE)
@@ -879,7 +882,7 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
     g.smem = b->lists ? list_smem(b->block, g.vcap) : vbytes + sizeof(uint32_t) * (size_t)g.res_words;
     if (g.smem > budget)
       return fail(infoli__fail(INFOLI_ERR_CAPACITY, "batch_create: %zu bytes of shared memory needed", g.smem));
-    if (set_attrs(b->block, budget, max_ctas) != cudaSuccess || (g.max_active = max_clusters(b->block, cs, g.smem, g.lanes)) <= 0)
+    if ((g.max_active = max_clusters(b->block, cs, g.smem, g.lanes)) <= 0)
       return fail(infoli__fail(INFOLI_ERR_CAPACITY, "batch_create: clusters of %d CTAs of %d threads cannot run",
                                cs, b->block));
     // greatest priority for the longest (lists), else for the largest networks
@@ -977,7 +980,7 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
     }
   }
   // the CTAs on the device at a time read their lists from L2 where they fit
-  const double in_flight = (double)rows_total * 512.0 * std::min(1.0, (double)kBatchSms / (double)b->cta.size());
+  const double in_flight = (double)rows_total * 512.0 * std::min(1.0, (double)sms / (double)b->cta.size());
   for (BatchGroup& g : b->groups) g.l2_keep = (float)std::min(1.0, kBatchL2Bytes / std::max(1.0, in_flight));
   auto upload = [&](void* dst, const void* src, size_t bytes) {
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, b->stream);

@@ -39,6 +39,30 @@ struct alignas(16) BatchCta {
   int pad0;
 };
 
+// ---- rules for entry lists (batches)
+enum { kListMaxCtas = 16 };  // CTAs per network
+
+// CTAs of `block` threads of a network whose receivers take `lanes` lanes each.
+inline int list_ctas(int n, int lanes, int block) { return (n * lanes + block - 1) / block; }
+
+// Lanes per receiver: two where they cost no further CTA, and for networks
+// whose CTAs would still run when all others are done (more than 3/4 of an
+// SM's share of the whole batch each), as long as the device runs clusters of
+// that many CTAs (runs[cs]; beyond 8 that depends on the device).
+inline int list_lanes(int n, double edges, double all_edges, int block, int sms, const bool runs[kListMaxCtas + 1]) {
+  const int one = list_ctas(n, 1, block), two = list_ctas(n, 2, block);
+  if (two > kListMaxCtas || !runs[two]) return 1;
+  return two == one || edges / one > 0.75 * all_edges / sms ? 2 : 1;
+}
+
+// Entry lists (16 bits per edge, 512 bytes per pair row) rather than bitmask
+// rows: where they take no more than half of the free memory, and with the
+// bitmasks that they are packed from no more than nine tenths.
+inline bool lists_fit(long long pair_rows, long long bit_words, double mem_free) {
+  const double entries = (double)pair_rows * 512.0;
+  return pair_rows <= INT32_MAX && entries <= 0.5 * mem_free && entries + (double)bit_words * 4.0 <= 0.9 * mem_free;
+}
+
 // One network of a lane launch.
 struct LaneNet {
   float* st;             // [INFOLI_NSTATE * n] device SoA (reference order; the Ca2+ row is not used)
