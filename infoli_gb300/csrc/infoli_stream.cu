@@ -193,12 +193,11 @@ __device__ __forceinline__ bool stream_wait(const StepArgs& a, uint64_t* bar, un
 template <bool KAHAN, bool EDGE_G, bool BYTE, int N>
 __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int s_abort;  // a wait of this step gave up: set before the step's first CTA barrier
-  // The launch ends: set between that barrier and the step's last one, where
-  // every warp reads it.  (s_abort itself may be set again by the producer of
-  // the next step, and a slow warp that read it then would leave a step before
-  // the others, which wait for it without a limit.)
-  __shared__ int s_stop;
+  // A wait of the step gave up, for even and odd steps: past a step's last
+  // barrier its flag stays as it is until every warp has read it, while the
+  // producer may already set the next step's (a warp that read that one would
+  // leave a step before the others, which wait for it without a limit).
+  __shared__ int s_abort[2];
   __shared__ int s_copied;  // steps of the launch whose copies have been issued
   __shared__ float s_peer[kStreamMaxCluster];  // set by a CTA of the cluster that gave up
   __shared__ unsigned long long s_prof[4];  // cycles: gate units, wait for the share, coupling, rest
@@ -240,7 +239,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   if (tid == 0) {
     mbar_init(mbar, 1);
     fence_mbar_init();
-    s_abort = s_stop = s_copied = 0;
+    s_abort[0] = s_abort[1] = s_copied = 0;
     for (int k = 0; k < kStreamMaxCluster; ++k) s_peer[k] = 0.0f;
   }
   const int row0 = cs == 1 ? w.cell_begin : w.tile_begin, nrows = cs == 1 ? w.n_cells : w.n_tiles;
@@ -275,6 +274,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   };
   for (int st_i = 0; st_i < a.n_steps; ++st_i) {
     const int step = a.step0 + st_i;
+    int* const gave_up = s_abort + (st_i & 1);
     const bool trace_now = tclock.take();
     // V^step is written and every thread past a CTA barrier: arrive (the
     // release covers the CTA's writes)
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
         while (ld_acquire_gpu(a.bar) < bar_target) {
           if (ld_relaxed_gpu(a.err) != 0 || globaltimer_ns() - t0 > a.timeout_ns) {
             device_error(a, DEV_ERR_BARRIER_TIMEOUT);
-            *(volatile int*)&s_abort = 1;
+            *(volatile int*)gave_up = 1;
             ok = false;
             break;
           }
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
 
     // ---------------- coupling
     couple_stream<KAHAN, EDGE_G, BYTE, N>(a, w, warp, lane, sm, rows, part, pol, [&]() {
-      if (!stream_wait(a, mbar, (unsigned)st_i & 1u, &s_abort)) s_abort = 1;
+      if (!stream_wait(a, mbar, (unsigned)st_i & 1u, gave_up)) *gave_up = 1;
       mark(1);
     });
     const int per = cs > 1 ? (w.n_tiles + cs - 1) / cs : 0;  // rows of a CTA of the cluster
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
         const int k = (q >= per) + (q >= 2 * per) + (q >= 3 * per);
         st_peer(peer_addr(smem_u32(sums + w.pad1 * cap + (q - k * per)), (unsigned)k), s);
       }
-      if (s_abort && tid < cs) st_peer(peer_addr(smem_u32(s_peer + w.pad1), (unsigned)tid), 1.0f);
+      if (*gave_up && tid < cs) st_peer(peer_addr(smem_u32(s_peer + w.pad1), (unsigned)tid), 1.0f);
       cluster_sync_all();
     }
     mark(2);
@@ -420,10 +420,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     if (trace_now) ++row;
     // a CTA that gave up takes its cluster with it (no CTA may leave while
     // another writes to its shared memory)
-    if (tid < cs && (cs > 1 ? s_peer[tid] != 0.0f : s_abort != 0)) s_stop = 1;
+    if (cs > 1 && tid < cs && s_peer[tid] != 0.0f) *gave_up = 1;
     __syncthreads();
     mark(3);
-    if (s_stop) break;
+    if (*gave_up) break;
   }
   if (prof) {
     unsigned long long* pr = a.prof + (size_t)blockIdx.x * kProfSlots;
