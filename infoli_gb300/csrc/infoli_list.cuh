@@ -9,6 +9,8 @@
 
 namespace infoli {
 
+constexpr float kListVScale = 0.12011224087864497f;  // squared: log2(e) / 100
+
 // The entries are read once per step: past L1, and in L2 with a policy that
 // keeps the share of the lines that fits (`keep`; the rest is
 // evicted first, so it does not push out the others).  L1::no_allocate alone
@@ -41,8 +43,10 @@ __device__ __forceinline__ float4 ld_streamg(const float4* p, uint64_t pol) {
 }
 
 // N entries of a lane (two per word of o): -(their terms) into nt (two
-// accumulators: even and odd entries), in V_dend x kVScale (the exponent is
-// -(dV')^2).  All gathers first, then the arithmetic in stages: a warp then
+// accumulators: even and odd entries), in V_dend x kListVScale (the exponent is
+// -(dV')^2), or with PLAIN in V_dend itself (the difference is scaled for the
+// exponent alone: an operation more per pair of entries, but no rounding of the
+// voltages before their difference is taken).  All gathers first, then the arithmetic in stages: a warp then
 // waits once per block and not once per pair of entries (2.03 against 2.7
 // cycles of an SM per warp and entry in a loop over shared memory without bank
 // conflicts; the SFU and the FMA pipe take about one each).
@@ -60,7 +64,7 @@ __device__ __forceinline__ void stream_gather(const float* sm, const uint4* o, f
   }
 }
 
-template <int N, bool EDGE_G>
+template <int N, bool EDGE_G, bool PLAIN = false>
 __device__ __forceinline__ void stream_terms(float2* x, const float4* g, float2 nvc2, float2& nt) {
   const float2 c08 = make_float2(0.8f, 0.8f), c02 = make_float2(0.2f, 0.2f);
 #pragma unroll
@@ -68,13 +72,14 @@ __device__ __forceinline__ void stream_terms(float2* x, const float4* g, float2 
   float2 e[N / 2];
 #pragma unroll
   for (int k = 0; k < N / 2; ++k) {
-    const float2 sq = __fmul2_rn(x[k], x[k]);
+    const float2 d = PLAIN ? __fmul2_rn(x[k], make_float2(kListVScale, kListVScale)) : x[k];
+    const float2 sq = __fmul2_rn(d, d);
     e[k] = make_float2(ex2_approx(-sq.x), ex2_approx(-sq.y));
   }
 #pragma unroll
   for (int k = 0; k < N / 2; ++k) {
-    float2 f = __ffma2_rn(c08, e[k], c02);
-    if (EDGE_G) f = __fmul2_rn(k % 2 ? make_float2(g[k / 2].z, g[k / 2].w) : make_float2(g[k / 2].x, g[k / 2].y), f);
+    const float2 f = __ffma2_rn(c08, e[k], c02);
+    if (EDGE_G) x[k] = __fmul2_rn(k % 2 ? make_float2(g[k / 2].z, g[k / 2].w) : make_float2(g[k / 2].x, g[k / 2].y), x[k]);
     nt = __ffma2_rn(f, x[k], nt);
   }
 }

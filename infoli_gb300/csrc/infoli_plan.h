@@ -132,6 +132,7 @@ typedef struct {
   int cluster;     // stream plan: CTAs per cluster (sender shares)
   int rows_cap;    // stream plan with cluster > 1: staged V_dend of the cluster's receivers
   int block;       // stream plan: entries per lane taken at a time (8, or 16 for long lane-chunks)
+  int plain;       // stream plan: differences of V_dend itself, not of V_dend x kVScale
   int byte_off;    // stream plan: entries are byte offsets (the staged floats fit in 64 KB), else float indices
 } SmemShape;
 

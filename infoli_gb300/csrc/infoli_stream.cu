@@ -54,7 +54,7 @@ __device__ __forceinline__ void st_peer(uint32_t a, float v) {
 // quads, and a quad.  The next block's entries are loaded before this one's
 // arithmetic, across groups too, and the first group's before `wait` (the wait
 // for V_dend): no load latency stands between blocks.
-template <bool KAHAN, bool EDGE_G, bool BYTE, int N, class Wait>
+template <bool KAHAN, bool EDGE_G, bool PLAIN, bool BYTE, int N, class Wait>
 __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& w, int warp, int lane, const float* sm,
                                               const float* rows, float* part, uint64_t pol, Wait wait) {
   const int* wt = a.probes + w.pad0 + warp;
@@ -125,23 +125,23 @@ __device__ __forceinline__ void couple_stream(const StepArgs& a, const CtaWork& 
 #pragma unroll
         for (int i = 0; i < N / 4; ++i) now[i] = gc[i];
         if (nq >= 0) load_g(nq, gc);
-        stream_terms<N, EDGE_G>(x, now, nvc2, nt);
+        stream_terms<N, EDGE_G, PLAIN>(x, now, nvc2, nt);
       } else {
-        stream_terms<N, EDGE_G>(x, gc, nvc2, nt);
+        stream_terms<N, EDGE_G, PLAIN>(x, gc, nvc2, nt);
       }
       s.add(nt);
     }
     if (pair) {
       float2 x[4], nt = s.start();
       stream_gather<8, BYTE>(sm, &left_pair, x);
-      stream_terms<8, false>(x, &gt, nvc2, nt);
+      stream_terms<8, false, PLAIN>(x, &gt, nvc2, nt);
       s.add(nt);
     }
     if (odd) {
       float2 x[2], nt = s.start();
       const uint4 o = make_uint4(left_quad.x, left_quad.y, 0u, 0u);
       stream_gather<4, BYTE>(sm, &o, x);
-      stream_terms<4, EDGE_G>(x, &gt, nvc2, nt);
+      stream_terms<4, EDGE_G, PLAIN>(x, &gt, nvc2, nt);
       s.add(nt);
     }
     part[ld >> 16] = s.total();
@@ -190,9 +190,10 @@ __device__ __forceinline__ bool stream_wait(const StepArgs& a, uint64_t* bar, un
   return true;
 }
 
-template <bool KAHAN, bool EDGE_G, bool BYTE, int N>
+template <bool KAHAN, bool EDGE_G, bool PLAIN, bool BYTE, int N>
 __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_constant__ StepArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr float kScale = PLAIN ? 1.0f : kVScale, kBack = PLAIN ? 1.0f : kInvVScale;
   // A wait of the step gave up, for even and odd steps: past a step's last
   // barrier its flag stays as it is until every warp has read it, while the
   // producer may already set the next step's (a warp that read that one would
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     v.Vd = a.vd[a.step0 & 1][cell];
     v.Vs = st[F_VS * np + cell];
     v.Va = st[F_VA * np + cell];
-    a.vds[a.step0 & 1][cell] = v.Vd * kVScale;
+    a.vds[a.step0 & 1][cell] = v.Vd * kScale;
   }
   const VoltCoef vk = volt_coef(a.P);
   const uint64_t pol = l2_policy(a.l2_keep);
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
     __syncwarp();
 
     // ---------------- coupling
-    couple_stream<KAHAN, EDGE_G, BYTE, N>(a, w, warp, lane, sm, rows, part, pol, [&]() {
+    couple_stream<KAHAN, EDGE_G, PLAIN, BYTE, N>(a, w, warp, lane, sm, rows, part, pol, [&]() {
       if (!stream_wait(a, mbar, (unsigned)st_i & 1u, gave_up)) *gave_up = 1;
       mark(1);
     });
@@ -403,12 +404,12 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
       for (int k = 0; k < cs; ++k) ic += sums[k * cap + tid];
     }
     if (owner) {
-      ic *= kInvVScale;
+      ic *= kBack;
       if (!EDGE_G) ic *= a.g_uniform;
       v.Vd = voltage_second(a.P, vk, v.Vd, vh, ic, s_app[tid]);
       v.Vs = vh.Vs;
       v.Va = vh.Va;
-      a.vds[(step + 1) & 1][cell] = v.Vd * kVScale;
+      a.vds[(step + 1) & 1][cell] = v.Vd * kScale;
       if (trace_now) {
         float* tr = a.trace + (size_t)row * a.trace_nq * np + cell;
         int qi = 0;
@@ -453,15 +454,17 @@ __global__ void __launch_bounds__(kStreamThreads, 1) stream_kernel(const __grid_
   }
 }
 
-template <bool K, bool G, int N>
-const void* stream_fn2(bool byte_off) {
-  return byte_off ? (const void*)stream_kernel<K, G, true, N> : (const void*)stream_kernel<K, G, false, N>;
+template <bool G, bool P, int N>
+const void* stream_fn2(bool kahan, bool byte_off) {
+  if (kahan) return byte_off ? (const void*)stream_kernel<true, G, P, true, N> : (const void*)stream_kernel<true, G, P, false, N>;
+  return byte_off ? (const void*)stream_kernel<false, G, P, true, N> : (const void*)stream_kernel<false, G, P, false, N>;
 }
 
-const void* stream_fn(bool kahan, bool edge_g, bool byte_off, int block) {
-  if (edge_g) return kahan ? stream_fn2<true, true, 8>(byte_off) : stream_fn2<false, true, 8>(byte_off);
-  if (block == 8) return kahan ? stream_fn2<true, false, 8>(byte_off) : stream_fn2<false, false, 8>(byte_off);
-  return kahan ? stream_fn2<true, false, 16>(byte_off) : stream_fn2<false, false, 16>(byte_off);
+const void* stream_fn(const SmemShape& s, bool edge_g) {
+  const bool k = s.kahan != 0, b = s.byte_off != 0;
+  if (edge_g) return stream_fn2<true, true, 8>(k, b);
+  if (s.block == 8) return s.plain ? stream_fn2<false, true, 8>(k, b) : stream_fn2<false, false, 8>(k, b);
+  return s.plain ? stream_fn2<false, true, 16>(k, b) : stream_fn2<false, false, 16>(k, b);
 }
 
 void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, int cluster, size_t smem,
@@ -485,7 +488,7 @@ void stream_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int grid, i
 
 cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t stream) {
   const size_t smem = stream_layout(a.shape).total;
-  const void* fn = stream_fn(a.shape.kahan != 0, a.edge_g != nullptr, a.shape.byte_off != 0, a.shape.block);
+  const void* fn = stream_fn(a.shape, a.edge_g != nullptr);
   cudaError_t e = allow_shared_memory((const void*)fn);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg;
@@ -496,7 +499,7 @@ cudaError_t launch_stream_kernel(const StepArgs& a, int grid, cudaStream_t strea
 }
 
 int max_stream_ctas(int cluster, size_t smem) {
-  const void* fn = stream_fn(true, true, false, 8);
+  const void* fn = stream_fn2<true, true, 8>(true, false);
   if (allow_shared_memory((const void*)fn) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
