@@ -63,7 +63,7 @@ enum { kGatherMaxMeanDegree = 384 };
 
 // Stream plans are for edges that do not stay on chip.  Auto mode takes them
 //   - with the whole V_dend array as one share (up to about 50,000 cells), except
-//     for one conductance at a density of 1 / kStreamMaxDensityInv or more,
+//     for one conductance at a density of kStreamMaxDensity or more,
 //     where a bit per pair is shorter than 16 bits per edge by more than the
 //     walk of the bits costs;
 //   - with the senders shared by a cluster's CTAs for rows of at least
@@ -83,6 +83,24 @@ enum { kStampedMaxWords = 4500, kStampedMaxCells = 192 };
 enum { kStreamMinDegree = 16 };
 constexpr double kStreamMaxDensity = 0.45;
 
+// A vector whose resize() leaves new elements as they are: the threads that fill
+// a large table touch its pages first.
+template <class T>
+struct UnclearedAllocator : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = UnclearedAllocator<U>;
+  };
+  template <class U>
+  void construct(U*) noexcept {}
+  template <class U, class A, class... B>
+  void construct(U* p, A&& a, B&&... b) {
+    ::new ((void*)p) U(std::forward<A>(a), std::forward<B>(b)...);
+  }
+};
+template <class T>
+using Uncleared = std::vector<T, UnclearedAllocator<T>>;
+
 struct Plan {
   int grid = 0, threads = 0, tile_cap = 0, nbuf = 1, max_slots = 0;
   SmemShape shape{};                  // shared-memory shape of the launch
@@ -91,8 +109,8 @@ struct Plan {
   std::vector<TileDesc> tiles;
   std::vector<ChunkDesc> chunks;
   std::vector<CellSlots> cell_slots;  // [n]
-  std::vector<uint16_t> edges;
-  std::vector<float> edge_g;          // empty unless per-edge g
+  Uncleared<uint16_t> edges;
+  Uncleared<float> edge_g;            // empty unless per-edge g
   std::vector<int> probes;            // stamped mode: progress-probe cells
   std::vector<int2_t> gdesc;          // stamped mode: {slot, recv} per lane-chunk, 32 per group
   std::vector<int32_t> gcol;          // gather mode: sender ids, column by column per CTA;
