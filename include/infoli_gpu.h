@@ -510,6 +510,11 @@ int infoli_server_destroy(infoli_server* sv);
  * infoli_sim_run, which keeps the FP64 value between runs.
  * Device waits (the grid barrier) give up after INFOLI_WAIT_TIMEOUT_MS
  * (default 4000 ms) and return INFOLI_ERR_TIMEOUT.
+ * The kernel's CTAs (one per 32 cells, at most one per SM) run at the same
+ * time, two to an SM: from about 4,900 cells on a call waits until other
+ * kernels leave it half of the SMs.  INFOLI_NOALLOC_CTAS=<n> in the
+ * environment lets it run on fewer CTAs (of at most 512 cells), for callers
+ * whose other work holds most of the SMs for long.
  * The only scratch (V_dend double buffer, barrier counter, error word) is a
  * static device array of fixed size in the library, so networks are limited
  * to 65536 cells (INFOLI_ERR_CAPACITY beyond).  Every GPU that loads the

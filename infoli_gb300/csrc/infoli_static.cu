@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 
@@ -271,7 +272,12 @@ extern "C" int infoli_run_noalloc(const float* params, int n_cells, const int64_
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess)
     return infoli__fail(INFOLI_ERR_CUDA, "run_noalloc: cudaDeviceGetAttribute: %s", cudaGetErrorString(e));
-  const int per_cta = std::max(kNoAllocMinCells, (n_cells + nsm - 1) / nsm);
+  // as many CTAs as SMs, or as the caller's environment allows it beside other
+  // work (two of them fit on an SM)
+  int most = nsm;
+  if (const char* s = getenv("INFOLI_NOALLOC_CTAS")) most = std::max(1, std::min(nsm, atoi(s)));
+  most = std::max(most, (n_cells + kNoAllocBlock - 1) / kNoAllocBlock);
+  const int per_cta = std::max(kNoAllocMinCells, (n_cells + most - 1) / most);
   const int grid = (n_cells + per_cta - 1) / per_cta, cap = (per_cta + 31) & ~31;
   const size_t smem = noalloc_smem(cap);
   if (per_cta > kNoAllocBlock)

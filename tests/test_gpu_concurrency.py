@@ -86,3 +86,47 @@ def test_batch_create_beside_a_running_simulation(ig):
         second.run(30)
         assert np.array_equal(second.get_state(), first.get_state())
         second.close()
+
+
+def _noalloc(ig, torch, n, steps):
+    """A call of the allocation-free run: its state after `steps` steps."""
+    import ctypes as C
+
+    conf = O.read_parameters(CONF)
+    rp, col, g = ig.gen_fixed_degree(n, 30, 4, (0.02, 0.06))
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (rp, col, g, hetero_state(conf, n, 5).reshape(-1))]
+    torch.cuda.synchronize()
+    ptr = [C.c_void_p(t.data_ptr()) for t in dev]
+    side = torch.cuda.Stream()
+    params, lib = np.ascontiguousarray(conf[:23], np.float32), ig.capi.load()
+
+    def call():
+        rc = lib.infoli_run_noalloc(params.ctypes.data_as(C.c_void_p), n, ptr[0], ptr[1], ptr[2], 0.04, 0, 0, 0.0, ptr[3], 0,
+                                    steps, None, C.c_void_p(side.cuda_stream))
+        assert rc == 0, lib.infoli_last_error()
+        return dev[3].cpu().numpy()
+
+    return call
+
+
+@pytest.mark.parametrize("sms,ctas", [(76, None), (140, "10")])
+def test_noalloc_beside_a_running_simulation(ig, sms, ctas, monkeypatch):
+    """On half of the SMs it runs as it is, on a dozen with as few CTAs as its cells need."""
+    import torch
+
+    if torch.cuda.get_device_properties(0).multi_processor_count < 152:
+        pytest.skip("sized for 152 SMs")
+    if ctas:
+        monkeypatch.setenv("INFOLI_NOALLOC_CTAS", ctas)
+    conf, n = O.read_parameters(CONF), 10000
+    call, again = _noalloc(ig, torch, 5003, 100), _noalloc(ig, torch, 5003, 100)
+    want = call()
+    rp, col = ig.gen_grid_gaussian(100, 100, 10.0, 18.0, 3)
+    with ig.Simulation(n, conf, rp, col, init_state=hetero_state(conf, n, 3), grid=sms) as busy:
+        assert busy.plan_info()["grid"] == sms
+        busy.run(10)
+        busy.launch(300_000)
+        lib_done = again()
+        assert not busy.query()
+        busy.sync()
+    assert np.array_equal(lib_done, want)
