@@ -63,12 +63,6 @@ __device__ __forceinline__ unsigned cluster_rank() {
 
 // Store a float into the shared memory of CTA `peer` of this cluster at the
 // address that `local` has in this CTA.
-// The V_dend buffers hold V * kVScale (kVScale^2 = log2(e) / 100), so a
-// coupling term's exponent is -(dV')^2 with dV' = kVScale dV: one multiply
-// less per edge; the sums are scaled back once per receiver.
-constexpr float kVScale = 0.12011224087864497f;
-constexpr float kInvVScale = 8.325546111576978f;
-
 __device__ __forceinline__ void st_peer(float* local, unsigned peer, float v) {
   const unsigned la = smem_u32(local);
   unsigned ra;

@@ -9,7 +9,11 @@
 
 namespace infoli {
 
-constexpr float kListVScale = 0.12011224087864497f;  // squared: log2(e) / 100
+// Where V_dend x kVScale is held instead of V_dend (kVScale^2 = log2(e) / 100),
+// a coupling term's exponent is -(dV')^2 with dV' = kVScale dV, one multiply less
+// per edge; the sums are scaled back once per receiver.
+constexpr float kVScale = 0.12011224087864497f;
+constexpr float kInvVScale = 8.325546111576978f;
 
 // The entries are read once per step: past L1, and in L2 with a policy that
 // keeps the share of the lines that fits (`keep`; the rest is
@@ -43,7 +47,7 @@ __device__ __forceinline__ float4 ld_streamg(const float4* p, uint64_t pol) {
 }
 
 // N entries of a lane (two per word of o): -(their terms) into nt (two
-// accumulators: even and odd entries), in V_dend x kListVScale (the exponent is
+// accumulators: even and odd entries), in V_dend x kVScale (the exponent is
 // -(dV')^2), or with PLAIN in V_dend itself (the difference is scaled for the
 // exponent alone: an operation more per pair of entries, but no rounding of the
 // voltages before their difference is taken).  All gathers first, then the arithmetic in stages: a warp then
@@ -72,7 +76,7 @@ __device__ __forceinline__ void stream_terms(float2* x, const float4* g, float2 
   float2 e[N / 2];
 #pragma unroll
   for (int k = 0; k < N / 2; ++k) {
-    const float2 d = PLAIN ? __fmul2_rn(x[k], make_float2(kListVScale, kListVScale)) : x[k];
+    const float2 d = PLAIN ? __fmul2_rn(x[k], make_float2(kVScale, kVScale)) : x[k];
     const float2 sq = __fmul2_rn(d, d);
     e[k] = make_float2(ex2_approx(-sq.x), ex2_approx(-sq.y));
   }

@@ -2,16 +2,11 @@
 // gate state in shared memory, the trace countdown.
 #pragma once
 #include "infoli_kernels.cuh"
+#include "infoli_list.cuh"
 
 namespace infoli {
 
 constexpr float kNegLog2eOver100 = -0.014426950408889634f;  // -log2(e)/100
-// Stamped plans keep V_dend x kVScale in the window copy and the scaled-V cell
-// array (kVScale^2 = log2(e) / 100): a coupling term's exponent is then
-// -(dV')^2 with dV' = kVScale dV, one multiply less per edge; the partial sums
-// are scaled back once per receiver.
-constexpr float kVScale = 0.12011224087864497f;
-constexpr float kInvVScale = 8.325546111576978f;
 
 // One gate unit of local cell r on shared-memory state: its gates (field f at
 // sG[f * cap + r], Ca2+ in sCa), the compartment's voltage (sV: V_dend, V_soma,
