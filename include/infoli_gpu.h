@@ -68,7 +68,12 @@ enum {
 #define INFOLI_TRACE_DEND 4
 
 /* flags for infoli_sim_desc.flags */
-#define INFOLI_F_KAHAN 1     /* Kahan-compensated FP32 coupling sums */
+/* Compensated FP32 coupling sums.  How many terms are added plainly before a
+ * compensated addition depends on the plan: one (gathers, tiles), two (stamped
+ * words), 4 or 8 (entry lists of large networks and of batches), up to 32
+ * (bitmask rows); partial sums of a receiver are added with their errors, the
+ * sums of a cluster's two or four CTAs plainly. */
+#define INFOLI_F_KAHAN 1
 
 /* ------------------------------------------------------------------------ */
 /* library                                                                   */

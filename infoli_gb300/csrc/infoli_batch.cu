@@ -1,7 +1,8 @@
 // Batched simulation of many independent networks in one captured graph.
 //
-// Each network's cells are split over the CTAs of ONE thread-block cluster
-// (up to 8 CTAs of 1024 threads; one thread per cell, state in registers).
+// Each network's cells are split over the CTAs of ONE thread-block cluster, one
+// thread per cell (bitmask rows: up to 8 CTAs of 1,024 threads or 16 of 512, state
+// in registers; entry lists: up to 16 CTAs, gate state in shared memory).
 // Every CTA keeps the whole network's V_dend, double-buffered, in its shared
 // memory; a new V_dend is written to the CTA's own copy and, through
 // distributed shared memory, to the copies of the network's other CTAs, and
@@ -15,9 +16,10 @@
 // coupling's arithmetic).  Two ways to run them:
 //   - entry lists (list_kernel, batches): the rows are turned into 16-bit
 //     entries on the device when the batch is made, and streamed every step,
-//     one receiver per lane;
+//     one or two lanes per receiver;
 //   - bitmask rows (batch_kernel: the serving lane, and batches whose lists
-//     would take more than half of the free memory): a receiver walks the set
+//     would take more than half of the free memory or that were asked for
+//     them): a receiver walks the set
 //     bits of its row.  Rows are stored word-major so consecutive receivers
 //     read consecutive words; a network whose rows fit keeps them in shared
 //     memory for the launch, otherwise they are streamed every step.
@@ -756,9 +758,9 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
     bits_base[i] = bits_total;
     bits_total += (long long)n * ((n + 31) / 32 + 2);
   }
-  // time per step of a network ~ its mean row weight (set bits per receiver)
-  // plus a constant for the cell update: heavy networks are launched first
-  // and the pair rows of every warp's entry list: its longest row in eights
+  // Time per step of a network ~ its mean row weight (set bits per receiver)
+  // plus a constant for the cell update: heavy networks are launched first.
+  // Entry lists: the pair rows of every warp, its longest row in eights.
   std::vector<double> weight(d->n_nets);
   std::vector<std::vector<int2>> groups(d->n_nets);  // first pair row within the network, pairs per lane
   std::vector<std::vector<int>> degree(d->n_nets);
@@ -844,8 +846,9 @@ extern "C" int infoli_batch_create(const infoli_batch_desc* d, infoli_batch** ou
   const int max_ctas = b->lists ? std::max(max_cs, (int)kListMaxCtas) : max_cs;
   // Launches by the time a network's CTAs take (edges per CTA), the longest at
   // the highest priority, and within that by cluster size: a long network of
-  // few CTAs would otherwise start among the last (128 networks: 27.7-28.9 ms
-  // by cluster size alone, 25.2-25.4 with four classes).
+  // few CTAs would otherwise start among the last (128 networks of 256 to 8,192
+  // cells, 200 steps: 27.7-28.9 ms by cluster size alone, 25.2-25.4 with four
+  // classes in the same runs; 25.2-27.5 from one run of the process to another).
   double longest = 0.0;
   for (int i = 0; i < d->n_nets; ++i) longest = std::max(longest, (double)edges[i] / ctas_of(i, lanes[i]));
   auto class_of = [&](int i) {

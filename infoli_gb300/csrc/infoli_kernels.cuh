@@ -46,9 +46,12 @@ struct StepArgs {
   // state
   float* vd[2];               // V_dend double buffer, V^step in vd[step & 1]
   unsigned long long* vll[2]; // stamped mode: (step << 32 | V_dend bits) per cell, slot step & 1
-  float* vds[2];              // bitmask plans: V_dend x kVScale (the staged tiles), V^step in vds[step & 1]
-  const int* probes;          // stamped mode: progress-probe cells (CtaWork::probe_begin..)
-  const int2* gdesc;          // stamped mode: {slot, recv} per lane-chunk (32 per group)
+  float* vds[2];              // what CTAs stage of V^step, in vds[step & 1]: bitmask plans V_dend x kVScale,
+                              // stream plans that or V_dend itself (SmemShape::plain)
+  const int* probes;          // stamped mode: progress-probe cells (CtaWork::probe_begin..); stream plans:
+                              // each warp's groups (CtaWork::pad0..)
+  const int2* gdesc;          // stamped mode: {slot, recv} per lane-chunk (32 per group); stream plans:
+                              // {first quad row, quads per lane} per group
   float l2_keep;              // stream plans: share of the entries' lines that L2 should keep
   int n_cells;                // cells in the network (stamped words >= n_cells are never written)
   float* st;                  // F_COUNT x n_pad floats

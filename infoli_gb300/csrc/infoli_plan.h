@@ -17,7 +17,7 @@
 // Edge entries are 16-bit offsets from the tile start (a tile is at most
 // 65536 floats), so one gather from shared memory per edge.
 //
-// Two ways of exchanging V_dend between steps:
+// Two ways of exchanging V_dend between the steps of such plans:
 //   * barrier mode: V_dend double buffer in global memory, one grid barrier
 //     per step, tiles staged by bulk async copies (any window size);
 //   * stamped mode (every CTA's window fits in shared memory at once): every
@@ -29,6 +29,9 @@
 //     no slot is overwritten before its readers are done, until their stamps
 //     show the step it needs.  No grid barrier: each CTA waits only for its
 //     own neighbourhood.
+// Networks whose edges do not stay on chip have plans of their own (SmemShape::
+// gather): gathers through L2 or from staged tiles, adjacency bits, or entry lists
+// streamed over shares of V_dend (StreamLayout), all with the grid barrier.
 #pragma once
 #include <stddef.h>
 #include <stdint.h>
@@ -225,9 +228,10 @@ static inline INFOLI_HD SmemLayout smem_layout(SmemShape s) {
 // 100,000 cells x 100 senders with conductances, 6.96 against 6.80 at 6,007 x
 // 1,500, 4.17 against 4.10 at 48,017 x 33)
 // 24 warps, not 32: 80 registers a thread keep the loads of the coupling and
-// the gate units unspilled, which is worth more than the warps (13.1 -> 11.7 us
-// per step at 100,000 cells x 100 senders with conductances, 8.9 -> 8.3 at
-// 10,000 x 2,000, 4.4 -> 4.15 at 48,017 x 33).
+// the gate units unspilled (16 bytes spill with conductances per edge), which is
+// worth more than the warps (13.1 -> 11.7 us per step at 100,000 cells x 100
+// senders with conductances, 8.9 -> 8.3 at 10,000 x 2,000, 4.4 -> 4.15 at 48,017
+// x 33).
 enum { kStreamThreads = 768, kStreamWarps = 24, kStreamMaxCluster = 4 };
 typedef struct {
   size_t rows, part, sums, mbar, slots, app, total;
