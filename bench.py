@@ -31,8 +31,8 @@ Default line (--workload all), one JSON line with three parts:
   density U(0.01, 0.30), through the library's request loop; against the same
   requests run alone one after another (first in, first out) on the same GPU.
 
---impl reference times the reference's own OpenMP build on the host cores, or
-says that it is unavailable where that cannot be made.
+--impl reference times the reference's own OpenMP build (or, where it could
+not be built, the oracle's restatement of its loop) on the host cores.
 --case NAME runs one named small case once and prints its device time (the
 commands in profiles/ use these under ncu).
 """
@@ -317,30 +317,50 @@ def run_reference(args, world, rank):
     """Reference arm: the reference's own OpenMP build at the headline's cell
     count and mean degree (its CLI generates a uniform random network; it cannot
     express the Gaussian grid), 1,000 timesteps per bench step, timed by its own
-    clock; a line that says so where that build cannot be made or run."""
+    clock; the oracle port of its loop when the build is unavailable."""
     if rank != 0:
         return 0
     n = ROWS * COLS
     p = grid_stand_in_p()
     threads, model = host_cpu()
     sim_ms = STEPS_PER_ITER * 0.05
-    if reference_binary() is None:
-        print(json.dumps({"impl": "reference", "unavailable": "the reference's sources are not on this machine, so its "
-                                                              "OpenMP build cannot be made"}))
-        return 0
-    total = 0.0
-    for k in range(-args.warmup, args.steps):
-        r = run_reference_binary(n, p, sim_ms, threads)
-        if r is None:
-            print(json.dumps({"impl": "reference", "unavailable": "a run of the reference's OpenMP build failed"}))
-            return 0
-        if k >= 0:
+    kind = "reference"
+    if reference_binary() is not None:
+        for _ in range(args.warmup):
+            run_reference_binary(n, p, sim_ms, threads)
+        total = 0.0
+        for _ in range(args.steps):
+            r = run_reference_binary(n, p, sim_ms, threads)
+            if r is None:
+                kind = None
+                break
             total += r[1]
-    steps_per = reference_sim_steps(sim_ms)
-    sample = (f"per bench step one run of the untouched reference OpenMP build (src/openmp/infoli.c + "
-              f"src/utils/utils.c, gcc -O3 -fopenmp): -n {n} -p {p:.6f} -t {sim_ms:g} = {steps_per} "
-              f"timesteps, uniform random network with the grid's mean degree, trace every 100 steps, "
-              f"its own execution-time clock")
+        steps_per = reference_sim_steps(sim_ms)
+        sample = (f"per bench step one run of the untouched reference OpenMP build (src/openmp/infoli.c + "
+                  f"src/utils/utils.c, gcc -O3 -fopenmp): -n {n} -p {p:.6f} -t {sim_ms:g} = {steps_per} "
+                  f"timesteps, uniform random network with the grid's mean degree, trace every 100 steps, "
+                  f"its own execution-time clock")
+    else:
+        kind = None
+    if kind is None:
+        from oracle import oracle as O
+
+        O.build()
+        import numpy as np
+
+        kind = "port"
+        rp, col = O.gen_uniform(n, p, SEED)
+        conf = O.read_parameters(CONF_PATH)
+        st = O.default_state(n, conf)
+        st[0] += np.random.default_rng(SEED).uniform(-1, 1, n).astype(np.float32)
+        for _ in range(args.warmup):
+            cpu_port_rate(conf, n, rp, col, st, 10, threads)
+        total = 0.0
+        steps_per = 100
+        for _ in range(args.steps):
+            total += cpu_port_rate(conf, n, rp, col, st, steps_per, threads)[1]
+        sample = (f"reference build unavailable on this host; the oracle's restatement of its loop "
+                  f"(oracle/, C + OpenMP), {steps_per} timesteps per bench step, uniform network at p={p:.6f}")
     value = n * steps_per * args.steps / total
     line = {
         "impl": "reference", "metric": "cell-steps/s", "value": value, "unit": "cell-steps/s",
@@ -351,7 +371,7 @@ def run_reference(args, world, rank):
                    "timesteps_per_step": steps_per, "trace": f"V_axon every {TRACE_EVERY} timesteps",
                    "topology": "uniform random at the same cell count and mean degree (the reference's "
                                "generator, src/openmp/infoli.c:337-375)"},
-        "cpu_baseline": {"value": value, "unit": "cell-steps/s", "cores": threads, "cpu": model, "kind": "reference",
+        "cpu_baseline": {"value": value, "unit": "cell-steps/s", "cores": threads, "cpu": model, "kind": kind,
                          "sample": sample},
         "e2e": {"value": value, "unit": "cell-steps/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
@@ -924,33 +944,47 @@ def run_gpu_batched(args, world, rank, local, warmup=None):
 def run_reference_batched(args, world, rank):
     if rank != 0:
         return 0
+    from oracle import oracle as O
+
+    O.build()
+    conf = O.read_parameters(CONF_PATH)
     threads, model = host_cpu()
     # the networks' sizes, densities and conductances (the same draws as the
     # GPU arm's workload), without building the bitmasks or loading the product
     meta = batched_draws()
     nets = [None] * BATCH_NETS
     rates = []
+    kind = "reference"
     if reference_batched_rate(nets, meta, threads, k=2) is None:
-        print(json.dumps({"impl": "reference", "unavailable": "the reference's OpenMP build cannot be made or run on this "
-                                                              "machine"}))
-        return 0
+        kind = None
     t_total = 0.0
     picks = []
-    for _ in range(args.warmup):
-        reference_batched_rate(nets, meta, threads, k=2)
-    for _ in range(args.steps):
-        r, t, picks = reference_batched_rate(nets, meta, threads, k=4)
-        rates.append(r)
-        t_total += t
-    sample = (f"per bench step the untouched reference OpenMP build on networks {picks} (-n size -p density, "
-              f"CONDUCTANCE = its g, 100 timesteps, its own clock), extrapolated")
+    if kind == "reference":
+        for _ in range(args.warmup):
+            reference_batched_rate(nets, meta, threads, k=2)
+        for _ in range(args.steps):
+            r, t, picks = reference_batched_rate(nets, meta, threads, k=4)
+            rates.append(r)
+            t_total += t
+        sample = (f"per bench step the untouched reference OpenMP build on networks {picks} (-n size -p density, "
+                  f"CONDUCTANCE = its g, 100 timesteps, its own clock), extrapolated")
+    else:
+        kind = "port"
+        conf, nets, st, meta = batched_workload()
+        for _ in range(args.warmup):
+            cpu_batched_rate(conf, nets, st, meta, threads, steps=2, k=2)
+        for _ in range(args.steps):
+            r, t, picks = cpu_batched_rate(conf, nets, st, meta, threads, steps=5, k=4)
+            rates.append(r)
+            t_total += t
+        sample = f"per bench step networks {picks} x 5 timesteps of the oracle port, extrapolated"
     value = statistics.mean(rates)
     line = {
         "impl": "reference", "metric": "sims/s", "value": value, "unit": "sims/s (10,000-timestep simulations)",
         "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": 1e3 * t_total / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic", "config": batched_config(meta),
-        "cpu_baseline": {"value": value, "unit": "sims/s", "cores": threads, "cpu": model, "kind": "reference",
+        "cpu_baseline": {"value": value, "unit": "sims/s", "cores": threads, "cpu": model, "kind": kind,
                          "sample": sample},
         "e2e": {"value": value, "unit": "sims/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
